@@ -18,8 +18,9 @@
 //   * k_conv_tc: tcgen05 tensor cores (convnet_tc.cu), the default
 //   * k_conv_simt: CUDA cores, used as the device-side cross-check
 // Backward: data gradient = the same convolution with flipped taps and
-// transposed channels; weight gradient = per-CTA register accumulation over
-// many voxel lines, one float atomic per weight per CTA.
+// transposed channels; weight gradient = tensor-core products per voxel line
+// (convnet_wgrad.cu), register totals per CTA, one float atomic per weight
+// per CTA (k_conv_wgrad: the same on CUDA cores, with k_conv_simt).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -430,8 +431,14 @@ cudaError_t cnet_backward(CNet* n, cudaStream_t st) {
   float* gnext = n->g1;
   for (int l = 2; l >= 0; l--) {
     float* dw = n->grads + l * (WSZ + C);
-    prof_mark(st, CG_ST_OTHER);
-    k_conv_wgrad<<<cg_sm_count() * 2, T, wgrad_smem, st>>>(n->act[l], g, N, dw, dw + WSZ);
+    cudaError_t ew = cudaErrorNotSupported;
+    if (n->use_tc) ew = conv_wgrad_tc(n->act[l], g, N, dw, dw + WSZ, st);
+    if (ew == cudaErrorNotSupported) {
+      prof_mark(st, CG_ST_OTHER);
+      k_conv_wgrad<<<cg_sm_count() * 2, T, wgrad_smem, st>>>(n->act[l], g, N, dw, dw + WSZ);
+      ew = cudaGetLastError();
+    }
+    if (ew != cudaSuccess) return ew;
     if (l == 0) break;
     // data gradient through layer l, then through the activation of layer l-1
     prof_mark(st, CG_ST_OTHER);

@@ -59,6 +59,10 @@ cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16*
                             float4* out4, cudaStream_t st);
 cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bfloat16* w,
                                   float* out_f, cudaStream_t st);
+// Weight gradient on tensor cores (convnet_wgrad.cu), added to dw [27][16][16]
+// and db [16]; cudaErrorNotSupported when N is no multiple of 16.
+cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, float* dw, float* db,
+                          cudaStream_t st);
 // Device error word of the tensor-core kernels (bounded waits that gave up).
 unsigned conv_tc_error_word();
 // Pipeline of the tensor-core convolutions: -1 by mesh size, 0 two stages,

@@ -1,0 +1,229 @@
+// Weight gradient of the 3x3x3 periodic convolution on tensor cores:
+//   dW[t][ci][co] += sum_v in[v + off(t)][ci] g[v][co],   db[co] += sum_v g[v][co]
+// with bf16 activations and float32 gradients, summed in float32.
+//
+// For one z run of up to 128 voxels of a line (x, y) this is, per tap, a
+// 16 x 16 product over the run, D[ci][co] = A^T g with A the run of the tap's
+// input line: m16n8k16 tensor-core products whose operands ldmatrix.trans
+// reads in place, since both lie in shared memory as [z][channel] (two
+// 8-channel halves of 16-byte rows: any 8 rows are conflict-free, and the z
+// shift of a tap is a start one row on).
+//
+// g keeps its float32 value: it is split into three bf16 terms (8 + 8 + 8
+// bits, each the rounded rest of the one before), which multiply the same
+// bf16 activations exactly, so the products are those of the float32 sum.
+// The leading term and the two small ones accumulate apart, and every run's
+// sums are added to float32 totals in registers (round to nearest), so no
+// tensor-core accumulation chain is longer than 16 products of 16.
+//
+// Nine warps, one per (dx, dy) input line, three dz taps each: the three taps
+// share the g operands, 6 ldmatrix.x4 for 18 products.  A CTA walks runs of
+// consecutive y: the three lines of a row sit in a ring of four slots, so a
+// run loads one new row of three lines, by cp.async
+// while the previous run multiplies.  2 CTAs per SM (80 KB, <= 112
+// registers).
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "convnet.h"
+
+namespace {
+
+constexpr int C = CNET_C;
+constexpr int RUN = 128;                          // voxels of a run at most
+constexpr int ROWS = RUN + 2;
+constexpr int HALF_BYTES = ROWS * 16;
+constexpr int LINE_BYTES = 2 * HALF_BYTES;
+constexpr int RING_BYTES = 12 * LINE_BYTES;       // 4 rows of 3 lines
+constexpr int G_BYTES = RUN * C * 4;              // one run of g, float32
+constexpr int PLANE_BYTES = RUN * C * 2;          // one bf16 term of it
+constexpr int SMEM_BYTES = RING_BYTES + 2 * G_BYTES + 3 * PLANE_BYTES;
+constexpr int THREADS = 288;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                    uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Row y (periodic) of the lines x-1, x, x+1, voxels z0 - 1 .. z0 + len, into a
+// ring slot.
+__device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in, int N, int x,
+                                           int y, int z0, int len, uint32_t slot) {
+  y = y < 0 ? y + N : (y >= N ? y - N : y);
+  const int rows = len + 2;
+  for (int i = threadIdx.x; i < 6 * rows; i += THREADS) {
+    const int h = i & 1, j = (i >> 1) % rows, l = (i >> 1) / rows;
+    int xx = x + l - 1, zz = z0 + j - 1;
+    xx = xx < 0 ? xx + N : (xx >= N ? xx - N : xx);
+    zz = zz < 0 ? zz + N : (zz >= N ? zz - N : zz);
+    cp16(slot + l * LINE_BYTES + h * HALF_BYTES + j * 16,
+         in + (((size_t)xx * N + y) * N + zz) * C + h * 8);
+  }
+}
+
+// Two gradients split into three bf16 pairs: the rounded value, the rounded
+// rest, and what that leaves.
+__device__ __forceinline__ void split2(float2 g, __nv_bfloat162 (&t)[3]) {
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    t[s] = __floats2bfloat162_rn(g.x, g.y);
+    g.x -= __low2float(t[s]);
+    g.y -= __high2float(t[s]);
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, 2)
+    k_conv_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ g, int N,
+                    float* __restrict__ dw, float* __restrict__ db) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  const uint32_t ring = smem_u32(sm);
+  float* const stage = reinterpret_cast<float*>(sm + RING_BYTES);     // [2][RUN][C]
+  uint8_t* const planes = sm + RING_BYTES + 2 * G_BYTES;              // [3][half][RUN] x 16 B
+  const uint32_t pl = smem_u32(planes);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lx = warp / 3, ly = warp % 3;          // this warp's input line (dx + 1, dy + 1)
+  // ldmatrix row addresses: A's four 8x8 blocks are (half 0, z 0-7), (half 1,
+  // z 0-7), (half 0, z 8-15), (half 1, z 8-15); B's (half 0, z 0-7), (half 0,
+  // z 8-15), (half 1, z 0-7), (half 1, z 8-15)
+  const uint32_t offA =
+      (uint32_t)(((lane >> 3) & 1) * HALF_BYTES + ((lane & 7) + ((lane >> 4) & 1) * 8) * 16);
+  const uint32_t offB = (uint32_t)(((lane >> 4) & 1) * (PLANE_BYTES / 2) +
+                                   ((lane & 7) + ((lane >> 3) & 1) * 8) * 16);
+  float tot[3][2][4];
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) tot[d][h][q] = 0.0f;
+  float2 bsum = make_float2(0.0f, 0.0f);           // channels 2 (tid % 8), + 1
+
+  // runs in the order (x, z run, y); a CTA takes a contiguous range
+  const int nz = (N + RUN - 1) / RUN;
+  const int nruns = N * nz * N;
+  const int per = (nruns + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int r1 = min(nruns, ((int)blockIdx.x + 1) * per);
+  for (int r = (int)blockIdx.x * per; r < r1;) {
+    const int y0 = r % N, z0 = (r / N) % nz * RUN, x = r / (N * nz);
+    const int len = min(RUN, N - z0);              // a multiple of 16
+    const int cnt = min(r1 - r, N - y0);           // runs of this (x, z0)
+    const auto load_g = [&](int i) {
+      const float* src = g + (((size_t)x * N + y0 + i) * N + z0) * C;
+      const uint32_t dst = smem_u32(stage + (i & 1) * RUN * C);
+      for (int k = tid; k < len * C / 4; k += THREADS) cp16(dst + 16 * k, src + 4 * k);
+    };
+    for (int j = 0; j < 3; j++)
+      gather_row(in, N, x, y0 - 1 + j, z0, len, ring + j * 3 * LINE_BYTES);
+    load_g(0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = 0; i < cnt; i++) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      // rows i .. i+2 and this run's g are there, and every warp is done with
+      // run i - 1: its row i - 1, the other stage and the planes are free
+      __syncthreads();
+      if (i + 1 < cnt) {
+        gather_row(in, N, x, y0 + i + 2, z0, len, ring + ((i + 3) & 3) * 3 * LINE_BYTES);
+        load_g(i + 1);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const float2* sg = reinterpret_cast<const float2*>(stage + (i & 1) * RUN * C);
+      for (int k = tid; k < len * C / 2; k += THREADS) {
+        const float2 v = sg[k];
+        bsum.x += v.x;
+        bsum.y += v.y;
+        __nv_bfloat162 t[3];
+        split2(v, t);
+        const int z = k >> 3, c = 2 * (k & 7);
+        uint8_t* d = planes + (c >> 3) * (PLANE_BYTES / 2) + z * 16 + (c & 7) * 2;
+#pragma unroll
+        for (int s = 0; s < 3; s++) *reinterpret_cast<__nv_bfloat162*>(d + s * PLANE_BYTES) = t[s];
+      }
+      __syncthreads();
+      const uint32_t a0 = ring + (uint32_t)((((i + ly) & 3) * 3 + lx) * LINE_BYTES) + offA;
+      float hi[3][2][4], lo[3][2][4];
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) hi[d][h][q] = lo[d][h][q] = 0.0f;
+#pragma unroll 1
+      for (int z = 0; z < len; z += 16) {
+        uint32_t a[3][4], b[4];
+#pragma unroll
+        for (int d = 0; d < 3; d++) ldsm4t(a[d], a0 + (uint32_t)((z + d) * 16));
+#pragma unroll
+        for (int s = 2; s >= 0; s--) {
+          ldsm4t(b, pl + (uint32_t)(s * PLANE_BYTES + z * 16) + offB);
+#pragma unroll
+          for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) mma(s ? lo[d][h] : hi[d][h], a[d], b[2 * h], b[2 * h + 1]);
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) tot[d][h][q] += hi[d][h][q] + lo[d][h][q];
+    }
+    r += cnt;
+    __syncthreads();                               // the ring is refilled for the next x
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // accumulator q of a lane: ci = lane / 4 (+ 8 for q >= 2), co = 2 (lane % 4) + q % 2
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int ci = (lane >> 2) + (q >> 1) * 8, co = h * 8 + 2 * (lane & 3) + (q & 1);
+        atomicAdd(dw + ((warp * 3 + d) * C + ci) * C + co, tot[d][h][q]);
+      }
+  // THREADS is a multiple of 8, so a thread kept to one channel pair; the four
+  // lanes of a warp that share it add up first
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+    bsum.x += __shfl_xor_sync(0xffffffffu, bsum.x, o);
+    bsum.y += __shfl_xor_sync(0xffffffffu, bsum.y, o);
+  }
+  if (lane < 8) {
+    atomicAdd(db + 2 * lane, bsum.x);
+    atomicAdd(db + 2 * lane + 1, bsum.y);
+  }
+}
+
+}  // namespace
+
+cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, float* dw, float* db,
+                          cudaStream_t st) {
+  if (N % 16) return cudaErrorNotSupported;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_conv_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  if (attr != cudaSuccess) return attr;
+  const int nruns = N * N * ((N + RUN - 1) / RUN);
+  const int cap = 2 * cg_sm_count();
+  prof_mark(st, CG_ST_OTHER);
+  k_conv_wgrad_tc<<<nruns < cap ? nruns : cap, THREADS, SMEM_BYTES, st>>>(in, g, N, dw, db);
+  return cudaGetLastError();
+}

@@ -156,3 +156,43 @@ def test_line_ring_conv_bit_identical(gpu_lib):
     np.testing.assert_allclose(grads[0], grads[1], rtol=1e-4, atol=1e-6 * np.abs(grads[0]).max())
     assert gpu_lib.cg_net_set_conv_variant(5) != 0
     net.close()
+
+
+@pytest.mark.parametrize("n", [16, 48, 128, 144])
+def test_tensor_core_weight_gradient(gpu_lib, n):
+    """The tensor-core weight gradient of the last layer against float64, on
+    meshes of one and of two z runs per line and with remainders of 16.  The
+    first two layers are set to exact copies (powers of two of non-negative
+    bf16 inputs), so the last layer's input is known bit for bit.  Bound: the
+    float32 sums of a weight take at most 2 x 8 tensor-core steps per run, one
+    addition per run of a CTA and one atomic per CTA, each at most 2^-23 of
+    the sum of |terms|."""
+    from cola_halo_b200.learned import ConvNet
+    rng = np.random.default_rng(n)
+    net = ConvNet(n, seed=1)
+    p = np.zeros(net.nparams, dtype=np.float32)
+    w = p.reshape(3, CR.LAYER)[:, : CR.WSZ].reshape(3, 27, 16, 16)
+    for c in range(16):
+        w[0, 13, c % 2, c] = 2.0 ** -(c // 2)
+        w[1, 13, c, c] = 1.0
+    net.set_params(p)
+    x = CR.bf16(rng.uniform(0, 1, (n, n, n, 2)).astype(np.float32)).numpy()
+    g = (rng.normal(0, 1, (n, n, n, 3)) * 10.0 ** rng.uniform(-6, 0, (n, n, n, 1))).astype(
+        np.float32)
+    got = net.backward_host(x, g).reshape(3, CR.LAYER)[2].astype(np.float64)
+    net.close()
+    act = np.concatenate([x.astype(np.float64) * 2.0 ** -k for k in range(8)], axis=-1)
+    act, g64 = act.reshape(n, n, n, 16), g.astype(np.float64)
+    runs = n * n * -(-n // 128)
+    steps = 16 * -(-runs // 148) + 592
+    for t in range(27):
+        a = np.roll(act, (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2)).reshape(-1, 16)
+        want = a.T @ g64.reshape(-1, 3)
+        size = a.T @ np.abs(g64.reshape(-1, 3))
+        d = got[: CR.WSZ].reshape(27, 16, 16)[t]
+        assert (np.abs(d[:, :3] - want) <= steps * 2.0 ** -23 * size).all(), t
+        assert (d[:, 3:] == 0).all()
+    db = got[CR.WSZ:]
+    size = np.abs(g64).sum(axis=(0, 1, 2))
+    assert (np.abs(db[:3] - g64.sum(axis=(0, 1, 2))) <= 128 * steps * 2.0 ** -23 * size).all()
+    assert (db[3:] == 0).all()

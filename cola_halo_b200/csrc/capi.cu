@@ -737,7 +737,7 @@ extern "C" int cg_net_backward_host(cg_net* h, const float* in2, const float* gr
   for (size_t v = 0; v < nv; v++)
     for (int c = 0; c < 3; c++) g[v * CNET_C + c] = grad3[3 * v + c];
   CG_CHECK(cudaMemcpyAsync(h->n.g0, g.data(), g.size() * 4, cudaMemcpyHostToDevice, h->st), "ul");
-  CG_CHECK(cnet_backward(&h->n, h->st), "backward");
+  CG_CHECK(cnet_backward(&h->n, h->st, false), "backward");
   CG_CHECK(cudaMemcpyAsync(grads, h->n.grads, sizeof(float) * CNET_PARAMS, cudaMemcpyDeviceToHost,
                            h->st), "dl");
   CG_CHECK(cudaStreamSynchronize(h->st), "sync");
@@ -762,9 +762,9 @@ extern "C" int cg_net_train_step(cg_net* h, cg_sim* coarse, cg_sim* fine, float 
   const float* fc[3] = {coarse->ps.f[0], coarse->ps.f[1], coarse->ps.f[2]};
   CG_CHECK(cnet_features(&h->n, coarse->pm.dens, st), "features");
   CG_CHECK(cnet_target(&h->n, x, coarse->ps.n, coarse->L, ff, fc, st), "target");
-  CG_CHECK(cnet_forward(&h->n, st), "forward");
+  CG_CHECK(cnet_forward(&h->n, st, false), "forward");
   CG_CHECK(cnet_loss_grad(&h->n, 1.0 / (double)coarse->ps.n, st), "loss");
-  CG_CHECK(cnet_backward(&h->n, st), "backward");
+  CG_CHECK(cnet_backward(&h->n, st, true), "backward");
   if (lr > 0) CG_CHECK(cnet_adam(&h->n, lr, st), "adam");
   if (loss) {
     CG_CHECK(cudaMemcpyAsync(loss, h->n.loss, sizeof(double), cudaMemcpyDeviceToHost, st), "loss");

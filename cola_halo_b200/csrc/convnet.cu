@@ -48,11 +48,14 @@ __device__ __forceinline__ int wrapi(int i, int N) { return i < 0 ? i + N : (i >
 // ------------------------------------------------------------- SIMT conv
 // out[v][co] = act(b[co] + sum_t sum_ci W[t][ci][co] in[v + off(t)][ci]),
 // off(t) = (t/9 - 1, (t/3)%3 - 1, t%3 - 1); FLIP uses -off(t) and W[t][co][ci]
-// (the data gradient of the forward convolution).
+// (the data gradient of the forward convolution).  gate (NULL: none): the
+// leaky-ReLU backward of the layer below, out *= (gate > 0 ? 1 : 0.1), with
+// that layer's output (same sign as its pre-activation).
 template <bool FLIP>
 __global__ void __launch_bounds__(T) k_conv_simt(const __nv_bfloat16* __restrict__ in, int N,
                                                  const __nv_bfloat16* __restrict__ w,
                                                  const float* __restrict__ bias, int act,
+                                                 const __nv_bfloat16* __restrict__ gate,
                                                  float* __restrict__ out_f,
                                                  __nv_bfloat16* __restrict__ out_b,
                                                  float4* __restrict__ out4) {
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(T) k_conv_simt(const __nv_bfloat16* __restrict
     for (int co = 0; co < C; co++) {
       float a = acc[co];
       if (act) a = a > 0.0f ? a : 0.1f * a;
+      if (gate && __bfloat162float(gate[v * C + co]) <= 0.0f) a *= 0.1f;
       acc[co] = a;
     }
     if (out_f) {
@@ -159,36 +163,42 @@ __global__ void __launch_bounds__(T) k_conv_wgrad(const __nv_bfloat16* __restric
   if (threadIdx.x < C) atomicAdd(db + threadIdx.x, bacc);
 }
 
-// Leaky-ReLU backward in place: g *= (y > 0 ? 1 : 0.1), y the layer output
-// (same sign as the pre-activation).
-__global__ void k_act_back(float* __restrict__ g, const __nv_bfloat16* __restrict__ y, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * T + threadIdx.x; i < n; i += (size_t)gridDim.x * T)
-    if (__bfloat162float(y[i]) <= 0.0f) g[i] *= 0.1f;
-}
-
 __global__ void k_f2b(const float* __restrict__ a, __nv_bfloat16* __restrict__ b, size_t n) {
   for (size_t i = (size_t)blockIdx.x * T + threadIdx.x; i < n; i += (size_t)gridDim.x * T)
     b[i] = __float2bfloat16_rn(a[i]);
 }
 
 // Masked mean-squared-error gradient on the 3 output channels:
-// L = sum_v m_v sum_c (o_vc - r_vc)^2 / sum_v m_v;  g = dL/do.
-__global__ void k_loss(const float* __restrict__ o, const float* __restrict__ r,
-                       const float* __restrict__ m, size_t nv, double inv_msum,
-                       float* __restrict__ g, double* __restrict__ loss) {
+// L = sum_v m_v sum_c (o_vc - r_vc)^2 / sum_v m_v;  g = dL/do, with the
+// residual target r_v = inv_scale (sum of the residuals) / m_v (0 where m_v
+// is 0) formed from the deposit's sums `resid` (x, y, z, mass).  Four threads per
+// voxel write its 16 channels (float32 and bf16) in coalesced runs, 13 of
+// them zero: HBM-bound on the 96 bytes written and 32 read (128^3: 156 us
+// for the 16-channel scalar form with a separate normalisation pass).
+__global__ void k_loss(const float4* __restrict__ o, const float4* __restrict__ resid, size_t nv,
+                       float inv_scale, double inv_msum, float4* __restrict__ g,
+                       uint2* __restrict__ gb, double* __restrict__ loss) {
   double acc = 0.0;
-  for (size_t v = (size_t)blockIdx.x * T + threadIdx.x; v < nv; v += (size_t)gridDim.x * T) {
-    const float mv = m[v];
+  for (size_t i = (size_t)blockIdx.x * T + threadIdx.x; i < 4 * nv; i += (size_t)gridDim.x * T) {
+    float4 gv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if ((i & 3) == 0) {
+      const float4 ov = o[i >> 2], rs = resid[i >> 2];
+      const float mv = rs.w;
+      const float oc[3] = {ov.x, ov.y, ov.z}, rc[3] = {rs.x, rs.y, rs.z};
+      float gc[3];
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      float gv = 0.0f;
-      if (c < 3) {
-        const float d = o[v * C + c] - r[v * 3 + c];
+      for (int c = 0; c < 3; c++) {
+        const float d = oc[c] - (mv > 0 ? __fmul_rn(rc[c] / mv, inv_scale) : 0.0f);
         acc += (double)mv * d * d;
-        gv = (float)(2.0 * inv_msum) * mv * d;
+        gc[c] = (float)(2.0 * inv_msum) * mv * d;
       }
-      g[v * C + c] = gv;
+      gv = make_float4(gc[0], gc[1], gc[2], 0.0f);
     }
+    g[i] = gv;
+    const __nv_bfloat162 b0 = __floats2bfloat162_rn(gv.x, gv.y);
+    const __nv_bfloat162 b1 = __floats2bfloat162_rn(gv.z, gv.w);
+    gb[i] = make_uint2(*reinterpret_cast<const unsigned*>(&b0),
+                       *reinterpret_cast<const unsigned*>(&b1));
   }
   for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc * inv_msum);
@@ -235,39 +245,41 @@ __global__ void k_potential(float2* __restrict__ s, int N) {
   }
 }
 
+// Periodic cells (lower, upper) and fraction of one coordinate in mesh units.
+struct Axis { int i0, i1; float d; };
+__device__ __forceinline__ Axis axis_cells(float X, int N) {
+  const int i = (int)floorf(X);
+  Axis a;
+  a.d = X - i;
+  a.i0 = i;
+  if ((unsigned)i >= (unsigned)N) a.i0 = (i % N + N) % N;   // outside the box
+  a.i1 = a.i0 + 1 == N ? 0 : a.i0 + 1;
+  return a;
+}
+
 // CIC deposit of per-particle values (3 components) and mass on a periodic
-// coarse mesh (plain periodic CIC: the residual target, not the PM density).
+// coarse mesh (plain periodic CIC: the residual target, not the PM density):
+// one 16-byte atomic per corner for the three residuals and the mass (128^3
+// particles: 346 us with four scalar atomics per corner).
 __global__ void k_deposit_resid(const float* __restrict__ x0, const float* __restrict__ x1,
                                 const float* __restrict__ x2, const float* __restrict__ fa0,
                                 const float* __restrict__ fa1, const float* __restrict__ fa2,
                                 const float* __restrict__ fb0, const float* __restrict__ fb1,
                                 const float* __restrict__ fb2, long long n, int N, float scale,
-                                float* __restrict__ r, float* __restrict__ m) {
+                                float4* __restrict__ r) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T) {
-    const float X = x0[i] * scale, Y = x1[i] * scale, Z = x2[i] * scale;
-    const int ix = (int)floorf(X), iy = (int)floorf(Y), iz = (int)floorf(Z);
-    const float dx = X - ix, dy = Y - iy, dz = Z - iz;
+    const Axis x = axis_cells(x0[i] * scale, N), y = axis_cells(x1[i] * scale, N),
+               z = axis_cells(x2[i] * scale, N);
     const float res[3] = {fa0[i] - fb0[i], fa1[i] - fb1[i], fa2[i] - fb2[i]};
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const int ax = c >> 2, ay = (c >> 1) & 1, az = c & 1;
-      const float w = (ax ? dx : 1 - dx) * (ay ? dy : 1 - dy) * (az ? dz : 1 - dz);
-      const int xx = ((ix + ax) % N + N) % N, yy = ((iy + ay) % N + N) % N,
-                zz = ((iz + az) % N + N) % N;
-      const size_t v = ((size_t)xx * N + yy) * N + zz;
-      atomicAdd(m + v, w);
-#pragma unroll
-      for (int a = 0; a < 3; a++) atomicAdd(r + 3 * v + a, w * res[a]);
+      const float w = (ax ? x.d : 1 - x.d) * (ay ? y.d : 1 - y.d) * (az ? z.d : 1 - z.d);
+      const size_t v = ((size_t)(ax ? x.i1 : x.i0) * N + (ay ? y.i1 : y.i0)) * N +
+                       (az ? z.i1 : z.i0);
+      atomicAdd(r + v, make_float4(w * res[0], w * res[1], w * res[2], w));
     }
-  }
-}
-
-__global__ void k_normalise_resid(float* __restrict__ r, const float* __restrict__ m, size_t nv,
-                                  float inv_scale) {
-  for (size_t v = (size_t)blockIdx.x * T + threadIdx.x; v < nv; v += (size_t)gridDim.x * T) {
-    const float mv = m[v];
-    for (int a = 0; a < 3; a++) r[3 * v + a] = mv > 0 ? r[3 * v + a] / mv * inv_scale : 0.0f;
   }
 }
 
@@ -278,17 +290,15 @@ __global__ void k_apply(const float* __restrict__ x0, const float* __restrict__ 
                         float* __restrict__ f1, float* __restrict__ f2) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T) {
-    const float X = x0[i] * scale, Y = x1[i] * scale, Z = x2[i] * scale;
-    const int ix = (int)floorf(X), iy = (int)floorf(Y), iz = (int)floorf(Z);
-    const float dx = X - ix, dy = Y - iy, dz = Z - iz;
+    const Axis x = axis_cells(x0[i] * scale, N), y = axis_cells(x1[i] * scale, N),
+               z = axis_cells(x2[i] * scale, N);
     float acc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const int ax = c >> 2, ay = (c >> 1) & 1, az = c & 1;
-      const float w = (ax ? dx : 1 - dx) * (ay ? dy : 1 - dy) * (az ? dz : 1 - dz);
-      const int xx = ((ix + ax) % N + N) % N, yy = ((iy + ay) % N + N) % N,
-                zz = ((iz + az) % N + N) % N;
-      const float4 ov = o[((size_t)xx * N + yy) * N + zz];
+      const float w = (ax ? x.d : 1 - x.d) * (ay ? y.d : 1 - y.d) * (az ? z.d : 1 - z.d);
+      const float4 ov = __ldg(o + ((size_t)(ax ? x.i1 : x.i0) * N + (ay ? y.i1 : y.i0)) * N +
+                              (az ? z.i1 : z.i0));
       acc[0] += w * ov.x;
       acc[1] += w * ov.y;
       acc[2] += w * ov.z;
@@ -323,8 +333,7 @@ cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed) {
   CN_TRY(cudaMalloc(&n->g0, sizeof(float) * nv * C));
   CN_TRY(cudaMalloc(&n->g1, sizeof(float) * nv * C));
   CN_TRY(cudaMalloc(&n->gb, sizeof(__nv_bfloat16) * nv * C));
-  CN_TRY(cudaMalloc(&n->target, sizeof(float) * nv * 3));
-  CN_TRY(cudaMalloc(&n->mass, sizeof(float) * nv));
+  CN_TRY(cudaMalloc(&n->resid, sizeof(float4) * nv));
   CN_TRY(cudaMalloc(&n->loss, sizeof(double)));
   CN_TRY(cudaMalloc(&n->phi, sizeof(float) * nv));
   CN_TRY(cudaMalloc(&n->spec, sizeof(float2) * (size_t)(N / 2 + 1) * N * N));
@@ -370,7 +379,7 @@ void cnet_free(CNet* n) {
   cudaFree(n->trainable); cudaFree(n->wb);
   for (int l = 0; l < 3; l++) cudaFree(n->act[l]);
   cudaFree(n->out); cudaFree(n->out4); cudaFree(n->g0); cudaFree(n->g1); cudaFree(n->gb);
-  cudaFree(n->target); cudaFree(n->mass); cudaFree(n->loss); cudaFree(n->phi);
+  cudaFree(n->resid); cudaFree(n->loss); cudaFree(n->phi);
   cudaFree(n->spec);
   mesh_fft_free(&n->fft);
   memset(n, 0, sizeof(*n));
@@ -386,7 +395,8 @@ cudaError_t cnet_sync_bf16(CNet* n, cudaStream_t st) {
 
 static cudaError_t conv(const CNet* n, const __nv_bfloat16* in, const __nv_bfloat16* w,
                         const float* bias, int act, float* of, __nv_bfloat16* ob, bool flip,
-                        cudaStream_t st, float4* o4 = nullptr) {
+                        cudaStream_t st, float4* o4 = nullptr,
+                        const __nv_bfloat16* gate = nullptr) {
   const int N = n->N;
   const long long nv = (long long)N * N * N;
   if (n->use_tc && !flip) {
@@ -394,14 +404,14 @@ static cudaError_t conv(const CNet* n, const __nv_bfloat16* in, const __nv_bfloa
     if (e != cudaErrorNotSupported) return e;
   }
   if (n->use_tc && flip) {
-    cudaError_t e = conv_tc_backward_data(in, N, w, of, st);
+    cudaError_t e = conv_tc_backward_data(in, N, w, gate, of, ob, st);
     if (e != cudaErrorNotSupported) return e;
   }
   prof_mark(st, CG_ST_OTHER);
   if (flip)
-    k_conv_simt<true><<<grid_for(nv), T, 0, st>>>(in, N, w, bias, act, of, ob, o4);
+    k_conv_simt<true><<<grid_for(nv), T, 0, st>>>(in, N, w, bias, act, gate, of, ob, o4);
   else
-    k_conv_simt<false><<<grid_for(nv), T, 0, st>>>(in, N, w, bias, act, of, ob, o4);
+    k_conv_simt<false><<<grid_for(nv), T, 0, st>>>(in, N, w, bias, act, gate, of, ob, o4);
   return cudaGetLastError();
 }
 
@@ -416,8 +426,11 @@ cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full) {
 }
 
 // Backward from g0 = dL/dout (3 output channels, float [v][16]); parameter
-// gradients into n->grads.
-cudaError_t cnet_backward(CNet* n, cudaStream_t st) {
+// gradients into n->grads.  Each data gradient comes out of its convolution
+// with the activation below applied, in float32 for the weight gradient and in
+// bf16 for the next convolution (the second bf16 buffer is the memory of the
+// [v][16] output, which nothing reads once its gradient is known).
+cudaError_t cnet_backward(CNet* n, cudaStream_t st, bool gb_ready) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
   const size_t wgrad_smem = sizeof(float) * (9 * (N + 2) * C + N * C);
@@ -429,6 +442,12 @@ cudaError_t cnet_backward(CNet* n, cudaStream_t st) {
   cudaMemsetAsync(n->grads, 0, sizeof(float) * CNET_PARAMS, st);
   float* g = n->g0;
   float* gnext = n->g1;
+  __nv_bfloat16* gb = n->gb;
+  __nv_bfloat16* gbnext = reinterpret_cast<__nv_bfloat16*>(n->out);
+  if (!gb_ready) {
+    prof_mark(st, CG_ST_OTHER);
+    k_f2b<<<grid_for((long long)nv * C), T, 0, st>>>(g, gb, nv * C);
+  }
   for (int l = 2; l >= 0; l--) {
     float* dw = n->grads + l * (WSZ + C);
     cudaError_t ew = cudaErrorNotSupported;
@@ -441,13 +460,12 @@ cudaError_t cnet_backward(CNet* n, cudaStream_t st) {
     if (ew != cudaSuccess) return ew;
     if (l == 0) break;
     // data gradient through layer l, then through the activation of layer l-1
-    prof_mark(st, CG_ST_OTHER);
-    k_f2b<<<grid_for((long long)nv * C), T, 0, st>>>(g, n->gb, nv * C);
-    cudaError_t e = conv(n, n->gb, n->wb + l * WSZ, nullptr, 0, gnext, nullptr, true, st);
+    // (the first layer's gradient feeds its weights alone)
+    cudaError_t e = conv(n, gb, n->wb + l * WSZ, nullptr, 0, gnext, l > 1 ? gbnext : nullptr,
+                         true, st, nullptr, n->act[l]);
     if (e != cudaSuccess) return e;
-    prof_mark(st, CG_ST_OTHER);
-    k_act_back<<<grid_for((long long)nv * C), T, 0, st>>>(gnext, n->act[l], nv * C);
     float* tmp = g; g = gnext; gnext = tmp;
+    __nv_bfloat16* tb = gb; gb = gbnext; gbnext = tb;
   }
   return cudaGetLastError();
 }
@@ -456,8 +474,9 @@ cudaError_t cnet_loss_grad(CNet* n, double inv_msum, cudaStream_t st) {
   const size_t nv = (size_t)n->N * n->N * n->N;
   cudaMemsetAsync(n->loss, 0, sizeof(double), st);
   prof_mark(st, CG_ST_OTHER);
-  k_loss<<<grid_for((long long)nv), T, 0, st>>>(n->out, n->target, n->mass, nv, inv_msum, n->g0,
-                                                n->loss);
+  k_loss<<<grid_for(4 * (long long)nv), T, 0, st>>>(n->out4, n->resid, nv, 1.0f / n->out_scale,
+                                                    inv_msum, reinterpret_cast<float4*>(n->g0),
+                                                    reinterpret_cast<uint2*>(n->gb), n->loss);
   return cudaGetLastError();
 }
 
@@ -491,15 +510,11 @@ cudaError_t cnet_target(CNet* n, const float* const x[3], long long np, float bo
                         cudaStream_t st) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
-  cudaMemsetAsync(n->target, 0, sizeof(float) * nv * 3, st);
-  cudaMemsetAsync(n->mass, 0, sizeof(float) * nv, st);
+  cudaMemsetAsync(n->resid, 0, sizeof(float4) * nv, st);
   prof_mark(st, CG_ST_OTHER);
   k_deposit_resid<<<grid_for(np), T, 0, st>>>(x[0], x[1], x[2], f_fine[0], f_fine[1], f_fine[2],
                                               f_coarse[0], f_coarse[1], f_coarse[2], np, N,
-                                              (float)N / boxsize, n->target, n->mass);
-  prof_mark(st, CG_ST_OTHER);
-  k_normalise_resid<<<grid_for((long long)nv), T, 0, st>>>(n->target, n->mass, nv,
-                                                           1.0f / n->out_scale);
+                                              (float)N / boxsize, n->resid);
   return cudaGetLastError();
 }
 

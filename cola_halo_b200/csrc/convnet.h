@@ -28,8 +28,8 @@ struct CNet {
   float* g0;                   // gradient buffers [v][16]
   float* g1;
   __nv_bfloat16* gb;           // bf16 copy of the gradient fed to the data-gradient conv
-  float* target;               // residual target [v][3] (in output units)
-  float* mass;                 // deposited mass [v]
+                               //   (a second one reuses out's memory, cnet_backward)
+  float4* resid;               // deposited residual sums and mass [v] (x, y, z, mass)
   double* loss;
   float* phi;                  // potential [v]
   float2* spec;                // half spectrum scratch
@@ -43,8 +43,10 @@ cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st);
 // full: also write the [v][16] output that the loss and the host API read
 // (the packed out4 is always written)
 cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true);
+// loss and dL/dout (g0 and its bf16 copy gb) from out4 and the residual sums
 cudaError_t cnet_loss_grad(CNet* n, double inv_msum, cudaStream_t st);
-cudaError_t cnet_backward(CNet* n, cudaStream_t st);
+// gb_ready: gb holds g0 in bf16 already
+cudaError_t cnet_backward(CNet* n, cudaStream_t st, bool gb_ready);
 cudaError_t cnet_adam(CNet* n, float lr, cudaStream_t st);
 cudaError_t cnet_target(CNet* n, const float* const x[3], long long np, float boxsize,
                         const float* const f_fine[3], const float* const f_coarse[3],
@@ -57,8 +59,11 @@ cudaError_t cnet_apply(const CNet* n, const float* const x[3], long long np, flo
 cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
                             const float* bias, int act, float* out_f, __nv_bfloat16* out_b,
                             float4* out4, cudaStream_t st);
+// gate (or NULL): the layer below's output, whose leaky-ReLU backward scales
+// the result; out_b (or NULL): a bf16 copy
 cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bfloat16* w,
-                                  float* out_f, cudaStream_t st);
+                                  const __nv_bfloat16* gate, float* out_f, __nv_bfloat16* out_b,
+                                  cudaStream_t st);
 // Weight gradient on tensor cores (convnet_wgrad.cu), added to dw [27][16][16]
 // and db [16]; cudaErrorNotSupported when N is no multiple of 16.
 cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, float* dw, float* db,

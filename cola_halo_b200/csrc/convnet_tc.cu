@@ -108,8 +108,9 @@ __device__ __forceinline__ void gather(const __nv_bfloat16* __restrict__ in, int
 template <bool FLIP, int STAGES, int CPS>
 __global__ void __launch_bounds__(THREADS, CPS)
     k_conv_tc(const __nv_bfloat16* __restrict__ in, int N, const __nv_bfloat16* __restrict__ w,
-              const float* __restrict__ bias, int act, float* __restrict__ out_f,
-              __nv_bfloat16* __restrict__ out_b, float4* __restrict__ out4) {
+              const float* __restrict__ bias, int act, const __nv_bfloat16* __restrict__ gate,
+              float* __restrict__ out_f, __nv_bfloat16* __restrict__ out_b,
+              float4* __restrict__ out4) {
   extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* const stage0 = sm;
   uint8_t* const stage1 = sm + (STAGES - 1) * STAGE_BYTES;
@@ -212,6 +213,7 @@ __global__ void __launch_bounds__(THREADS, CPS)
       for (int c = 0; c < C; c++) {
         float a = __uint_as_float(r[c]) + (bias ? bias[c] : 0.0f);
         if (act) a = a > 0.0f ? a : 0.1f * a;
+        if (gate && __bfloat162float(gate[v * C + c]) <= 0.0f) a *= 0.1f;
         o[c] = a;
       }
       if (out_f) {
@@ -274,8 +276,9 @@ __device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in,
 template <bool FLIP>
 __global__ void __launch_bounds__(THREADS, 3)
     k_conv_ring(const __nv_bfloat16* __restrict__ in, int N, const __nv_bfloat16* __restrict__ w,
-                const float* __restrict__ bias, int act, float* __restrict__ out_f,
-                __nv_bfloat16* __restrict__ out_b, float4* __restrict__ out4) {
+                const float* __restrict__ bias, int act, const __nv_bfloat16* __restrict__ gate,
+                float* __restrict__ out_f, __nv_bfloat16* __restrict__ out_b,
+                float4* __restrict__ out4) {
   extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* const ring = sm;
   uint8_t* sB = sm + RING_BYTES;
@@ -367,6 +370,7 @@ __global__ void __launch_bounds__(THREADS, 3)
         for (int c = 0; c < C; c++) {
           float a = __uint_as_float(r[c]) + (bias ? bias[c] : 0.0f);
           if (act) a = a > 0.0f ? a : 0.1f * a;
+          if (gate && __bfloat162float(gate[v * C + c]) <= 0.0f) a *= 0.1f;
           o[c] = a;
         }
         if (out_f) {
@@ -403,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 3)
 
 template <bool FLIP>
 cudaError_t launch_ring(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
-                        const float* bias, int act, float* of, __nv_bfloat16* ob, float4* o4,
+                        const float* bias, int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4,
                         cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
@@ -415,13 +419,13 @@ cudaError_t launch_ring(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
   }
   const int grid = 3 * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);
-  k_conv_ring<FLIP><<<grid, THREADS, ring_smem_bytes(), st>>>(in, N, w, bias, act, of, ob, o4);
+  k_conv_ring<FLIP><<<grid, THREADS, ring_smem_bytes(), st>>>(in, N, w, bias, act, gate, of, ob, o4);
   return cudaGetLastError();
 }
 
 template <bool FLIP, int STAGES, int CPS>
 cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const float* bias,
-                     int act, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
+                     int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_tc<FLIP, STAGES, CPS>,
@@ -435,7 +439,7 @@ cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, con
   const int grid = ntiles < CPS * sms ? ntiles : CPS * sms;
   prof_mark(st, CG_ST_OTHER);
   k_conv_tc<FLIP, STAGES, CPS><<<grid, THREADS, smem_bytes(STAGES), st>>>(in, N, w, bias, act,
-                                                                         of, ob, o4);
+                                                                         gate, of, ob, o4);
   return cudaGetLastError();
 }
 
@@ -459,12 +463,12 @@ int conv_variant(int N) {
 
 template <bool FLIP>
 cudaError_t launch(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const float* bias,
-                   int act, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
+                   int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
   if (N < TILE_M || N % TILE_M) return cudaErrorNotSupported;
   const int v = conv_variant(N);
-  if (v == 2) return launch_ring<FLIP>(in, N, w, bias, act, of, ob, o4, st);
-  if (v == 1) return launch_v<FLIP, 1, 4>(in, N, w, bias, act, of, ob, o4, st);
-  return launch_v<FLIP, 2, 2>(in, N, w, bias, act, of, ob, o4, st);
+  if (v == 2) return launch_ring<FLIP>(in, N, w, bias, act, gate, of, ob, o4, st);
+  if (v == 1) return launch_v<FLIP, 1, 4>(in, N, w, bias, act, gate, of, ob, o4, st);
+  return launch_v<FLIP, 2, 2>(in, N, w, bias, act, gate, of, ob, o4, st);
 }
 
 }  // namespace
@@ -472,12 +476,13 @@ cudaError_t launch(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const
 cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
                             const float* bias, int act, float* out_f, __nv_bfloat16* out_b,
                             float4* out4, cudaStream_t st) {
-  return launch<false>(in, N, w, bias, act, out_f, out_b, out4, st);
+  return launch<false>(in, N, w, bias, act, nullptr, out_f, out_b, out4, st);
 }
 
 cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bfloat16* w,
-                                  float* out_f, cudaStream_t st) {
-  return launch<true>(g, N, w, nullptr, 0, out_f, nullptr, nullptr, st);
+                                  const __nv_bfloat16* gate, float* out_f, __nv_bfloat16* out_b,
+                                  cudaStream_t st) {
+  return launch<true>(g, N, w, nullptr, 0, gate, out_f, out_b, nullptr, st);
 }
 
 int conv_tc_set_variant(int v) {

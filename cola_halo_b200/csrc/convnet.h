@@ -71,5 +71,5 @@ cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, float*
 // Device error word of the tensor-core kernels (bounded waits that gave up).
 unsigned conv_tc_error_word();
 // Pipeline of the tensor-core convolutions: -1 by mesh size, 0 two stages,
-// 1 one stage, 2 the line ring (128^3 only).  -1 returned on a bad value.
+// 1 one stage, 2 the sweep along y (the default).  -1 returned on a bad value.
 int conv_tc_set_variant(int v);

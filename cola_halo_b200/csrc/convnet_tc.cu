@@ -12,6 +12,7 @@
 // buffer started dz rows further on: the z shift costs no copy.  B_t are the
 // tap weights in the no-swizzle core-matrix layout (LBO 128 B, SBO 256 B).
 //
+// k_conv_sweep, the default, reuses the lines along y (below).  In k_conv_tc
 // CTAs are persistent over tiles, 4 per SM with one line buffer each: one
 // thread issues the tile's 27 MMAs (M=128, N=16, K=16), tcgen05.commit
 // arrives on an mbarrier, the cp.async gather of the next tile starts, and
@@ -165,12 +166,14 @@ __global__ void __launch_bounds__(THREADS, CPS)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0) {
-      for (int t = 0; t < 27; t++) {
-        // tap (dx, dy, dz): line t / 3, started dz = t % 3 rows on
+      for (int k = 0; k < 27; k++) {
+        // tap (dx, dy, dz), in the order dy, dx, dz (k_conv_sweep's): line t / 3,
+        // started dz = t % 3 rows on
+        const int t = (k / 3 % 3) * 9 + (k / 9) * 3 + k % 3;
         const uint64_t da =
             umma_desc(smem_u32(s + (t / 3) * LINE_BYTES + (t % 3) * 16), HALF_BYTES, 128);
         const uint64_t db = umma_desc(smem_u32(sB + t * B_BYTES), 128, 256);
-        const uint32_t acc = t > 0 ? 1u : 0u;
+        const uint32_t acc = k > 0 ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
@@ -244,155 +247,222 @@ __global__ void __launch_bounds__(THREADS, CPS)
                  : "memory");
 }
 
-// The same convolution for a 128^3 mesh (one tile per line), with the input
-// lines reused along y.  A CTA walks a contiguous run of lines (x, y),
-// (x, y+1), ...: tile (x, y) reads the lines (x-1..x+1, y-1..y+1), so the
-// next tile needs only the three lines of row y+2.  The rows sit in a ring
-// of four slots of three lines (x-1, x, x+1); row j of the run goes to slot
-// j mod 4 in its own cp.async group.  While tile i's epilogue runs, the
-// slot that tile i's row y-1 used is refilled with row y+3, so a tile
-// waits for one new row of 12 KB instead of gathering 37 KB.  The MMAs,
-// their order and their operands are those of k_conv_tc: bit-identical
-// output.  3 CTAs per SM (62 KB each).
-constexpr int RING_BYTES = 12 * LINE_BYTES;      // 49920
-__host__ __device__ constexpr int ring_smem_bytes() { return RING_BYTES + 27 * B_BYTES + 64; }
+// The same convolution, sweeping along y with every input row used once.  A
+// CTA owns the z tiles (x0, y, z0) and (x0 + 1, y, z0) for a run of y.  Input
+// row y' (the four lines x0-1 .. x0+2) adds to the outputs of rows y'-1, y'
+// and y'+1 at once: one MMA of M = 128 voxels, N = 48 columns (the three
+// rows' 16 output channels, with the weights of dy = +1, 0, -1) and K = 16
+// per output line, dx and dz.  The A operand (128 rows of 32 bytes from shared
+// memory) is what an MMA of N <= 64 waits for, so this does 9 reads of it per
+// output line where one tile at a time (N = 16) needs 27; and the lines come
+// from L2 twice per output line instead of three (k_conv_ring before this) or
+// nine times.
+//
+// The three accumulators of an output column x sit in tensor-memory slots o
+// mod 3 (o the output row counted from the run's start).  The rows y'-1, y',
+// y'+1 take every slot once, in a cyclic order that moves by one per row, so
+// the B operand of a tap pair (dx, dz) is stored as five blocks of 16 channels, dy
+// = +1, 0, -1, +1, 0, and the row's window of three starts at block 2, 1 or 0.
+// After a row's MMAs the slot of output o = i - 2 (i the row) is complete: its
+// threads read it, set it to zero for output o + 3 and hand the tensor memory
+// back; bias, activation and stores then run beside the next row's MMAs.  The
+// next row's lines arrive by cp.async meanwhile.  4 CTAs per SM (57 KB, 128
+// tensor-memory columns each).
+//
+// Per output the products are added in the order dy, dx, dz, as in k_conv_tc:
+// bit-identical.
+constexpr int SROW_BYTES = 4 * LINE_BYTES;       // four lines of one input row
+constexpr int SB_BYTES = 5 * B_BYTES;            // five 16-channel blocks per (dx, dz)
+constexpr int SLOTS = 3;
+__host__ __device__ constexpr int sweep_smem_bytes() {
+  return 2 * SROW_BYTES + 9 * SB_BYTES + 64;
+}
+constexpr int SWEEP_CPS = 4;
+constexpr uint32_t kIdesc48 = (kIdesc & ~(0x3Fu << 17)) | ((48u >> 3) << 17);
 
-// cp.async of row y (periodic) of the lines x-1, x, x+1 into ring slot `slot`
-// (line dx+1 of the slot; rows z = -1 .. 128, two 8-channel halves).
-__device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in, int N, int x,
-                                           int y, uint8_t* slot) {
+// cp.async of row y (periodic) of the lines x0-1 .. x0+2, voxels z0 - 1 ..
+// z0 + 128, into a row buffer.
+__device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in, int N, int x0,
+                                           int y, int z0, uint8_t* row) {
   y = y < 0 ? y + N : (y >= N ? y - N : y);
-  for (int i = threadIdx.x; i < 3 * ROWS * 2; i += THREADS) {
+  for (int i = threadIdx.x; i < 4 * ROWS * 2; i += THREADS) {
     const int h = i & 1, j = (i >> 1) % ROWS, L = (i >> 1) / ROWS;
-    int xx = x + L - 1, zz = j - 1;
+    int xx = x0 + L - 1, zz = z0 + j - 1;
     xx = xx < 0 ? xx + N : (xx >= N ? xx - N : xx);
     zz = zz < 0 ? zz + N : (zz >= N ? zz - N : zz);
     const __nv_bfloat16* src = in + (((size_t)xx * N + y) * N + zz) * C + h * 8;
-    const uint32_t dst = smem_u32(slot + L * LINE_BYTES + h * HALF_BYTES + j * 16);
+    const uint32_t dst = smem_u32(row + L * LINE_BYTES + h * HALF_BYTES + j * 16);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
   }
 }
 
+// 16 accumulator columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t a) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(a));
+}
+__device__ __forceinline__ void tmem_zero16(uint32_t a) {
+  const uint32_t z = 0;
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+      :: "r"(a), "r"(z) : "memory");
+}
+
+// Bias, activation or gate, and the stores of one voxel's 16 channels.
+__device__ __forceinline__ void store_voxel(const uint32_t (&r)[16], size_t v,
+                                            const float* __restrict__ bias, int act,
+                                            const __nv_bfloat16* __restrict__ gate,
+                                            float* __restrict__ out_f,
+                                            __nv_bfloat16* __restrict__ out_b,
+                                            float4* __restrict__ out4) {
+  float o[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    float a = __uint_as_float(r[c]) + (bias ? bias[c] : 0.0f);
+    if (act) a = a > 0.0f ? a : 0.1f * a;
+    o[c] = a;
+  }
+  if (gate) {
+    uint4 gq[2] = {reinterpret_cast<const uint4*>(gate + v * C)[0],
+                   reinterpret_cast<const uint4*>(gate + v * C)[1]};
+    const __nv_bfloat16* gv = reinterpret_cast<const __nv_bfloat16*>(gq);
+#pragma unroll
+    for (int c = 0; c < C; c++)
+      if (__bfloat162float(gv[c]) <= 0.0f) o[c] *= 0.1f;
+  }
+  if (out_f) {
+    float4* d = reinterpret_cast<float4*>(out_f + v * C);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      d[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+  }
+  if (out_b) {
+    __nv_bfloat16 hb[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) hb[c] = __float2bfloat16_rn(o[c]);
+    uint4* d = reinterpret_cast<uint4*>(out_b + v * C);
+    d[0] = *reinterpret_cast<const uint4*>(&hb[0]);
+    d[1] = *reinterpret_cast<const uint4*>(&hb[8]);
+  }
+  if (out4) out4[v] = make_float4(o[0], o[1], o[2], o[3]);
+}
+
 template <bool FLIP>
-__global__ void __launch_bounds__(THREADS, 3)
-    k_conv_ring(const __nv_bfloat16* __restrict__ in, int N, const __nv_bfloat16* __restrict__ w,
-                const float* __restrict__ bias, int act, const __nv_bfloat16* __restrict__ gate,
-                float* __restrict__ out_f, __nv_bfloat16* __restrict__ out_b,
-                float4* __restrict__ out4) {
+__global__ void __launch_bounds__(THREADS, SWEEP_CPS)
+    k_conv_sweep(const __nv_bfloat16* __restrict__ in, int N, const __nv_bfloat16* __restrict__ w,
+                 const float* __restrict__ bias, int act, const __nv_bfloat16* __restrict__ gate,
+                 float* __restrict__ out_f, __nv_bfloat16* __restrict__ out_b,
+                 float4* __restrict__ out4) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  uint8_t* const ring = sm;
-  uint8_t* sB = sm + RING_BYTES;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sB + 27 * B_BYTES);
+  uint8_t* sB = sm + 2 * SROW_BYTES;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sB + 9 * SB_BYTES);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 :: "r"(smem_u32(tslot)), "r"(32) : "memory");
+                 :: "r"(smem_u32(tslot)), "r"(128) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(mbar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = tid; i < 27 * C * C; i += THREADS) {
-    const int t = i / (C * C), n = (i / C) % C, k = i % C;
-    const __nv_bfloat16 v = FLIP ? w[((26 - t) * C + n) * C + k]
-                                 : w[(t * C + k) * C + n];
-    *reinterpret_cast<__nv_bfloat16*>(sB + t * B_BYTES + cm_off(n, k)) = v;
+  // B of (dx, dz): blocks dy = +1, 0, -1, +1, 0; element (n = output channel,
+  // k = input channel) of tap t
+  for (int i = tid; i < 9 * 5 * C * C; i += THREADS) {
+    const int k = i % C, n = i / C % C, b = i / (C * C) % 5, p = i / (5 * C * C);
+    const int t = (p / 3) * 9 + (2 - b % 3) * 3 + p % 3;
+    const __nv_bfloat16 v = FLIP ? w[((26 - t) * C + n) * C + k] : w[(t * C + k) * C + n];
+    *reinterpret_cast<__nv_bfloat16*>(sB + p * SB_BYTES + cm_off(b * C + n, k)) = v;
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
+  const uint32_t mine = tmem + ((uint32_t)(warp * 32) << 16);
   const uint32_t bar = smem_u32(mbar);
-  const int nlines = N * N;
-  const int per = (nlines + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int l1 = min(nlines, (int)blockIdx.x * per + per);
+  // output rows in the order (x pair, z tile, y); a CTA takes a contiguous range
+  const int nz = N / TILE_M;
+  const int nrows = N / 2 * nz * N;
+  const int per = (nrows + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int l1 = min(nrows, ((int)blockIdx.x + 1) * per);
   uint32_t phase = 0;
   bool ok = true;
   for (int l = (int)blockIdx.x * per; l < l1 && ok;) {
-    const int x = l / N, y0 = l % N;
-    const int run = min(l1 - l, N - y0);          // tiles of this x in the CTA's range
-    // rows y0-1 .. y0+2 (loaded rows 0..3) into slots 0..3, one group each
-    for (int j = 0; j < 4; j++) {
-      if (j <= run + 1) gather_row(in, N, x, y0 - 1 + j, ring + j * 3 * LINE_BYTES);
+    const int y0 = l % N, z0 = (l / N) % nz * TILE_M, x0 = l / (N * nz) * 2;
+    const int run = min(l1 - l, N - y0);
+    gather_row(in, N, x0, y0 - 1, z0, sm);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int q = 0; q < 2 * SLOTS; q++) tmem_zero16(mine + 16 * q);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    uint32_t r[2][16];
+    // row i holds y' = y0 - 1 + i
+    for (int i = 0; i <= run + 1 && ok; i++) {
+      // the other buffer's row i - 1 has been multiplied
+      if (i <= run) gather_row(in, N, x0, y0 + i, z0, sm + ((i + 1) & 1) * SROW_BYTES);
       asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int i = 0; i < run && ok; i++) {
-      // loaded rows i .. i+2 complete (row i+3 may still be in flight)
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (tid == 0) {
-        for (int t = 0; t < 27; t++) {
-          // tap t: line L = t / 3 = (dx+1) * 3 + (dy+1), started dz = t % 3 rows on
-          const int L = t / 3;
-          const uint8_t* line = ring + (((i + L % 3) & 3) * 3 + L / 3) * LINE_BYTES;
-          const uint64_t da = umma_desc(smem_u32(line + (t % 3) * 16), HALF_BYTES, 128);
-          const uint64_t db = umma_desc(smem_u32(sB + t * B_BYTES), 128, 256);
-          const uint32_t acc = t > 0 ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-              :: "r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(acc)
-              : "memory");
+        const uint32_t row = smem_u32(sm + (i & 1) * SROW_BYTES);
+        const uint32_t b0 = smem_u32(sB) + (uint32_t)((2 - i % 3) * B_BYTES);
+        for (int xo = 0; xo < 2; xo++) {
+          for (int p = 0; p < 9; p++) {
+            // (dx, dz) = (p / 3, p % 3): line xo + dx, started dz rows on
+            const uint64_t da = umma_desc(
+                row + (uint32_t)((xo + p / 3) * LINE_BYTES + (p % 3) * 16), HALF_BYTES, 128);
+            const uint64_t db = umma_desc(b0 + (uint32_t)(p * SB_BYTES), 128, 256);
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                :: "r"(tmem + (uint32_t)(16 * SLOTS * xo)), "l"(da), "l"(db), "r"(kIdesc48),
+                   "r"(1u)
+                : "memory");
+          }
         }
         asm volatile(
             "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
             :: "r"(bar) : "memory");
+      }
+      // the output that row i - 1 completed, beside this row's MMAs
+      if (i >= 3) {
+        const size_t v = ((size_t)x0 * N + y0 + i - 3) * N + z0 + tid;
+        store_voxel(r[0], v, bias, act, gate, out_f, out_b, out4);
+        store_voxel(r[1], v + (size_t)N * N, bias, act, gate, out_f, out_b, out4);
       }
       const bool got = mbar_wait(bar, phase);
       ok = __syncthreads_and(got ? 1 : 0) != 0;
       if (!ok && tid == 0) atomicOr(&g_tc_err, 1u);
       phase ^= 1u;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the MMAs have read loaded row i: its slot takes row i + 4
-      if (ok && i + 4 <= run + 1) gather_row(in, N, x, y0 - 1 + i + 4, ring + (i & 3) * 3 * LINE_BYTES);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      if (ok) {
-        uint32_t r[16];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-              "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-              "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const size_t v = (size_t)(l + i) * N + warp * 32 + lane;
-        float o[C];
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-          float a = __uint_as_float(r[c]) + (bias ? bias[c] : 0.0f);
-          if (act) a = a > 0.0f ? a : 0.1f * a;
-          if (gate && __bfloat162float(gate[v * C + c]) <= 0.0f) a *= 0.1f;
-          o[c] = a;
-        }
-        if (out_f) {
-          float4* d = reinterpret_cast<float4*>(out_f + v * C);
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            d[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-        }
-        if (out_b) {
-          __nv_bfloat16 hb[C];
-#pragma unroll
-          for (int c = 0; c < C; c++) hb[c] = __float2bfloat16_rn(o[c]);
-          uint4* d = reinterpret_cast<uint4*>(out_b + v * C);
-          d[0] = *reinterpret_cast<const uint4*>(&hb[0]);
-          d[1] = *reinterpret_cast<const uint4*>(&hb[8]);
-        }
-        if (out4) out4[v] = make_float4(o[0], o[1], o[2], o[3]);
-      }
+      const uint32_t slot = mine + (uint32_t)(16 * ((i + 1) % SLOTS));
+      tmem_ld16(r[0], slot);
+      tmem_ld16(r[1], slot + 16 * SLOTS);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tmem_zero16(slot);
+      tmem_zero16(slot + 16 * SLOTS);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
     }
-    // the run's prefetches land before the ring is refilled for the next x
+    if (ok) {
+      const size_t v = ((size_t)x0 * N + y0 + run - 1) * N + z0 + tid;
+      store_voxel(r[0], v, bias, act, gate, out_f, out_b, out4);
+      store_voxel(r[1], v + (size_t)N * N, bias, act, gate, out_f, out_b, out4);
+    }
+    // every copy has landed and every MMA has completed: the buffers are free
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     l += run;
@@ -401,25 +471,27 @@ __global__ void __launch_bounds__(THREADS, 3)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(128)
                  : "memory");
 }
 
 template <bool FLIP>
-cudaError_t launch_ring(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
-                        const float* bias, int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4,
-                        cudaStream_t st) {
+cudaError_t launch_sweep(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
+                         const float* bias, int act, const __nv_bfloat16* gate, float* of,
+                         __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv_ring<FLIP>,
+    cudaError_t e = cudaFuncSetAttribute(k_conv_sweep<FLIP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         ring_smem_bytes());
+                                         sweep_smem_bytes());
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  const int grid = 3 * cg_sm_count();
+  const int nrows = N / 2 * (N / TILE_M) * N;
+  const int cap = SWEEP_CPS * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);
-  k_conv_ring<FLIP><<<grid, THREADS, ring_smem_bytes(), st>>>(in, N, w, bias, act, gate, of, ob, o4);
+  k_conv_sweep<FLIP><<<nrows < cap ? nrows : cap, THREADS, sweep_smem_bytes(), st>>>(
+      in, N, w, bias, act, gate, of, ob, o4);
   return cudaGetLastError();
 }
 
@@ -443,12 +515,9 @@ cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, con
   return cudaGetLastError();
 }
 
-// pipeline variant: 2 (default at 128^3) = the line ring (k_conv_ring);
-// 1 (default for larger meshes) = one stage, 4 CTAs/SM; 0 = two stages,
-// 2 CTAs/SM.  Without the ring, at 128^3 the one-stage form is 1.2x faster
-// than the two-stage one: the tile loop is latency-bound and more resident
-// CTAs hide more of it than the prefetch does.  COLAGPU_CONV_VARIANT=0/1/2
-// selects one (2 only at 128^3).
+// pipeline variant: 2 (the default) = the sweep along y (k_conv_sweep); 1 =
+// one tile at a time, one stage, 4 CTAs/SM; 0 = two stages, 2 CTAs/SM.
+// COLAGPU_CONV_VARIANT=0/1/2 selects one.
 int g_conv_variant = -1;      // conv_tc_set_variant
 
 int conv_variant(int N) {
@@ -457,8 +526,8 @@ int conv_variant(int N) {
     return e ? atoi(e) : -1;
   }();
   const int v = forced >= 0 ? forced : g_conv_variant;
-  if (v == 0 || v == 1 || (v == 2 && N == TILE_M)) return v;
-  return N == TILE_M ? 2 : 1;
+  (void)N;
+  return v == 0 || v == 1 ? v : 2;
 }
 
 template <bool FLIP>
@@ -466,7 +535,7 @@ cudaError_t launch(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const
                    int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
   if (N < TILE_M || N % TILE_M) return cudaErrorNotSupported;
   const int v = conv_variant(N);
-  if (v == 2) return launch_ring<FLIP>(in, N, w, bias, act, gate, of, ob, o4, st);
+  if (v == 2) return launch_sweep<FLIP>(in, N, w, bias, act, gate, of, ob, o4, st);
   if (v == 1) return launch_v<FLIP, 1, 4>(in, N, w, bias, act, gate, of, ob, o4, st);
   return launch_v<FLIP, 2, 2>(in, N, w, bias, act, gate, of, ob, o4, st);
 }

@@ -204,8 +204,9 @@ int cg_net_set_scales(cg_net* h, float in_delta, float in_phi, float out_scale);
 /* 1: tcgen05 convolutions (default); 0: CUDA-core convolutions. */
 int cg_net_set_tensor_cores(cg_net* h, int on);
 /* Pipeline of the tensor-core convolutions, for every net: -1 by mesh size
- * (the default), 0 two stages, 1 one stage, 2 the line ring that reuses
- * input lines along y (128^3 meshes).  All give bit-identical outputs. */
+ * (the default), 0 two stages, 1 one stage, 2 the sweep that uses each
+ * input row for the three output rows it touches.  All give bit-identical
+ * outputs. */
 int cg_net_set_conv_variant(int variant);
 /* Host-array forward / backward (checks): in2 [v][2] scaled features,
  * out3 [v][3] raw outputs, grad3 = dLoss/dout3, grads [num_params]. */

@@ -196,3 +196,22 @@ def test_tensor_core_weight_gradient(gpu_lib, n):
     size = np.abs(g64).sum(axis=(0, 1, 2))
     assert (np.abs(db[:3] - g64.sum(axis=(0, 1, 2))) <= 128 * steps * 2.0 ** -23 * size).all()
     assert (db[3:] == 0).all()
+
+
+def test_conv_sweep_two_tiles_per_line(gpu_lib):
+    """At 256^3 a line has two tiles of 128 voxels and a CTA's run of rows
+    crosses columns: the sweep's outputs are bit for bit those of one tile at
+    a time."""
+    from cola_halo_b200.learned import ConvNet
+    n = 256
+    x = np.random.default_rng(6).normal(0, 1, (n, n, n, 2)).astype(np.float32)
+    net = ConvNet(n, seed=3)
+    out = []
+    try:
+        for v in (1, 2):
+            assert gpu_lib.cg_net_set_conv_variant(v) == 0
+            out.append(net.forward_host(x))
+    finally:
+        gpu_lib.cg_net_set_conv_variant(-1)
+        net.close()
+    np.testing.assert_array_equal(out[0], out[1])

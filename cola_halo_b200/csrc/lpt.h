@@ -13,13 +13,3 @@ int lpt_generate(int nc, double boxsize, int seed, double omega_m, double a_init
 
 // Release the device buffers kept between lpt_generate calls.
 void lpt_dropin_release();
-
-// Host RANLUX (48-bit, luxury 202): the generator of lpt.c:172-233.
-struct Ranlux48 {
-  double x[12];
-  double carry;
-  int ir, jr, ir_old;
-  int pr;
-  void seed(unsigned long s);
-  double uniform();
-};

@@ -3,8 +3,9 @@
 //
 //  1. seed table: one RANLUX stream on the host (lpt.c:172-207)
 //  2. modes: one thread per (kx, ky) column seeds its own RANLUX stream with
-//     the table entry and draws phase / amplitude for kz = 0..N/2-1
-//     (lpt.c:219-351), writing the Zel'dovich displacement spectra
+//     the table entry and draws phase / amplitude for kz = 0..N/2-1; then one
+//     thread per mode writes the Zel'dovich displacement spectra
+//     (lpt.c:219-351)
 //  3. gradients i k_j psi_i, six c2r (lpt.c:358-403)
 //  4. second-order source in real space, r2c (lpt.c:409-427)
 //  5. 2LPT displacement spectra -i k/k^2 S, c2r (lpt.c:440-503)
@@ -28,64 +29,61 @@ namespace {
 
 constexpr int T = CG_THREADS;
 constexpr double kUlp48 = 1.0 / 281474976710656.0;   // 2^-48
+constexpr unsigned long long kMask48 = (1ULL << 48) - 1;
 
 // ------------------------------------------------------------- RANLUX-48
 // Luscher's RANLUX in 48-bit form: x_k = x_{k-5} - x_{k-12} - c (mod 1) on
-// 12 words held as doubles in [0,1); 202 steps per block of 12 delivered
-// numbers (luxury level 1); seeding from a 31-bit shift register
-// b(n+31) = b(n) xor b(n+18) of the seed's bits.
-struct DevRanlux {
-  double x[12];
-  double carry;
-  int ir, jr, ir_old;
+// 12 words; 202 steps per block of 12 delivered numbers (luxury level 1);
+// seeding from a 31-bit shift register b(n+31) = b(n) xor b(n+18) of the
+// seed's bits.  The words are multiples of 2^-48, held as 48-bit integers: a
+// step is a 64-bit difference whose sign is the next borrow and whose low 48
+// bits are the new word, so the chain from borrow to borrow is one
+// subtraction and one shift.
+//
+// The words are kept in the order in which they are delivered next: x[k] is
+// the k-th oldest, and step k replaces x[k mod 12] from x[(k + 7) mod 12].
+struct Rlx {
+  unsigned long long x[12];
+  unsigned c;
 };
 
-__host__ __device__ inline void rlx_seed(double* x, double* carry, int* ir, int* jr, int* ir_old,
-                                         unsigned long s) {
+__host__ __device__ __forceinline__ void rlx_seed(Rlx& r, unsigned s) {
   if (s == 0) s = 1;
-  int bits[31];
-  unsigned long v = s & 0xFFFFFFFFUL;
-  for (int k = 0; k < 31; k++) { bits[k] = (int)(v & 1UL); v >>= 1; }
-  int ib = 0, jb = 18;
+  unsigned v = s & 0x7fffffffu;
+#pragma unroll
   for (int w = 0; w < 12; w++) {
-    double acc = 0.0;
+    unsigned long long acc = 0;
     for (int l = 0; l < 48; l++) {
-      acc = 2.0 * acc + (double)(bits[ib] ^ 1);
-      bits[ib] ^= bits[jb];
-      ib = ib == 30 ? 0 : ib + 1;
-      jb = jb == 30 ? 0 : jb + 1;
+      acc = 2 * acc + ((v & 1u) ^ 1u);
+      v = (v >> 1) | (((v ^ (v >> 18)) & 1u) << 30);
     }
-    x[w] = acc * kUlp48;
+    r.x[w] = acc;
   }
-  *carry = 0.0;
-  *ir = 11;
-  *jr = 7;
-  *ir_old = 0;
+  r.c = 0;
 }
 
-__host__ __device__ inline void rlx_refill(double* x, double* carry, int* ir, int* jr, int* ir_old,
-                                           int pr) {
-  int i = *ir, j = *jr;
-  double c = *carry;
-  for (int k = 0; k < pr; k++) {
-    double y = x[j] - x[i] - c;
-    if (y < 0.0) { c = kUlp48; y += 1.0; }
-    else c = 0.0;
-    x[i] = y;
-    i = i == 11 ? 0 : i + 1;
-    j = j == 11 ? 0 : j + 1;
-  }
-  *ir = i;
-  *jr = j;
-  *ir_old = i;
-  *carry = c;
+__host__ __device__ __forceinline__ void rlx_step(Rlx& r, int i, int j) {
+  const unsigned long long d = r.x[j] - r.x[i] - r.c;
+  r.c = (unsigned)(d >> 63);
+  r.x[i] = d & kMask48;
 }
 
-__host__ __device__ inline double rlx_uniform(double* x, double* carry, int* ir, int* jr,
-                                              int* ir_old, int pr) {
-  *ir = *ir == 11 ? 0 : *ir + 1;
-  if (*ir == *ir_old) rlx_refill(x, carry, ir, jr, ir_old, pr);
-  return x[*ir];
+// One block: 202 = 16 x 12 + 10 steps at compile-time places (the words stay
+// in registers), then the words move up by the 10 places so that x[0] .. x[11]
+// are the 12 numbers delivered.
+__host__ __device__ __forceinline__ void rlx_block(Rlx& r) {
+#pragma unroll 1
+  for (int b = 0; b < 16; b++) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) rlx_step(r, k, (k + 7) % 12);
+  }
+#pragma unroll
+  for (int k = 0; k < 10; k++) rlx_step(r, k, (k + 7) % 12);
+  unsigned long long t[12];
+#pragma unroll
+  for (int k = 0; k < 12; k++) t[k] = r.x[(k + 10) % 12];
+#pragma unroll
+  for (int k = 0; k < 12; k++) r.x[k] = t[k];
 }
 
 // --------------------------------------------------------------- modes
@@ -109,61 +107,80 @@ __device__ __forceinline__ double kvec_of(int i, int N, double kf) {
   return (i < N / 2 ? (double)i : -(double)(N - i)) * kf;
 }
 
-// lpt.c:219-351: modes of column (i, j); cd_a[k][i][j] for k < N/2.
-__global__ void __launch_bounds__(T) k_modes(int N, double box, const unsigned* __restrict__ seeds,
+// The draws of column t = (i, j): out[k][t] = (phase, amplitude) in [0, 1), for
+// k < N/2.  lpt.c:232-240 draws the amplitude again while it is 0, so then the
+// pairs shift by one: draw(n) below is the n-th number of the stream.
+// Latency-bound: a serial chain of 202 N / 12 steps per column, one column per
+// thread (N^2 of them), so the CTAs are small enough to reach every SM.
+constexpr int kDrawThreads = 64;
+__global__ void __launch_bounds__(kDrawThreads) k_draws(int N,
+                                                        const unsigned* __restrict__ seeds,
+                                                        double2* __restrict__ out) {
+  const long long cols = (long long)N * N;
+  const long long t = (long long)blockIdx.x * kDrawThreads + threadIdx.x;
+  if (t >= cols) return;
+  Rlx r;
+  rlx_seed(r, seeds[t]);
+  bool half = false;           // a phase waits for its amplitude
+  double phase = 0.0;
+  int k = 0;
+  while (k < N / 2) {
+    rlx_block(r);
+#pragma unroll
+    for (int n = 0; n < 12; n++) {
+      if (!half) {
+        phase = (double)r.x[n] * kUlp48;
+        half = true;
+      } else if (r.x[n] != 0 && k < N / 2) {
+        out[k * cols + t] = make_double2(phase, (double)r.x[n] * kUlp48);
+        k++;
+        half = false;
+      }
+    }
+  }
+}
+
+// lpt.c:243-351: the mode (i, j, k) of the draws; cd_a[k][i][j] for k < N/2.
+__global__ void __launch_bounds__(T) k_modes(int N, double box, const double2* __restrict__ draws,
                                              const double* __restrict__ logk,
                                              const double* __restrict__ logD, int ntab,
                                              double norm, float2* __restrict__ c0,
                                              float2* __restrict__ c1, float2* __restrict__ c2) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)N * N) return;
-  const int i = (int)(t / N), j = (int)(t % N);
-  double x[12], carry;
-  int ir, jr, ir_old;
-  rlx_seed(x, &carry, &ir, &jr, &ir_old, seeds[(size_t)i * N + j]);
   const double kf = 2 * M_PI / box;
   const double fac = pow(2 * M_PI / box, 1.5);
   float2* cd[3] = {c0, c1, c2};
   const size_t plane = (size_t)N * N;
-  for (int k = 0; k < N / 2; k++) {
-    const double phase = rlx_uniform(x, &carry, &ir, &jr, &ir_old, 202) * 2 * M_PI;
-    double ampl;
-    do {
-      ampl = rlx_uniform(x, &carry, &ir, &jr, &ir_old, 202);
-    } while (ampl == 0.0);
-    if (i == N / 2 || j == N / 2 || k == N / 2) continue;
+  const size_t total = plane * (N / 2);
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(t / plane), i = (int)((t / N) % N), j = (int)(t % N);
+    if (i == N / 2 || j == N / 2) continue;
     if (i == 0 && j == 0 && k == 0) continue;
+    const double2 d = draws[t];
+    const double phase = d.x * 2 * M_PI;
     const double kv[3] = {kvec_of(i, N, kf), kvec_of(j, N, kf), kvec_of(k, N, kf)};
     const double kmag2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
     const double kmag = sqrt(kmag2);
     double p = power_spec(kmag, logk, logD, ntab, norm);
-    p *= -log(ampl);
+    p *= -log(d.y);
     const double delta = fac * sqrt(p);
     double sp, cp;
     sincos(phase, &sp, &cp);
-    if (k > 0) {
-      for (int a = 0; a < 3; a++)
-        cd[a][k * plane + (size_t)i * N + j] =
-            make_float2((float)(-kv[a] / kmag2 * delta * sp), (float)(kv[a] / kmag2 * delta * cp));
-    } else if (i == 0) {
-      if (j >= N / 2) continue;
-      const int jj = N - j;
-      for (int a = 0; a < 3; a++) {
-        cd[a][(size_t)i * N + j] =
-            make_float2((float)(-kv[a] / kmag2 * delta * sp), (float)(kv[a] / kmag2 * delta * cp));
-        cd[a][(size_t)i * N + jj] =
-            make_float2((float)(-kv[a] / kmag2 * delta * sp), (float)(-kv[a] / kmag2 * delta * cp));
+    // k = 0: this mode and its conjugate at (-i, -j), from one half of the plane
+    size_t conj = 0;
+    if (k == 0) {
+      if (i == 0) {
+        if (j >= N / 2) continue;
+        conj = (size_t)(N - j);
+      } else {
+        if (i >= N / 2) continue;
+        conj = (size_t)(N - i) * N + (j == 0 ? 0 : N - j);
       }
-    } else {
-      if (i >= N / 2) continue;
-      const int ii = N - i;
-      const int jj = j == 0 ? 0 : N - j;
-      for (int a = 0; a < 3; a++) {
-        cd[a][(size_t)i * N + j] =
-            make_float2((float)(-kv[a] / kmag2 * delta * sp), (float)(kv[a] / kmag2 * delta * cp));
-        cd[a][(size_t)ii * N + jj] =
-            make_float2((float)(-kv[a] / kmag2 * delta * sp), (float)(-kv[a] / kmag2 * delta * cp));
-      }
+    }
+    for (int a = 0; a < 3; a++) {
+      const float re = (float)(-kv[a] / kmag2 * delta * sp);
+      cd[a][t] = make_float2(re, (float)(kv[a] / kmag2 * delta * cp));
+      if (k == 0) cd[a][conj] = make_float2(re, (float)(-kv[a] / kmag2 * delta * cp));
     }
   }
 }
@@ -280,7 +297,10 @@ LptBuffers g_lpt;
 void release() {
   if (g_lpt.st) cudaStreamSynchronize(g_lpt.st);
   for (int a = 0; a < 3; a++) cudaFree(g_lpt.cd[a]);
-  for (int a = 0; a < 6; a++) { cudaFree(g_lpt.gs[a]); cudaFree(g_lpt.gr[a]); }
+  for (int a = 0; a < 6; a++) {
+    if (a != 1) cudaFree(g_lpt.gs[a]);         // gs[1] is the second half of gs[0]
+    cudaFree(g_lpt.gr[a]);
+  }
   cudaFree(g_lpt.seeds);
   cudaFree(g_lpt.tab);
   cudaFree(g_lpt.aos);
@@ -297,7 +317,10 @@ cudaError_t ensure(int N) {
   const size_t sb = sizeof(float2) * (size_t)(N / 2 + 1) * N * N;
   const size_t rb = sizeof(float) * (size_t)N * N * N;
   for (int a = 0; a < 3 && e == cudaSuccess; a++) e = cudaMalloc(&g_lpt.cd[a], sb);
-  for (int a = 0; a < 6 && e == cudaSuccess; a++) e = cudaMalloc(&g_lpt.gs[a], sb);
+  // the first two lie next to each other: the random draws use both
+  if (e == cudaSuccess) e = cudaMalloc(&g_lpt.gs[0], 2 * sb);
+  if (e == cudaSuccess) g_lpt.gs[1] = g_lpt.gs[0] + sb / sizeof(float2);
+  for (int a = 2; a < 6 && e == cudaSuccess; a++) e = cudaMalloc(&g_lpt.gs[a], sb);
   for (int a = 0; a < 6 && e == cudaSuccess; a++) e = cudaMalloc(&g_lpt.gr[a], rb);
   if (e == cudaSuccess) e = cudaMalloc(&g_lpt.seeds, sizeof(unsigned) * (size_t)N * N);
   if (e == cudaSuccess) e = cudaMalloc(&g_lpt.aos, 56 * (size_t)N * N * N);
@@ -312,18 +335,27 @@ cudaError_t ensure(int N) {
 }  // namespace
 
 // ------------------------------------------------------------ host RNG
-void Ranlux48::seed(unsigned long s) {
-  pr = 202;
-  rlx_seed(x, &carry, &ir, &jr, &ir_old, s);
-}
-double Ranlux48::uniform() { return rlx_uniform(x, &carry, &ir, &jr, &ir_old, pr); }
+// The stream of one seed (lpt.c:172-207), a block of 12 at a time.
+namespace {
+struct Ranlux48 {
+  Rlx r;
+  int n = 12;                  // delivered of the current block
+  explicit Ranlux48(unsigned s) { rlx_seed(r, s); }
+  double uniform() {
+    if (n == 12) {
+      rlx_block(r);
+      n = 0;
+    }
+    return (double)r.x[n++] * kUlp48;
+  }
+};
+}  // namespace
 
 void lpt_dropin_release() { release(); }
 
 // lpt.c:177-207
 static void seed_table(int N, int seed, std::vector<unsigned>& st) {
-  Ranlux48 r;
-  r.seed((unsigned long)seed);
+  Ranlux48 r((unsigned)seed);
   st.assign((size_t)N * N, 0u);
   auto draw = [&]() { return (unsigned)(0x7fffffff * r.uniform()); };
   for (int i = 0; i < N / 2; i++) {
@@ -373,11 +405,17 @@ int lpt_generate(int nc, double boxsize, int seed, double omega_m, double a_init
   if (e != cudaSuccess) return cg_set_error_from_lpt(CG_ECUDA, cudaGetErrorString(e));
   // 2. modes
   {
+    // the draws take the room of two of the gradient spectra (16 bytes for
+    // each of N^2 N/2 modes), which are written next
     const long long cols = (long long)N * N;
+    double2* draws = (double2*)g_lpt.gs[0];
     prof_mark(st, CG_ST_LPT);
-    k_modes<<<(int)((cols + T - 1) / T), T, 0, st>>>(N, boxsize, g_lpt.seeds, g_lpt.tab,
-                                                      g_lpt.tab + ntab, ntab, power.norm,
-                                                      g_lpt.cd[0], g_lpt.cd[1], g_lpt.cd[2]);
+    k_draws<<<(int)((cols + kDrawThreads - 1) / kDrawThreads), kDrawThreads, 0, st>>>(
+        N, g_lpt.seeds, draws);
+    prof_mark(st, CG_ST_LPT);
+    k_modes<<<grid_for(cols * (N / 2)), T, 0, st>>>(N, boxsize, draws, g_lpt.tab,
+                                                    g_lpt.tab + ntab, ntab, power.norm,
+                                                    g_lpt.cd[0], g_lpt.cd[1], g_lpt.cd[2]);
   }
   // 3. gradients and six c2r
   Spec6 g6;

@@ -39,3 +39,24 @@ def test_lpt_matches_reference(gpu_lib, ref, bbks_table, nc, L, seed):
     for k in (0.01, 0.1, 1.0, 3.0):
         assert abs(lib.PowerSpec(k) / ref.PowerSpec(k) - 1) < 1e-12
     assert abs(lib.GrowthFactor(a0, 1.0) / ref.GrowthFactor(a0, 1.0) - 1) < 1e-7
+
+
+@pytest.mark.parametrize("nc,seed", [(16, 100), (48, 1), (48, 0x7fffffff)])
+def test_lpt_matches_restatement(gpu_lib, bbks_table, nc, seed):
+    """The same against the oracle's numpy restatement: the random stream of
+    every column (its words as 48-bit integers on the device, as doubles in
+    the oracle) and the modes drawn from it, on a power-of-two and another
+    grid.  Tolerances as against lpt.c."""
+    from oracle import restate as R
+    a0, L = 0.1, 100.0
+    want = R.lpt_set_displacement(nc, L, seed, OM, a0, R.PowerTable(bbks_table))
+    lib = gpu_lib
+    lib.cg_dropin_set_abort(0)
+    lib.power_init(bbks_table.encode(), a0, 0.81, OM, 1 - OM)
+    lib.lpt_init(nc, None, 0)
+    pg = HostParticles(nc)
+    assert lib.lpt_set_displacement(a0, OM, seed, L, pg.ptr) == 0, lib.cg_last_error()
+    got = pg.local()
+    for k in ("dx1", "dx2"):
+        assert np.abs(got[k] - want[k]).max() < 2e-5 * np.abs(want[k]).max(), k
+    assert periodic_diff(got["x"], want["x"], L).max() < 2e-6 * L

@@ -9,17 +9,27 @@
 // members, wrapped into [0, L) (fof.c:287-322, 1141-1150), and the mean
 // velocity.  Here:
 //   1. wrap positions (move_particles2_min, fof.c:1042) and bin them on a
-//      grid of cells no smaller than ll (counting sort: count, scan, scatter)
-//   2. each particle tests the particles of the 27 neighbouring cells that
-//      come after it in cell order; a link joins the two sets of a
-//      lock-free union-find over the original particle indices (hooking the
-//      larger root under the smaller with atomicCAS, path halving)
-//   3. flatten to roots, count members, number the roots with >= nfof_min
-//      members in root order (a scan), accumulate the offsets from the root
+//      grid of cells no smaller than ll (counting sort: count with ranks,
+//      scan, scatter); from here on a particle is its slot in cell order
+//   2. the particles of crowded cells are put in the order of their sub-cells
+//   3. each particle tests the later particles of the cells within ll of it;
+//      a link joins the two sets of a lock-free union-find over the slots
+//      (hooking one root under the other with atomicCAS, in a scrambled order
+//      of the slots, path halving)
+//   4. flatten to roots, count members and find each group's smallest
+//      original index, number the groups with >= nfof_min members in the
+//      order of that index (a scan), accumulate the offsets from that
 //      particle and the velocities in double, and finish each halo.
-// The root of a group is its smallest original index, so the catalogue is
-// in a fixed order and each centre's reference member is fixed.  Every
-// retry loop is bounded; running out of iterations sets an error word.
+// So the catalogue is in a fixed order and each centre's reference member is
+// fixed.  Every retry loop is bounded; running out of iterations sets an
+// error word.
+//
+// 256^3 particles, L = 600, ll = 0.2 spacings, a third of them in halos: the
+// link kernel takes 8.8 ms (12.4 with all 27 neighbour cells and a union-find
+// over the original indices), and the whole call 13.5 to 14.2 ms (26.6).  The link
+// kernel is bound by its chains of dependent L2 loads: cell starts, candidate,
+// parent.  A warp for each crowded cell, its particles held in registers, took
+// 10.6 ms for those cells alone.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -59,35 +69,38 @@ __device__ __forceinline__ int cell_of(float x, float inv, int nc) {
   return c < 0 ? 0 : (c >= nc ? nc - 1 : c);
 }
 
+// Each particle's cell and its rank among the cell's arrivals.
 __global__ void k_fof_bin(const PMin* __restrict__ p, long long n, float L, float inv, int nc,
-                          float* __restrict__ xw, unsigned* __restrict__ key,
+                          unsigned* __restrict__ key, unsigned* __restrict__ rank,
                           unsigned* __restrict__ count) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T) {
-    const float x = wrap1(p[i].x[0], L), y = wrap1(p[i].x[1], L), z = wrap1(p[i].x[2], L);
-    xw[3 * i] = x;
-    xw[3 * i + 1] = y;
-    xw[3 * i + 2] = z;
+    const float4 q = *reinterpret_cast<const float4*>(p + i);
+    const float x = wrap1(q.x, L), y = wrap1(q.y, L), z = wrap1(q.z, L);
     const unsigned k =
         ((unsigned)cell_of(x, inv, nc) * nc + cell_of(y, inv, nc)) * nc + cell_of(z, inv, nc);
     key[i] = k;
-    atomicAdd(count + k, 1u);
+    rank[i] = atomicAdd(count + k, 1u);
   }
 }
 
-__global__ void k_fof_scatter(const float* __restrict__ xw, const unsigned* __restrict__ key,
-                              long long n, const unsigned* __restrict__ start,
-                              unsigned* __restrict__ cursor, float4* __restrict__ pos) {
+// Wrapped position and original index at the particle's slot; the slot starts
+// as a set of its own.
+__global__ void k_fof_scatter(const PMin* __restrict__ p, const unsigned* __restrict__ key,
+                              const unsigned* __restrict__ rank, long long n, float L,
+                              const unsigned* __restrict__ start, float4* __restrict__ pos,
+                              int* __restrict__ parent) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T) {
-    const unsigned k = key[i];
-    const unsigned slot = start[k] + atomicAdd(cursor + k, 1u);
-    pos[slot] = make_float4(xw[3 * i], xw[3 * i + 1], xw[3 * i + 2], __int_as_float((int)i));
+    const float4 q = *reinterpret_cast<const float4*>(p + i);
+    const unsigned slot = start[key[i]] + rank[i];
+    pos[slot] = make_float4(wrap1(q.x, L), wrap1(q.y, L), wrap1(q.z, L), __int_as_float((int)i));
+    parent[i] = (int)i;
   }
 }
 
 // ------------------------------------------------------------- union-find
-// parent[] over original particle indices; a root is parent[r] == r.
+// parent[] over slots; a root is parent[r] == r.
 __device__ __forceinline__ int find_root(int* parent, int x, unsigned* err) {
   for (int it = 0; it < kRetryLimit; it++) {
     const int p = __ldcg(parent + x);
@@ -100,26 +113,28 @@ __device__ __forceinline__ int find_root(int* parent, int x, unsigned* err) {
   return x;
 }
 
-__device__ __forceinline__ void unite(int* parent, int a, int b, unsigned* err) {
+// Which of two roots hangs under the other: a fixed scrambling of the slots.
+// With the slots' own order, threads that work through neighbouring slots at
+// once would hang every particle of a halo under the one before it, a chain as
+// long as the halo (256^3: the link kernel three times slower).
+__device__ __forceinline__ unsigned rank_of(int slot) { return (unsigned)slot * 2654435761u; }
+
+// Join the sets of a and b; returns the root they then share.
+__device__ __forceinline__ int unite(int* parent, int a, int b, unsigned* err) {
   for (int it = 0; it < kRetryLimit; it++) {
     a = find_root(parent, a, err);
     b = find_root(parent, b, err);
-    if (a == b) return;
-    if (a > b) {
+    if (a == b) return a;
+    if (rank_of(a) > rank_of(b)) {
       const int t = a;
       a = b;
       b = t;
     }
-    // hang the larger root under the smaller one if it is still a root
-    if (atomicCAS(parent + b, b, a) == b) return;
+    // hang the later root under the earlier one if it is still a root
+    if (atomicCAS(parent + b, b, a) == b) return a;
   }
   atomicOr(err, 2u);
-}
-
-__global__ void k_fof_init_parent(int* __restrict__ parent, long long n) {
-  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
-       i += (long long)gridDim.x * T)
-    parent[i] = (int)i;
+  return a;
 }
 
 // Squared distance of two wrapped positions with the periodic image formed
@@ -140,102 +155,287 @@ __device__ __forceinline__ float dist2(float4 a, float4 b, float L, float half) 
                    __fmul_rn(d[2], d[2]));
 }
 
-// One thread per particle in cell order: links to the particles of the 27
-// neighbouring cells that come later in cell order (each pair once).  With
-// fewer than 3 cells per dimension every cell is a neighbour.
-__global__ void k_fof_link(const float4* __restrict__ pos, long long n,
-                           const unsigned* __restrict__ start, const unsigned* __restrict__ count,
-                           int nc, float inv, float L, float ll2, int* __restrict__ parent,
-                           unsigned* __restrict__ err) {
+// Cells of one axis within `reach` of [x0, x1]: lo .. hi, unwrapped (below 0 or
+// above nc - 1 across the periodic face), or every cell.  reach is ll plus a
+// margin over the rounding of x +- reach, and cell_of never decreases with x, so
+// no particle closer than ll lies outside.
+__device__ __forceinline__ void cells_within(float x0, float x1, float reach, float L, float inv,
+                                             int nc, int& lo, int& hi) {
+  const float a = x0 - reach, b = x1 + reach;
+  lo = a < 0.0f ? cell_of(a + L, inv, nc) - nc : cell_of(a, inv, nc);
+  hi = b >= L ? cell_of(b - L, inv, nc) + nc : cell_of(b, inv, nc);
+  if (hi - lo + 1 >= nc) {
+    lo = 0;
+    hi = nc - 1;
+  }
+}
+
+// Cells with more than a warp of particles (and at most kSubMax), listed by
+// their first slot.
+constexpr int kSubMax = 2048;
+__global__ void k_fof_dense(const float4* __restrict__ pos, long long n,
+                            const unsigned* __restrict__ start, int nc, float inv,
+                            unsigned* __restrict__ list, unsigned* __restrict__ count) {
+  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
+       i += (long long)gridDim.x * T) {
+    const float4 a = pos[i];
+    const unsigned k = ((unsigned)cell_of(a.x, inv, nc) * nc + cell_of(a.y, inv, nc)) * nc +
+                       cell_of(a.z, inv, nc);
+    if (start[k] != (unsigned)i) continue;
+    const unsigned m = start[k + 1] - (unsigned)i;
+    if (m > 32 && m <= kSubMax) list[atomicAdd(count, 1u)] = k;
+  }
+}
+
+// Their particles in the order of 4^3 sub-cells (a counting sort in shared
+// memory), so that 32 consecutive slots of a halo are a compact clump: the
+// ranges and the blocks that k_fof_link looks at shrink with it.
+constexpr int kSubThreads = 128;
+__global__ void __launch_bounds__(kSubThreads) k_fof_subsort(
+    float4* __restrict__ pos, const unsigned* __restrict__ start, int nc, float inv,
+    const unsigned* __restrict__ list, const unsigned* __restrict__ count) {
+  __shared__ float4 buf[kSubMax];
+  __shared__ unsigned at[64];
+  const unsigned cells = *count;
+  for (unsigned c = blockIdx.x; c < cells; c += gridDim.x) {
+    const unsigned k = list[c], s0 = start[k], m = start[k + 1] - s0;
+    const float cx = (float)(k / nc / nc), cy = (float)(k / nc % nc), cz = (float)(k % nc);
+    const auto sub = [&](const float4& a) {
+      const int x = min(max((int)(4.0f * (a.x * inv - cx)), 0), 3);
+      const int y = min(max((int)(4.0f * (a.y * inv - cy)), 0), 3);
+      const int z = min(max((int)(4.0f * (a.z * inv - cz)), 0), 3);
+      return (x * 4 + y) * 4 + z;
+    };
+    if (threadIdx.x < 64) at[threadIdx.x] = 0;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < m; i += kSubThreads) {
+      buf[i] = pos[s0 + i];
+      atomicAdd(&at[sub(buf[i])], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned run = 0;
+      for (int b = 0; b < 64; b++) {
+        const unsigned v = at[b];
+        at[b] = run;
+        run += v;
+      }
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < m; i += kSubThreads)
+      pos[s0 + atomicAdd(&at[sub(buf[i])], 1u)] = buf[i];
+    __syncthreads();
+  }
+}
+
+// Bounding boxes of the blocks of 32 slots: box[2 b] the lower corner, box[2 b +
+// 1] the upper one.
+__global__ void k_fof_boxes(const float4* __restrict__ pos, long long n,
+                            float4* __restrict__ box) {
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
+       base += (long long)gridDim.x * T) {
+    const float4 a = pos[min(base + lane, n - 1)];
+    float lo[3] = {a.x, a.y, a.z}, hi[3] = {a.x, a.y, a.z};
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+      }
+    if (lane == 0) {
+      box[base / 16] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+      box[base / 16 + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+    }
+  }
+}
+
+// One thread per slot: links to the later slots of the cells within ll (each
+// pair once: the earlier slot tests it).  The cells of one (x, y) row are
+// consecutive in z, so a row is one range of slots, or two across the
+// periodic face, and rows before the particle's own hold no later slot.
+//
+// In halos, where a warp's 32 slots are a clump of at most two cells across,
+// its lanes take the same ranges (the cells within ll of the clump), so that
+// every candidate is one broadcast load for the warp, and skip the blocks of 32
+// candidates whose box is further than ll from the clump's.  Elsewhere the few
+// candidates are each lane's own.  ra is an ancestor of s: a candidate whose
+// parent it is belongs to the set already, which spares most pairs of a halo the
+// distance and both find_roots.
+__global__ void __launch_bounds__(T, 5) k_fof_link(const float4* __restrict__ pos, long long n,
+                                                   const float4* __restrict__ box,
+                                                   const unsigned* __restrict__ start, int nc,
+                                                   float inv, float L, float ll2, float reach,
+                                                   int* parent, unsigned* __restrict__ err) {
   const float half = 0.5f * L;
-  for (long long s = (long long)blockIdx.x * T + threadIdx.x; s < n;
-       s += (long long)gridDim.x * T) {
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
+       base += (long long)gridDim.x * T) {
+    const bool live = base + lane < n;
+    const unsigned s = (unsigned)(live ? base + lane : n - 1);
     const float4 a = pos[s];
-    const int ia = __float_as_int(a.w);
-    const int cx = cell_of(a.x, inv, nc), cy = cell_of(a.y, inv, nc), cz = cell_of(a.z, inv, nc);
-    const int span = nc >= 3 ? 3 : nc;
-    for (int ox = 0; ox < span; ox++) {
-      const int gx = nc >= 3 ? (cx + ox - 1 + nc) % nc : ox;
-      for (int oy = 0; oy < span; oy++) {
-        const int gy = nc >= 3 ? (cy + oy - 1 + nc) % nc : oy;
-        for (int oz = 0; oz < span; oz++) {
-          const int gz = nc >= 3 ? (cz + oz - 1 + nc) % nc : oz;
-          const unsigned k = ((unsigned)gx * nc + gy) * nc + gz;
-          const unsigned b0 = start[k], b1 = b0 + count[k];
-          for (unsigned t = b0 > (unsigned)s ? b0 : (unsigned)s + 1; t < b1; t++) {
-            const float4 b = pos[t];
-            if (dist2(a, b, L, half) < ll2) unite(parent, ia, __float_as_int(b.w), err);
-          }
-        }
+    float4 lo = box[base / 16], hi = box[base / 16 + 1];
+    unsigned own = (unsigned)cell_of(a.x, inv, nc) * nc + cell_of(a.y, inv, nc);
+    const float wide = fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * inv;
+    const bool clump = wide <= 2.0f;
+    if (clump) own = __reduce_min_sync(0xffffffffu, own);
+    else lo = hi = a;
+    int xl, xh, yl, yh, zl, zh;
+    cells_within(lo.x, hi.x, reach, L, inv, nc, xl, xh);
+    cells_within(lo.y, hi.y, reach, L, inv, nc, yl, yh);
+    cells_within(lo.z, hi.z, reach, L, inv, nc, zl, zh);
+    int ra = (int)s;
+    const auto test = [&](unsigned t, unsigned end) {
+      for (; t < end; t++) {
+        if (t <= s || __ldcg(parent + t) == ra) continue;
+        if (dist2(a, pos[t], L, half) < ll2) ra = unite(parent, ra, (int)t, err);
+      }
+    };
+    // slots of the cells z0 .. z1 of a row; `near`: no periodic face in between
+    const auto range = [&](unsigned row, int z0, int z1, bool near) {
+      unsigned t = max(start[row * nc + z0], (unsigned)base + 1);
+      const unsigned end = start[row * nc + z1 + 1];
+      if (!live) return;
+      if (!clump || !near) {
+        test(t, end);
+        return;
+      }
+      for (; t < end; t = (t & ~31u) + 32u) {
+        const float4 bl = box[t / 32 * 2], bh = box[t / 32 * 2 + 1];
+        if (bl.x > hi.x + reach || bh.x < lo.x - reach || bl.y > hi.y + reach ||
+            bh.y < lo.y - reach || bl.z > hi.z + reach || bh.z < lo.z - reach)
+          continue;
+        test(t, min(end, (t & ~31u) + 32u));
+      }
+    };
+    for (int x = xl; x <= xh; x++) {
+      const int gx = x < 0 ? x + nc : (x >= nc ? x - nc : x);
+      for (int y = yl; y <= yh; y++) {
+        const int gy = y < 0 ? y + nc : (y >= nc ? y - nc : y);
+        const unsigned row = (unsigned)gx * nc + gy;
+        if (row < own) continue;
+        // ranges that stand for every cell have no image of their own
+        const bool near = gx == x && gy == y && xh - xl + 1 < nc && yh - yl + 1 < nc &&
+                          zh - zl + 1 < nc;
+        if (zl < 0) range(row, zl + nc, nc - 1, false);
+        range(row, max(zl, 0), min(zh, nc - 1), near);
+        if (zh >= nc) range(row, 0, zh - nc, false);
       }
     }
   }
 }
 
-__global__ void k_fof_flatten(int* __restrict__ parent, long long n, unsigned* __restrict__ size,
-                              unsigned* __restrict__ err) {
-  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
-       i += (long long)gridDim.x * T) {
+// Every slot's root, and per root the members and their smallest original
+// index (lowest, set to 0xffffffff before).  The members of a group sit close
+// to each other in cell order: lanes with the same root add once.
+__global__ void k_fof_flatten(const float4* __restrict__ pos, int* __restrict__ parent,
+                              long long n, unsigned* __restrict__ size,
+                              unsigned* __restrict__ lowest, unsigned* __restrict__ err) {
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
+       base += (long long)gridDim.x * T) {
+    const long long i = base + lane;
+    const unsigned live = __ballot_sync(0xffffffffu, i < n);
+    if (i >= n) continue;
     const int r = find_root(parent, (int)i, err);
-    atomicAdd(size + r, 1u);
+    parent[i] = r;
+    const unsigned orig = (unsigned)__float_as_int(pos[i].w);
+    const unsigned same = __match_any_sync(live, r);
+    const unsigned low = __reduce_min_sync(same, orig);
+    if (lane == __ffs(same) - 1) {
+      atomicAdd(size + r, (unsigned)__popc(same));
+      atomicMin(lowest + r, low);
+    }
   }
 }
 
-// After flatten every particle's chain ends at its root; store it directly.
-__global__ void k_fof_roots(int* __restrict__ parent, long long n, unsigned* __restrict__ err) {
-  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
-       i += (long long)gridDim.x * T)
-    parent[i] = find_root(parent, (int)i, err);
-}
-
+// A halo's flag stands at its smallest original index.
 __global__ void k_fof_flag(const int* __restrict__ root, const unsigned* __restrict__ size,
-                           long long n, unsigned nmin, unsigned* __restrict__ flag) {
+                           const unsigned* __restrict__ lowest, long long n, unsigned nmin,
+                           unsigned* __restrict__ flag) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T)
-    flag[i] = (root[i] == (int)i && size[i] >= nmin) ? 1u : 0u;
+    if (root[i] == (int)i && size[i] >= nmin) flag[lowest[i]] = 1u;
 }
 
-// Per member: offset from the halo's root particle with the minimum-image
+// Wrapped position of an original particle.
+__device__ __forceinline__ float3 wrapped(const PMin* __restrict__ p, unsigned i, float L) {
+  const float4 q = *reinterpret_cast<const float4*>(p + i);
+  return make_float3(wrap1(q.x, L), wrap1(q.y, L), wrap1(q.z, L));
+}
+
+// Per member: offset from the halo's reference particle with the minimum-image
 // wrap of halo_particle (fof.c:304-313, float), summed in double with the
-// velocities.  acc[6 h + 0..2] = offsets, [3..5] = velocities.
-__global__ void k_fof_accum(const PMin* __restrict__ p, const float* __restrict__ xw,
-                            const int* __restrict__ root, const unsigned* __restrict__ hid,
-                            const unsigned* __restrict__ flag, long long n, float L,
+// velocities.  acc[6 h + 0..2] = offsets, [3..5] = velocities.  A warp whose
+// lanes all belong to one halo adds its sum once.
+__global__ void k_fof_accum(const PMin* __restrict__ p, const float4* __restrict__ pos,
+                            const int* __restrict__ root, const unsigned* __restrict__ size,
+                            const unsigned* __restrict__ lowest,
+                            const unsigned* __restrict__ hid, long long n, unsigned nmin, float L,
                             double* __restrict__ acc) {
   const float half = 0.5f * L;
-  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
-       i += (long long)gridDim.x * T) {
-    const int r = root[i];
-    if (!flag[r]) continue;
-    const unsigned h = hid[r];
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
+       base += (long long)gridDim.x * T) {
+    const long long i = base + lane;
+    const int r = i < n ? root[i] : -1;
+    const bool in = r >= 0 && size[r] >= nmin;
+    if (!__any_sync(0xffffffffu, in)) continue;
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    unsigned h = 0xffffffffu;
+    if (in) {
+      const unsigned ref = lowest[r];
+      h = hid[ref];
+      const float4 a = pos[i];
+      const float3 b = wrapped(p, ref, L);
+      const PMin& q = p[__float_as_int(a.w)];
+      const float d[3] = {__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z)};
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      float dx = __fsub_rn(xw[3 * i + k], xw[3 * (size_t)r + k]);
-      if (dx > half) dx = __fsub_rn(dx, L);
-      else if (dx < -half) dx = __fadd_rn(dx, L);
-      atomicAdd(acc + 6 * (size_t)h + k, (double)dx);
-      atomicAdd(acc + 6 * (size_t)h + 3 + k, (double)p[i].v[k]);
+      for (int k = 0; k < 3; k++) {
+        float dx = d[k];
+        if (dx > half) dx = __fsub_rn(dx, L);
+        else if (dx < -half) dx = __fadd_rn(dx, L);
+        v[k] = (double)dx;
+        v[3 + k] = (double)q.v[k];
+      }
+    }
+    if (__all_sync(0xffffffffu, h == __shfl_sync(0xffffffffu, h, 0))) {
+#pragma unroll
+      for (int k = 0; k < 6; k++)
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+      if (lane < 6) {
+        const double s = lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2]
+                       : lane == 3 ? v[3] : lane == 4 ? v[4] : v[5];
+        atomicAdd(acc + 6 * (size_t)h + lane, s);
+      }
+    } else if (in) {
+#pragma unroll
+      for (int k = 0; k < 6; k++) atomicAdd(acc + 6 * (size_t)h + k, v[k]);
     }
   }
 }
 
 // Halo h: centre x0 + mean offset wrapped into [0, L) as fof.c:1141-1147,
 // mean velocity (fof.c:1150).
-__global__ void k_fof_finish(const float* __restrict__ xw, const unsigned* __restrict__ size,
-                             const unsigned* __restrict__ hid, const unsigned* __restrict__ flag,
-                             long long n, float L, const double* __restrict__ acc,
-                             cg_halo* __restrict__ out, long long max_out) {
+__global__ void k_fof_finish(const PMin* __restrict__ p, const int* __restrict__ root,
+                             const unsigned* __restrict__ size,
+                             const unsigned* __restrict__ lowest,
+                             const unsigned* __restrict__ hid, long long n, unsigned nmin, float L,
+                             const double* __restrict__ acc, cg_halo* __restrict__ out,
+                             long long max_out) {
   for (long long r = (long long)blockIdx.x * T + threadIdx.x; r < n;
        r += (long long)gridDim.x * T) {
-    if (!flag[r]) continue;
-    const unsigned h = hid[r];
+    if (root[r] != (int)r || size[r] < nmin) continue;
+    const unsigned ref = lowest[r], h = hid[ref];
     if ((long long)h >= max_out) continue;
     const unsigned nf = size[r];
+    const float3 b = wrapped(p, ref, L);
+    const float x0[3] = {b.x, b.y, b.z};
     cg_halo o;
     o.nfof = (int)nf;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      float x = __fadd_rn(xw[3 * r + k], (float)(acc[6 * (size_t)h + k] / (double)nf));
+      float x = __fadd_rn(x0[k], (float)(acc[6 * (size_t)h + k] / (double)nf));
       if (x < 0.0f) x += L;
       if (x >= L) x -= L;
       o.x[k] = x;
@@ -245,11 +445,19 @@ __global__ void k_fof_finish(const float* __restrict__ xw, const unsigned* __res
   }
 }
 
-template <class TPtr>
-void release(TPtr*& p) {
-  if (p) cudaFree(p);
-  p = nullptr;
-}
+// One device block cut into arrays (16-byte aligned): a call takes and gives
+// back one allocation instead of a dozen, each of which costs a mapping and a
+// synchronisation (256^3: 10 of 26 ms).
+struct Block {
+  unsigned char* base = nullptr;
+  size_t used = 0;
+  template <class V>
+  V* cut(long long count) {
+    V* p = base ? reinterpret_cast<V*>(base + used) : nullptr;
+    used += (sizeof(V) * (size_t)count + 15) / 16 * 16;
+    return p;
+  }
+};
 
 }  // namespace
 
@@ -270,85 +478,111 @@ extern "C" int cg_fof(const void* pmin, long long np, float boxsize, float ll, i
   if (nc < 1) nc = 1;
   const long long ncells = nc * nc * nc;
   const float inv = (float)nc / boxsize;
-  const long long nblk = cgscan::scratch_entries(ncells > np ? ncells : np);
+  const long long nblk = cgscan::scratch_entries(ncells > np ? ncells + 1 : np);
+  // every cell of a linked pair lies within `reach`: ll, plus the rounding of
+  // the sums with positions up to 2 L
+  const float reach = ll * 1.0001f + boxsize * 4e-7f;
 
   cudaPointerAttributes attr;
   bool on_device = cudaPointerGetAttributes(&attr, pmin) == cudaSuccess &&
                    (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
   cudaGetLastError();   // a plain host pointer may leave an error behind
-  PMin* d_p = on_device ? (PMin*)pmin : nullptr;
-  float* xw = nullptr;
-  unsigned *key = nullptr, *count = nullptr, *start = nullptr, *cursor = nullptr;
-  unsigned *size = nullptr, *flag = nullptr, *hid = nullptr, *bsum = nullptr, *word = nullptr;
+  // (records are read as 16-byte vectors; a device array off that boundary,
+  // like a host array, is copied first)
+  const bool in_place = on_device && reinterpret_cast<uintptr_t>(pmin) % 16 == 0;
+  const PMin* d_p = nullptr;
+  PMin* own = nullptr;
+  unsigned *key = nullptr, *rank = nullptr, *start = nullptr, *size = nullptr, *lowest = nullptr;
+  unsigned *flag = nullptr, *bsum = nullptr, *word = nullptr;
   int* parent = nullptr;
-  float4* pos = nullptr;
-  double* acc = nullptr;
-  cg_halo* out = nullptr;
+  float4 *pos = nullptr, *box = nullptr;
+  Block blk;
+  const auto cut = [&] {
+    blk.used = 0;
+    word = blk.cut<unsigned>(4);              // [0] halos, [1] error, [2] dense cells
+    start = blk.cut<unsigned>(ncells + 1);    // counts, then starts; [ncells] = np
+    size = blk.cut<unsigned>(np);
+    flag = blk.cut<unsigned>(np);             // then the halo numbers
+    lowest = blk.cut<unsigned>(np);
+    parent = blk.cut<int>(np);
+    key = blk.cut<unsigned>(np);
+    rank = blk.cut<unsigned>(np);
+    pos = blk.cut<float4>(np);
+    box = blk.cut<float4>((np + 31) / 32 * 2);
+    bsum = blk.cut<unsigned>(nblk + 1);
+    own = blk.cut<PMin>(in_place ? 0 : np);
+    d_p = in_place ? (const PMin*)pmin : own;
+  };
+  cut();
   cudaStream_t st = 0;
-  cudaError_t e = cudaSuccess;
-  if (!on_device) {
-    e = cudaMalloc(&d_p, sizeof(PMin) * np);
-    if (e == cudaSuccess) e = cudaMemcpy(d_p, pmin, sizeof(PMin) * np, cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&xw, sizeof(float) * 3 * np);
-  if (e == cudaSuccess) e = cudaMalloc(&key, sizeof(unsigned) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&count, sizeof(unsigned) * ncells);
-  if (e == cudaSuccess) e = cudaMalloc(&start, sizeof(unsigned) * ncells);
-  if (e == cudaSuccess) e = cudaMalloc(&cursor, sizeof(unsigned) * ncells);
-  if (e == cudaSuccess) e = cudaMalloc(&pos, sizeof(float4) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&parent, sizeof(int) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&size, sizeof(unsigned) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&flag, sizeof(unsigned) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&hid, sizeof(unsigned) * np);
-  if (e == cudaSuccess) e = cudaMalloc(&bsum, sizeof(unsigned) * (nblk + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&word, sizeof(unsigned) * 2);   // [0] total, [1] error
-  if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, sizeof(unsigned) * ncells, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, sizeof(unsigned) * ncells, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(size, 0, sizeof(unsigned) * np, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(word, 0, sizeof(unsigned) * 2, st);
-  unsigned nh = 0, errw = 0;
+  cudaError_t e = cudaMalloc(&blk.base, blk.used);
+  if (e != cudaSuccess) blk.base = nullptr;
+  cut();
+  if (e == cudaSuccess && !in_place)
+    e = cudaMemcpy(own, pmin, sizeof(PMin) * np, cudaMemcpyDefault);
+  // word, counts, sizes and flags start at 0, the smallest indices at the top
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(word, 0, (unsigned char*)lowest - (unsigned char*)word, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(lowest, 0xff, sizeof(unsigned) * np, st);
+  unsigned nh = 0, hw[2] = {0, 0};
+  void* big = nullptr;
   if (e == cudaSuccess) {
     const int g = grid_for(np);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_bin<<<g, T, 0, st>>>(d_p, np, boxsize, inv, (int)nc, xw, key, count);
-    cgscan::exclusive(count, start, ncells, bsum, word, CG_ST_OTHER, st);
+    k_fof_bin<<<g, T, 0, st>>>(d_p, np, boxsize, inv, (int)nc, key, rank, start);
+    cgscan::exclusive(start, start, ncells + 1, bsum, nullptr, CG_ST_OTHER, st);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_scatter<<<g, T, 0, st>>>(xw, key, np, start, cursor, pos);
+    k_fof_scatter<<<g, T, 0, st>>>(d_p, key, rank, np, boxsize, start, pos, parent);
+    // (the list of dense cells goes where the ranks were)
     prof_mark(st, CG_ST_OTHER);
-    k_fof_init_parent<<<g, T, 0, st>>>(parent, np);
+    k_fof_dense<<<g, T, 0, st>>>(pos, np, start, (int)nc, inv, rank, word + 2);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_link<<<g, T, 0, st>>>(pos, np, start, count, (int)nc, inv, boxsize, ll * ll, parent,
-                                word + 1);
+    k_fof_subsort<<<cg_grid(np, 4), kSubThreads, 0, st>>>(pos, start, (int)nc, inv, rank,
+                                                          word + 2);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_flatten<<<g, T, 0, st>>>(parent, np, size, word + 1);
+    k_fof_boxes<<<g, T, 0, st>>>(pos, np, box);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_roots<<<g, T, 0, st>>>(parent, np, word + 1);
+    k_fof_link<<<g, T, 0, st>>>(pos, np, box, start, (int)nc, inv, boxsize, ll * ll, reach,
+                                parent, word + 1);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_flag<<<g, T, 0, st>>>(parent, size, np, (unsigned)nfof_min, flag);
-    cgscan::exclusive(flag, hid, np, bsum, word, CG_ST_OTHER, st);
+    k_fof_flatten<<<g, T, 0, st>>>(pos, parent, np, size, lowest, word + 1);
+    prof_mark(st, CG_ST_OTHER);
+    k_fof_flag<<<g, T, 0, st>>>(parent, size, lowest, np, (unsigned)nfof_min, flag);
+    cgscan::exclusive(flag, flag, np, bsum, word, CG_ST_OTHER, st);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpy(&nh, word, sizeof(unsigned), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(hw, word, sizeof(hw), cudaMemcpyDeviceToHost);
+    nh = hw[0];
     if (e == cudaSuccess && nh > 0) {
-      e = cudaMalloc(&acc, sizeof(double) * 6 * nh);
-      if (e == cudaSuccess) e = cudaMalloc(&out, sizeof(cg_halo) * nh);
-      if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * 6 * nh, st);
+      // the sums and the catalogue go where the cell keys and ranks were,
+      // unless the halos are so small that they need more
+      const size_t acc_bytes = (sizeof(double) * 6 * (size_t)nh + 15) / 16 * 16;
+      const size_t need = acc_bytes + sizeof(cg_halo) * (size_t)nh;
+      unsigned char* room = (unsigned char*)key;
+      if (need > (size_t)((unsigned char*)pos - room)) {
+        e = cudaMalloc(&big, need);
+        room = (unsigned char*)big;
+      }
+      double* acc = (double*)room;
+      cg_halo* out = (cg_halo*)(room + acc_bytes);
+      if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, acc_bytes, st);
       if (e == cudaSuccess) {
         prof_mark(st, CG_ST_OTHER);
-        k_fof_accum<<<g, T, 0, st>>>(d_p, xw, parent, hid, flag, np, boxsize, acc);
+        k_fof_accum<<<g, T, 0, st>>>(d_p, pos, parent, size, lowest, flag, np,
+                                     (unsigned)nfof_min, boxsize, acc);
         prof_mark(st, CG_ST_OTHER);
-        k_fof_finish<<<g, T, 0, st>>>(xw, size, hid, flag, np, boxsize, acc, out, nh);
+        k_fof_finish<<<g, T, 0, st>>>(d_p, parent, size, lowest, flag, np, (unsigned)nfof_min,
+                                      boxsize, acc, out, nh);
         e = cudaGetLastError();
       }
       const long long ncopy = max_halos < (long long)nh ? max_halos : (long long)nh;
       if (e == cudaSuccess && ncopy > 0)
         e = cudaMemcpy(halos, out, sizeof(cg_halo) * ncopy, cudaMemcpyDeviceToHost);
     }
-    if (e == cudaSuccess) e = cudaMemcpy(&errw, word + 1, sizeof(unsigned), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
-  if (!on_device) release(d_p);
-  release(xw); release(key); release(count); release(start); release(cursor); release(pos);
-  release(parent); release(size); release(flag); release(hid); release(bsum); release(word);
-  release(acc); release(out);
+  const unsigned errw = hw[1];
+  cudaFree(big);
+  cudaFree(blk.base);
   if (e != cudaSuccess) {
     char msg[200];
     snprintf(msg, sizeof(msg), "cg_fof: %s", cudaGetErrorString(e));

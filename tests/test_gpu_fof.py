@@ -135,3 +135,35 @@ def test_fof_edge_cases(gpu_lib):
     n = ctypes.c_longlong()
     assert gpu_lib.cg_fof(None, 10, 10.0, 0.5, 32, None, 0, ctypes.byref(n)) != 0
     assert gpu_lib.cg_fof(blob.ctypes.data, 5000, -1.0, 0.5, 32, None, 0, ctypes.byref(n)) != 0
+
+
+@pytest.mark.parametrize("ratio,device_offset", [(0.7, None), (1.5, None), (2.5, 0), (3.3, 8),
+                                                 (4.2, 0), (7.9, None), (31.0, 8)])
+def test_fof_cell_ranges(gpu_lib, ratio, device_offset):
+    """Cells within the linking length on grids of 1 to 31 cells per side (all
+    cells, ranges across the periodic faces in one or two pieces), and device
+    arrays on and off a 16-byte boundary, against the numpy restatement: equal
+    member counts, centres and velocities to float rounding."""
+    import torch
+    from cola_halo_b200.halos import fof
+    L = 50.0
+    ll = np.float32(L / ratio)
+    rng = np.random.default_rng(int(10 * ratio))
+    # pairs on either side of ll, clumps in the corners, and lone particles
+    pts = [rng.uniform(0, L, (300, 3))]
+    for c in ((0.0, 0.0, 0.0), (0.0, L / 2, L), (L / 3, L / 3, L / 3)):
+        pts.append((np.array(c) + rng.normal(0, float(ll) * 0.2, (90, 3))) % L)
+    x = np.minimum(np.concatenate(pts), np.nextafter(np.float32(L), np.float32(0)))
+    p = np.zeros(len(x), dtype=PARTICLE_MIN_DTYPE)
+    p["x"] = x
+    p["v"] = rng.normal(0, 100, (len(x), 3))
+    want = R.fof_halos(p["x"], p["v"], L, ll)
+    if device_offset is None:
+        got = fof(p, L, ll)
+    else:
+        d = torch.zeros(p.nbytes + 16, dtype=torch.uint8, device="cuda")
+        d[device_offset: device_offset + p.nbytes] = torch.from_numpy(p.view(np.uint8).copy())
+        torch.cuda.synchronize()
+        got = fof(d.data_ptr() + device_offset, L, ll, np_count=len(p))
+    assert len(want) >= 1
+    assert_catalogs_match(rows(got), want, L)

@@ -114,7 +114,9 @@ __global__ void __launch_bounds__(THREADS, 2)
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int q = 0; q < 4; q++) tot[d][h][q] = 0.0f;
-  float2 bsum = make_float2(0.0f, 0.0f);           // channels 2 (tid % 8), + 1
+  double2 bsum = make_double2(0.0, 0.0);           // channels 2 (tid % 8), + 1
+  __shared__ float bred[C];
+  if (tid < C) bred[tid] = 0.0f;
 
   // runs in the order (x, z run, y); a CTA takes a contiguous range
   const int nz = (N + RUN - 1) / RUN;
@@ -145,10 +147,11 @@ __global__ void __launch_bounds__(THREADS, 2)
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       const float2* sg = reinterpret_cast<const float2*>(stage + (i & 1) * RUN * C);
+      float2 bs = make_float2(0.0f, 0.0f);
       for (int k = tid; k < len * C / 2; k += THREADS) {
         const float2 v = sg[k];
-        bsum.x += v.x;
-        bsum.y += v.y;
+        bs.x += v.x;
+        bs.y += v.y;
         __nv_bfloat162 t[3];
         split2(v, t);
         const int z = k >> 3, c = 2 * (k & 7);
@@ -156,6 +159,8 @@ __global__ void __launch_bounds__(THREADS, 2)
 #pragma unroll
         for (int s = 0; s < 3; s++) *reinterpret_cast<__nv_bfloat162*>(d + s * PLANE_BYTES) = t[s];
       }
+      bsum.x += bs.x;
+      bsum.y += bs.y;
       __syncthreads();
       const uint32_t a0 = ring + (uint32_t)((((i + ly) & 3) * 3 + lx) * LINE_BYTES) + offA;
       float hi[3][2][4], lo[3][2][4];
@@ -200,17 +205,19 @@ __global__ void __launch_bounds__(THREADS, 2)
         const int ci = (lane >> 2) + (q >> 1) * 8, co = h * 8 + 2 * (lane & 3) + (q & 1);
         atomicAdd(dw + ((warp * 3 + d) * C + ci) * C + co, tot[d][h][q]);
       }
-  // THREADS is a multiple of 8, so a thread kept to one channel pair; the four
-  // lanes of a warp that share it add up first
+  // THREADS is a multiple of 8, so a thread kept to one channel pair; the CTA's
+  // sums meet in shared memory, then one atomic per channel
 #pragma unroll
   for (int o = 8; o < 32; o <<= 1) {
     bsum.x += __shfl_xor_sync(0xffffffffu, bsum.x, o);
     bsum.y += __shfl_xor_sync(0xffffffffu, bsum.y, o);
   }
   if (lane < 8) {
-    atomicAdd(db + 2 * lane, bsum.x);
-    atomicAdd(db + 2 * lane + 1, bsum.y);
+    atomicAdd(bred + 2 * lane, (float)bsum.x);
+    atomicAdd(bred + 2 * lane + 1, (float)bsum.y);
   }
+  __syncthreads();
+  if (tid < C) atomicAdd(db + tid, bred[tid]);
 }
 
 }  // namespace

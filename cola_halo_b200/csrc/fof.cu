@@ -25,11 +25,10 @@
 // error word.
 //
 // 256^3 particles, L = 600, ll = 0.2 spacings, a third of them in halos: the
-// link kernel takes 8.8 ms (12.4 with all 27 neighbour cells and a union-find
-// over the original indices), and the whole call 13.5 to 14.2 ms (26.6).  The link
-// kernel is bound by its chains of dependent L2 loads: cell starts, candidate,
-// parent.  A warp for each crowded cell, its particles held in registers, took
-// 10.6 ms for those cells alone.
+// link kernel takes 5.8 ms (12.4 with all 27 neighbour cells and a union-find
+// over the original indices; 8.8 with one candidate at a time), and the whole call
+// 10.2 ms (26.6).  The link kernel is bound by its chains of dependent L2 loads:
+// cell starts, candidates, parents.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -256,56 +255,99 @@ __global__ void k_fof_boxes(const float4* __restrict__ pos, long long n,
 // periodic face, and rows before the particle's own hold no later slot.
 //
 // In halos, where a warp's 32 slots are a clump of at most two cells across,
-// its lanes take the same ranges (the cells within ll of the clump), so that
-// every candidate is one broadcast load for the warp, and skip the blocks of 32
-// candidates whose box is further than ll from the clump's.  Elsewhere the few
-// candidates are each lane's own.  ra is an ancestor of s: a candidate whose
-// parent it is belongs to the set already, which spares most pairs of a halo the
-// distance and both find_roots.
+// its lanes take the same ranges (the cells within ll of the clump) and skip the
+// blocks of 32 candidates whose box is further than ll from the clump's.  Of a
+// block that is left each lane loads one candidate and finds its root.  Once the
+// clump is one set, candidates of that set drop out by one vote, and a link
+// takes all candidates of the set it joins out too, so that most blocks of a
+// halo cost two loads and no distance.  Elsewhere the few candidates are each
+// lane's own; their parents are loaded four at a time.
+//
+// ra is an ancestor of s: a candidate whose parent or root it is belongs to the
+// set already, for sets never split.
 __global__ void __launch_bounds__(T, 5) k_fof_link(const float4* __restrict__ pos, long long n,
                                                    const float4* __restrict__ box,
                                                    const unsigned* __restrict__ start, int nc,
                                                    float inv, float L, float ll2, float reach,
                                                    int* parent, unsigned* __restrict__ err) {
+  constexpr unsigned kAll = 0xffffffffu;
   const float half = 0.5f * L;
   const int lane = threadIdx.x & 31;
   for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
        base += (long long)gridDim.x * T) {
-    const bool live = base + lane < n;
-    const unsigned s = (unsigned)(live ? base + lane : n - 1);
+    // lanes past the end stand in for the last slot, which has no later one
+    const unsigned s = (unsigned)min(base + lane, n - 1);
     const float4 a = pos[s];
     float4 lo = box[base / 16], hi = box[base / 16 + 1];
     unsigned own = (unsigned)cell_of(a.x, inv, nc) * nc + cell_of(a.y, inv, nc);
     const float wide = fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * inv;
     const bool clump = wide <= 2.0f;
-    if (clump) own = __reduce_min_sync(0xffffffffu, own);
+    if (clump) own = __reduce_min_sync(kAll, own);
     else lo = hi = a;
     int xl, xh, yl, yh, zl, zh;
     cells_within(lo.x, hi.x, reach, L, inv, nc, xl, xh);
     cells_within(lo.y, hi.y, reach, L, inv, nc, yl, yh);
     cells_within(lo.z, hi.z, reach, L, inv, nc, zl, zh);
     int ra = (int)s;
+    // slots t .. end - 1, each lane its own
     const auto test = [&](unsigned t, unsigned end) {
-      for (; t < end; t++) {
-        if (t <= s || __ldcg(parent + t) == ra) continue;
-        if (dist2(a, pos[t], L, half) < ll2) ra = unite(parent, ra, (int)t, err);
+      t = max(t, s + 1);
+      for (; t < end; t += 4) {
+        int pr[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) pr[u] = t + u < end ? __ldcg(parent + t + u) : ra;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (pr[u] != ra && dist2(a, pos[t + u], L, half) < ll2)
+            ra = unite(parent, ra, (int)(t + u), err);
+      }
+    };
+    // slots t .. end - 1 of the block of 32 at `b`, the same for all lanes
+    const auto test_block = [&](unsigned b, unsigned t, unsigned end) {
+      const unsigned c = b + lane;
+      const bool in = c >= t && c < end;
+      const float4 q = pos[in ? c : s];
+      const int rc = in ? find_root(parent, (int)c, err) : -1;
+      ra = find_root(parent, ra, err);
+      int one;
+      __match_all_sync(kAll, ra, &one);
+      unsigned left = __ballot_sync(kAll, in && !(one && rc == ra));
+      while (left) {
+        const int j = __ffs(left) - 1;
+        left &= left - 1;
+        float4 d;
+        d.x = __shfl_sync(kAll, q.x, j);
+        d.y = __shfl_sync(kAll, q.y, j);
+        d.z = __shfl_sync(kAll, q.z, j);
+        const int rj = __shfl_sync(kAll, rc, j);
+        const bool hit = b + j > s && rj != ra && dist2(a, d, L, half) < ll2;
+        if (one) {
+          if (!__any_sync(kAll, hit)) continue;
+          if (lane == 0) ra = unite(parent, ra, rj, err);
+          ra = __shfl_sync(kAll, ra, 0);
+          left &= __ballot_sync(kAll, rc != rj);
+        } else if (hit) {
+          ra = unite(parent, ra, rj, err);
+        }
+        __syncwarp();
       }
     };
     // slots of the cells z0 .. z1 of a row; `near`: no periodic face in between
     const auto range = [&](unsigned row, int z0, int z1, bool near) {
       unsigned t = max(start[row * nc + z0], (unsigned)base + 1);
       const unsigned end = start[row * nc + z1 + 1];
-      if (!live) return;
-      if (!clump || !near) {
+      if (!clump) {
         test(t, end);
         return;
       }
       for (; t < end; t = (t & ~31u) + 32u) {
-        const float4 bl = box[t / 32 * 2], bh = box[t / 32 * 2 + 1];
-        if (bl.x > hi.x + reach || bh.x < lo.x - reach || bl.y > hi.y + reach ||
-            bh.y < lo.y - reach || bl.z > hi.z + reach || bh.z < lo.z - reach)
-          continue;
-        test(t, min(end, (t & ~31u) + 32u));
+        if (near) {
+          const float4 bl = box[t / 32 * 2], bh = box[t / 32 * 2 + 1];
+          if (bl.x > hi.x + reach || bh.x < lo.x - reach || bl.y > hi.y + reach ||
+              bh.y < lo.y - reach || bl.z > hi.z + reach || bh.z < lo.z - reach)
+            continue;
+        }
+        test_block(t & ~31u, t, end);
       }
     };
     for (int x = xl; x <= xh; x++) {

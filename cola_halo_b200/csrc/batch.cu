@@ -104,6 +104,7 @@ PmPlan view(const PmPlan& bufs, const MeshFFT& tab, int N, int factor, float L) 
   // false); from then on each z r2c leaves -1 behind for the next one
   p.keep_dens = false;
   p.dens_reset = false;
+  p.cell_order = false;
   return p;
 }
 
@@ -137,6 +138,7 @@ cudaError_t record_realization(cg_batch* b, Real& r, StreamBufs& sb) {
       // cell order, as cg_sim_move sorts (the pointers the captured kernels
       // get follow the exchange, so every relaunch repeats it)
       if ((e = particles_sort_cells(&r.ps, &r.order, sp.boxsize, st)) != cudaSuccess) return e;
+      p.cell_order = true;
       for (int a = 0; a < 3; a++) {
         cx[a] = r.ps.x[a];
         cv[a] = r.ps.v[a];

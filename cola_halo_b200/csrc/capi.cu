@@ -199,7 +199,7 @@ extern "C" int cg_sim_set_particles(cg_sim* s, const void* particles, long long 
   // forces already computed keep their meaning for particles given again in
   // the same order (the caller's order, which the upload restores)
   if (s->sorted) CG_CHECK(particles_unsort_forces(&s->ps, &s->order, s->st), "unsort forces");
-  s->sorted = false;
+  s->sorted = s->pm.cell_order = false;
   s->ps.n = np;
   s->a_x = a_x;
   s->a_v = a_v;
@@ -275,7 +275,7 @@ extern "C" int cg_sim_move(cg_sim* s) {
     // the caller's view is unchanged: outputs go back through orig
     s->aos_snapshot = false;
     CG_CHECK(particles_sort_cells(&s->ps, &s->order, s->L, s->st), "cell-order sort");
-    s->sorted = true;
+    s->sorted = s->pm.cell_order = true;
   }
   return CG_OK;
 }
@@ -617,7 +617,7 @@ extern "C" int cg_sim_copy_particles(cg_sim* dst, const cg_sim* src) {
   CG_CHECK(cudaMemcpyAsync(dst->ps.orig, src->ps.orig, 4 * n, cudaMemcpyDeviceToDevice, dst->st),
            "copy");
   dst->ps.n = src->ps.n;
-  dst->sorted = src->sorted;
+  dst->sorted = dst->pm.cell_order = src->sorted;
   dst->aos_snapshot = false;
   dst->a_x = src->a_x;
   dst->a_v = src->a_v;

@@ -63,6 +63,8 @@ struct PmPlan {
   bool keep_dens;           // the density must survive the force step (else the z r2c
                             //   resets it to -1 for the next deposit)
   bool dens_reset;          // dens holds -1 everywhere, not the last density
+  bool cell_order;          // the particles handed in are in cell order (reorder.cu), not
+                            //   in the caller's (a lattice, as a rule)
   CUtensorMap ztm[3];       // TMA maps of gsp[0..2] for the z transform's gather
   bool ztm_ok;              //   valid, landing-area form k_zi_tma
   bool zsw_ok;              //   valid, swizzled-tile form k_zi_sw (else, with neither,

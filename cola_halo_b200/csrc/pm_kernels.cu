@@ -134,29 +134,88 @@ __device__ __forceinline__ void deposit_one(float* __restrict__ d, const Cic& c,
   }
 }
 
+// deposit_one of a warp's clouds (every lane calls it; `live` lanes deposit),
+// with neighbouring lanes' clouds added up first where they fall into the same
+// group of four z cells of the same columns.  In lattice order consecutive
+// particles follow one another along z, so at PM factors 1 to 3 runs of
+// several lanes share a group, and the mesh update, bound by the rate of
+// 16-byte atomics in L2, takes one per run.  Sums go down the runs by shuffles
+// (four columns of four cells, and the cell past the group for clouds that
+// straddle its end).  Only the order of the float additions changes.
+__device__ __forceinline__ void deposit_warp(float* __restrict__ d, const Cic& c, bool live,
+                                             int N, float wpar) {
+  const int lane = threadIdx.x & 31;
+  // (i0, j0, k0 / 4): 11, 10 and 8 bits; i0 in [-1, N - 1] reaches the mesh
+  const bool in = live && c.i0 >= -1 && c.i0 < N;
+  const unsigned key =
+      in ? ((unsigned)(c.i0 + 1) << 18) | ((unsigned)c.j0 << 8) | (unsigned)(c.k0 >> 2)
+         : 0xffffffffu;
+  const unsigned before = __shfl_up_sync(0xffffffffu, key, 1);
+  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+  if (heads == 0xffffffffu) {
+    if (in) deposit_one(d, c, N, wpar);
+    return;
+  }
+  const float T2W = __fmul_rn(c.t2, wpar), D2W = __fmul_rn(c.d2, wpar);
+  const int q = c.k0 & 3;
+  float v[4][5];        // columns (i0, j0), (i0, j1), (i1, j0), (i1, j1); cells 0-3 and the next
+#pragma unroll
+  for (int col = 0; col < 4; col++) {
+    const float wi = col & 2 ? c.d1 : c.t1, wj = col & 1 ? D2W : T2W;
+    const float w0 = in ? __fmul_rn(__fmul_rn(c.t3, wi), wj) : 0.0f;
+    const float w1 = in ? __fmul_rn(__fmul_rn(c.d3, wi), wj) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 5; k++) v[col][k] = (k == q ? w0 : 0.0f) + (k == q + 1 ? w1 : 0.0f);
+  }
+  // lanes of this lane's run after it
+  const unsigned later = lane == 31 ? 0u : heads >> (lane + 1);
+  const int rest = later ? __ffs(later) - 1 : 31 - lane;
+  for (int o = 1; __any_sync(0xffffffffu, rest >= o); o <<= 1) {
+    // after the steps 1 .. o/2 a lane holds the sum of itself and the next o - 1
+#pragma unroll
+    for (int col = 0; col < 4; col++)
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        const float t = __shfl_down_sync(0xffffffffu, v[col][k], o);
+        if (rest >= o) v[col][k] += t;
+      }
+  }
+  if (!in || !((heads >> lane) & 1u)) return;
+  const int g = c.k0 & ~3, kn = g + 4 >= N ? 0 : g + 4;
+#pragma unroll
+  for (int col = 0; col < 4; col++) {
+    const int i = col & 2 ? c.i1 : c.i0;
+    if (i < 0 || i >= N) continue;
+    const size_t at = cell(i, col & 1 ? c.j1 : c.j0, 0, N);
+    atomicAdd(reinterpret_cast<float4*>(d + at + g),
+              make_float4(v[col][0], v[col][1], v[col][2], v[col][3]));
+    if (v[col][4] != 0.0f) atomicAdd(d + at + kn, v[col][4]);
+  }
+}
+
 // PtoMesh (pm.c:229-276) incl. the buffer copy of send_buffer_positions
-// (pm.c:437-445, 477-481).  The mesh holds -1 on entry (pm.c:221-224).
+// (pm.c:437-445, 477-481).  The mesh holds -1 on entry (pm.c:221-224).  One
+// particle per thread, so that the CTAs in flight work on neighbouring
+// particles: a grid-stride loop spreads them over the whole lattice and its mesh
+// planes fall out of L2 (halos formed, 256^3 particles: on 512^3 504 us against
+// 1043, on 768^3 813 against 1643).
 __global__ void __launch_bounds__(T) k_deposit(const float* __restrict__ x0,
                                                const float* __restrict__ x1,
                                                const float* __restrict__ x2, long long n,
                                                float* __restrict__ dens, int N, float scale,
                                                float wpar, float x_right, float shiftx,
                                                unsigned* __restrict__ err) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) {
-    const float px = x0[i], py = x1[i], pz = x2[i];
-    Cic c = cic_index(px, py, pz, N, scale);
-    if (!c.ok) {
-      atomicOr(err, isfinite(px) && isfinite(py) && isfinite(pz) ? CG_ERR_BAD_CELL
-                                                                  : CG_ERR_NONFINITE);
-      continue;
-    }
-    deposit_one(dens, c, N, wpar);
-    if (px > x_right) {
-      Cic g = cic_index(__fadd_rn(px, shiftx), py, pz, N, scale);
-      if (g.ok) deposit_one(dens, g, N, wpar);
-    }
+  const long long i = (long long)blockIdx.x * T + threadIdx.x;
+  const bool have = i < n;
+  const float px = have ? x0[i] : 0.0f, py = have ? x1[i] : 0.0f, pz = have ? x2[i] : 0.0f;
+  Cic c = cic_index(px, py, pz, N, scale);
+  if (!c.ok)
+    atomicOr(err, isfinite(px) && isfinite(py) && isfinite(pz) ? CG_ERR_BAD_CELL
+                                                                : CG_ERR_NONFINITE);
+  deposit_warp(dens, c, have && c.ok, N, wpar);
+  if (have && c.ok && px > x_right) {
+    Cic g = cic_index(__fadd_rn(px, shiftx), py, pz, N, scale);
+    if (g.ok) deposit_one(dens, g, N, wpar);
   }
 }
 
@@ -172,8 +231,13 @@ __global__ void __launch_bounds__(T) k_deposit(const float* __restrict__ x0,
 // take the global path, as does every particle of a CTA whose box is large.
 // Shapes of the box deposit (particles per CTA, box cells of shared memory),
 // a schedule parameter per mesh size chosen by cg_sim_tune_deposit on the
-// particles of a run (variant 0 by default); chunk 0: every cloud takes the
-// global atomics (k_deposit).
+// particles of a run; chunk 0: every cloud takes the global atomics
+// (k_deposit).  Variant 0 (the default) is the first box for particles in cell
+// order, where a chunk in a halo covers few cells; in lattice order a chunk
+// spans the box along z whatever its particles do, no box fits, and variant 0
+// takes k_deposit, which merges neighbours along z (us, boxes against that:
+// halos formed, 128^3 on 128^3 76, 53; 256^3 on 512^3 594, 504; on 768^3 895, 813;
+// lattice, 256^3 on 512^3 333, 266; on 768^3 424, 374; 512^3 on 1024^3 2620, 2080).
 struct DepCfg { int chunk, vmax; };
 constexpr DepCfg kDepCfg[PM_NUM_DEP_VARIANTS] = {
     {512, 3072}, {256, 3072}, {1024, 6144}, {2048, 12288}, {512, 6144}, {0, 0}};
@@ -318,16 +382,17 @@ __device__ __forceinline__ float interp_one(const float* __restrict__ m, const C
   return f;
 }
 
-// Grid of the interpolation: 5 CTAs per SM of grid-stride threads, so that
-// the particles in flight at any time are a window of about 190k (about 3
-// particle planes of a 256^3 lattice order).  The mesh planes they gather
-// from, for the three force meshes, then stay in L2 (768^3: about 70 MB
-// against 126 MB): 0.92-0.95 ms per step against 1.15 ms with 16 CTAs per
-// SM, whose 600k-particle window reached about 200 MB of planes.  3 CTAs per
-// SM leave too few warps in flight (1.12 ms).
-constexpr int kInterpCtasPerSm = 5;
-
-__global__ void __launch_bounds__(T) k_interp(const float* __restrict__ x0,
+// One particle per thread, so that the CTAs in flight gather for a window of
+// neighbouring particles, whose mesh planes stay in L2.  40 registers: 6 CTAs
+// per SM.  Alone, us, against a grid of 5 CTAs per SM that strides over the
+// particles: 256^3 particles on 768^3, halos formed: 1000, 1500 (lattice: 490,
+// 530); 512^3 on 1024^3, lattice: 3490, 3590; 128^3 on 384^3: 114, 116.
+//
+// The gather lives on L1 where halos have formed (1000 us there become 1900 with
+// a quarter of L1 and 4200 with the least of it), so the kernel asks for the
+// largest L1 (interp_prefer_l1); without that the SMs may keep the division that
+// the transforms before it, or of another stream, have set.
+__global__ void __launch_bounds__(T, 6) k_interp(const float* __restrict__ x0,
                                               const float* __restrict__ x1,
                                               const float* __restrict__ x2, long long n,
                                               const float* __restrict__ m0,
@@ -336,29 +401,32 @@ __global__ void __launch_bounds__(T) k_interp(const float* __restrict__ x0,
                                               float* __restrict__ f0, float* __restrict__ f1,
                                               float* __restrict__ f2, int N, float scale,
                                               float x_right, float shiftx, int xlo, int xhi) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) {
-    const float px = x0[i], py = x1[i], pz = x2[i];
-    Cic c = cic_index(px, py, pz, N, scale);
-    float a = 0.0f, b = 0.0f, d = 0.0f;
-    if (c.ok) {
-      a = interp_one(m0, c, N, xlo, xhi);
-      b = interp_one(m1, c, N, xlo, xhi);
-      d = interp_one(m2, c, N, xlo, xhi);
-      if (px > x_right) {
-        Cic g = cic_index(__fadd_rn(px, shiftx), py, pz, N, scale);
-        if (g.ok) {
-          a = __fadd_rn(a, interp_one(m0, g, N, xlo, xhi));
-          b = __fadd_rn(b, interp_one(m1, g, N, xlo, xhi));
-          d = __fadd_rn(d, interp_one(m2, g, N, xlo, xhi));
-        }
+  const long long i = (long long)blockIdx.x * T + threadIdx.x;
+  if (i >= n) return;
+  const float px = x0[i], py = x1[i], pz = x2[i];
+  Cic c = cic_index(px, py, pz, N, scale);
+  float a = 0.0f, b = 0.0f, d = 0.0f;
+  if (c.ok) {
+    a = interp_one(m0, c, N, xlo, xhi);
+    b = interp_one(m1, c, N, xlo, xhi);
+    d = interp_one(m2, c, N, xlo, xhi);
+    if (px > x_right) {
+      Cic g = cic_index(__fadd_rn(px, shiftx), py, pz, N, scale);
+      if (g.ok) {
+        a = __fadd_rn(a, interp_one(m0, g, N, xlo, xhi));
+        b = __fadd_rn(b, interp_one(m1, g, N, xlo, xhi));
+        d = __fadd_rn(d, interp_one(m2, g, N, xlo, xhi));
       }
     }
-    f0[i] = a;
-    f1[i] = b;
-    f2[i] = d;
   }
+  f0[i] = a;
+  f1[i] = b;
+  f2[i] = d;
+}
+
+cudaError_t interp_prefer_l1() {
+  return cudaFuncSetAttribute((const void*)k_interp, cudaFuncAttributePreferredSharedMemoryCarveout,
+                              cudaSharedmemCarveoutMaxL1);
 }
 
 // ------------------------------------------------------------ FFT passes
@@ -1778,13 +1846,15 @@ cudaError_t pm_colbins_reserve(PmPlan* p, long long n) {
   return e;
 }
 
+unsigned particle_grid(long long n) { return (unsigned)((n + T - 1) / T); }
+
 template <int V>
 void deposit_variant(PmPlan* p, const float* const x[3], long long n, cudaStream_t st) {
   constexpr DepCfg c = kDepCfg[V];
   prof_mark(st, CG_ST_DEPOSIT);
   if constexpr (c.chunk == 0) {
-    k_deposit<<<grid_for(n), T, 0, st>>>(x[0], x[1], x[2], n, p->dens, p->N, p->scale, p->wpar,
-                                         p->x_right, p->shiftx, p->err);
+    k_deposit<<<particle_grid(n), T, 0, st>>>(x[0], x[1], x[2], n, p->dens, p->N, p->scale,
+                                              p->wpar, p->x_right, p->shiftx, p->err);
   } else {
     k_deposit_box<c.chunk, c.vmax><<<(unsigned)((n + c.chunk - 1) / c.chunk), T,
                                      sizeof(float) * c.vmax, st>>>(
@@ -1818,6 +1888,20 @@ void launch_deposit(PmPlan* p, const float* const x[3], long long n, int v, cuda
     case 5: deposit_variant<5>(p, x, n, st); break;
     default: deposit_variant<0>(p, x, n, st);
   }
+}
+
+// The deposit variant of the schedule; 0 leaves the choice to the order of
+// the particles (kDepCfg), and to their number: below kMergeFrom the one-pass
+// deposit is a fraction of a wave and as long as its atomics' latency, and the
+// boxes take no longer (32^3 on 96^3: 31.0 us a force with boxes, 31.3 without;
+// 128^3 on 128^3: 214 and 190) and add each particle's share in one order from
+// run to run.
+constexpr long long kMergeFrom = 1 << 17;
+int deposit_by_order(const PmPlan* p, long long n, int v) {
+  return v == 0 && !p->cell_order && n >= kMergeFrom ? PM_NUM_DEP_VARIANTS - 1 : v;
+}
+int deposit_choice(const PmPlan* p, long long n) {
+  return deposit_by_order(p, n, sched_for(p->N).dep);
 }
 
 bool pm_supported_mesh(int N) {
@@ -1985,6 +2069,7 @@ cudaError_t pm_plan_alloc(PmPlan* p, int N, int factor, float L) {
   CG_TRY(cudaMemset(p->dsum, 0, sizeof(double)));
   CG_TRY(cudaMemset(p->err, 0, sizeof(unsigned)));
   CG_TRY(set_all_smem(N));
+  CG_TRY(interp_prefer_l1());
   bool zexplicit = false;
   const int zmode = z_gather_mode(N, &zexplicit);
   p->zsw_ok = zmode == 2 && encode_zi_maps(p, true);
@@ -2156,7 +2241,7 @@ cudaError_t pm_deposit(PmPlan* p, const float* const x[3], long long n, cudaStre
   p->dens_stale = false;
   if (n > 0) {
     static const bool plain = getenv("COLAGPU_DEPOSIT") && getenv("COLAGPU_DEPOSIT")[0] == 'p';
-    launch_deposit(p, x, n, plain ? PM_NUM_DEP_VARIANTS - 1 : sched_for(p->N).dep, st);
+    launch_deposit(p, x, n, plain ? PM_NUM_DEP_VARIANTS - 1 : deposit_choice(p, n), st);
   }
   return cudaGetLastError();
 }
@@ -2415,7 +2500,7 @@ cudaError_t pm_interp(PmPlan* p, const float* const x[3], long long n, float* co
                       cudaStream_t st) {
   if (n > 0) {
     prof_mark(st, CG_ST_INTERP);
-    k_interp<<<cg_grid(n, kInterpCtasPerSm), T, 0, st>>>(x[0], x[1], x[2], n, p->fmesh[0], p->fmesh[1],
+    k_interp<<<particle_grid(n), T, 0, st>>>(x[0], x[1], x[2], n, p->fmesh[0], p->fmesh[1],
                                         p->fmesh[2], f[0], f[1], f[2], p->N, p->scale,
                                         p->x_right, p->shiftx, 0, p->N);
   }
@@ -2470,11 +2555,11 @@ cudaError_t pm_slab_density(PmPlan* p, int x0, int nx, const float* const x[3], 
                                                n4, -1.0f);
   PmPlan q = *p;
   q.x_right = INFINITY;      // the buffer copies are deposited by the next rank
-  if (n > 0) launch_deposit(&q, x, n, sched_for(N).dep, st);
+  if (n > 0) launch_deposit(&q, x, n, deposit_choice(p, n), st);
   if (nb > 0) {
     prof_mark(st, CG_ST_DEPOSIT);
-    k_deposit<<<grid_for(nb), T, 0, st>>>(bx[0], bx[1], bx[2], nb, p->dens, N, p->scale,
-                                          p->wpar, INFINITY, 0.0f, p->err);
+    k_deposit<<<particle_grid(nb), T, 0, st>>>(bx[0], bx[1], bx[2], nb, p->dens, N, p->scale,
+                                               p->wpar, INFINITY, 0.0f, p->err);
   }
   cudaMemsetAsync(p->dsum, 0, sizeof(double), st);
   prof_mark(st, CG_ST_FZ);
@@ -2534,13 +2619,13 @@ cudaError_t pm_slab_interp(PmPlan* p, int x0, int nx, const float* const x[3], l
   if (x0 < 0 || nx < 1 || x0 + nx > N) return cudaErrorInvalidValue;
   if (n > 0) {
     prof_mark(st, CG_ST_INTERP);
-    k_interp<<<cg_grid(n, kInterpCtasPerSm), T, 0, st>>>(x[0], x[1], x[2], n, p->fmesh[0], p->fmesh[1],
+    k_interp<<<particle_grid(n), T, 0, st>>>(x[0], x[1], x[2], n, p->fmesh[0], p->fmesh[1],
                                         p->fmesh[2], f[0], f[1], f[2], N, p->scale, INFINITY,
                                         0.0f, x0, x0 + nx);
   }
   if (nb > 0) {
     prof_mark(st, CG_ST_INTERP);
-    k_interp<<<grid_for(nb), T, 0, st>>>(bx[0], bx[1], bx[2], nb, p->fmesh[0], p->fmesh[1],
+    k_interp<<<particle_grid(nb), T, 0, st>>>(bx[0], bx[1], bx[2], nb, p->fmesh[0], p->fmesh[1],
                                          p->fmesh[2], bf[0], bf[1], bf[2], N, p->scale,
                                          INFINITY, 0.0f, x0, x0 + nx);
   }
@@ -2591,7 +2676,7 @@ cudaError_t pm_tune_deposit(PmPlan* p, const float* const x[3], long long n, cud
       prof_mark(st, CG_ST_FILL);
       k_fill<<<grid_for((long long)n4), T, 0, st>>>(reinterpret_cast<float4*>(p->dens), n4, -1.0f);
       cudaEventRecord(a, st);
-      launch_deposit(p, x, n, v, st);
+      launch_deposit(p, x, n, deposit_by_order(p, n, v), st);
       cudaEventRecord(b, st);
       e = cudaEventSynchronize(b);
       float tr = 0.0f;

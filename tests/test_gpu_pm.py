@@ -150,3 +150,38 @@ def test_deposit_variants_match_oracle(gpu_lib, bbks_table):
     finally:
         gpu_lib.cg_set_deposit_variant(N, old)
     assert gpu_lib.cg_set_deposit_variant(N, 99) != 0
+
+
+@pytest.mark.parametrize("N", [16, 48])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 257, 300])
+def test_merged_deposit_runs(gpu_lib, N, n):
+    """The deposit that merges neighbouring lanes, at particle counts around a
+    warp's and a block's end: all particles in one cell whose cloud lies inside
+    a group of four cells, straddles two or wraps in z; a walk along z; buffer
+    copies in the last x cell; and two cells in turn.  n float additions onto a
+    cell of at most S, each off by S / 2^24 at most, and three per weight."""
+    from cola_halo_b200 import PARTICLE_DTYPE, Simulation
+    L = float(N)
+    i = np.arange(n)
+    u = np.random.default_rng(n).uniform(0.05, 0.95, (n, 3))
+    patterns = {
+        "inside": u + [5, 6, 8], "straddle": u + [5, 6, 7], "wrap": u + [5, N - 1, N - 1],
+        "walk": np.stack([u[:, 0] + 3, u[:, 1] + 9, (0.3 * i) % N], axis=1),
+        "copy": u + [N - 1, 2, 11], "turns": u + np.where(i % 2, 4, 10)[:, None],
+    }
+    old = gpu_lib.cg_get_deposit_variant(N)
+    assert gpu_lib.cg_set_deposit_variant(N, gpu_lib.cg_deposit_variants() - 1) == 0
+    try:
+        sim = Simulation(N, N, L, OM, np_capacity=max(n, N ** 3))
+        sim.keep_density(True)
+        for name, x in patterns.items():
+            p = np.zeros(n, dtype=PARTICLE_DTYPE)
+            p["x"] = x
+            sim.set_particles(p, 0.1, 0.1)
+            sim.forces()
+            want = R.cic_deposit(p["x"].copy(), N, L, 1)
+            tol = (n + 8) * 2.0 ** -24 * (np.abs(want).max() + 2)
+            assert np.abs(sim.get_mesh(0) - want).max() <= tol, name
+        sim.close()
+    finally:
+        gpu_lib.cg_set_deposit_variant(N, old)

@@ -417,12 +417,14 @@ struct SmemSw8 {
 };
 
 // Global lines with compile-time strides: element n of line b at
-// p[b * LS + n * ES] (a stage's legs then sit at constant offsets).
-template <size_t LS, size_t ES>
+// p[b * LS + n * ES] (a stage's legs then sit at constant offsets).  RO:
+// loads through the read-only path, for memory the kernel does not write.
+template <size_t LS, size_t ES, bool RO = true>
 struct GmemC {
   float2* p;
   __device__ __forceinline__ cplx ld(int b, int n) const {
-    const float2 v = __ldg(p + (size_t)b * LS + (size_t)n * ES);
+    const float2* q = p + (size_t)b * LS + (size_t)n * ES;
+    const float2 v = RO ? __ldg(q) : *q;
     return cplx{v.x, v.y};
   }
   __device__ __forceinline__ void st(int b, int n, cplx v) const {

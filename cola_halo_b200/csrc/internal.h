@@ -69,7 +69,7 @@ struct PmPlan {
   bool ztm_ok;              //   valid, landing-area form k_zi_tma
   bool zsw_ok;              //   valid, swizzled-tile form k_zi_sw (else, with neither,
                             //   the cp.async gather runs)
-  CUtensorMap xtm[3];       // TMA maps of spec, gsp[1], gsp[2] for the x pass's gather
+  CUtensorMap xtm[2];       // TMA maps of spec, gsp[1] for the x pass's gather
   bool xsw_ok;              //   valid (else the x pass loads directly)
   int xtm_tk;               //   the columns per CTA the maps were encoded for
   bool dens_stale;          // dens does not hold the last force step's density (the
@@ -103,8 +103,8 @@ cudaError_t mesh_r2c(const MeshFFT* f, const float* real, float2* spec, cudaStre
 cudaError_t mesh_c2r(const MeshFFT* f, float2* spec, float* real, cudaStream_t st);
 
 // Schedule of the FFT passes of one mesh size: which compiled variant of the
-// strided x pass and of the fused Green pass runs (pm_kernels.cu kFxCfg,
-// kGreenCfg).  Variants other than 0 exist from 256 up (Green: up to 768).
+// strided x pass and of the fused Green pass runs (pm_kernels.cu fx_cfg,
+// green_cfg).  Variants other than 0 exist from 256 up (Green: up to 768).
 #define PM_NUM_FX_VARIANTS 3
 #define PM_NUM_GREEN_VARIANTS 7
 #define PM_NUM_DEP_VARIANTS 6

@@ -47,6 +47,7 @@ bool x_maps_for(PmPlan* p, int tk);
 namespace {
 
 constexpr int T = CG_THREADS;
+constexpr size_t kL2Bytes = (size_t)126 << 20;
 constexpr int TY = 16;   // z-lines per CTA in FZ / ZI
 constexpr int BY = 8;    // y-lines per CTA in FY
 
@@ -441,12 +442,10 @@ using cgfft::SmemLine;
 // Schedules of the strided x pass and the fused y Green pass.  Variant 0
 // is the default; the others are compiled for meshes from MIN_TUNED_N up
 // and chosen per mesh size by the autotuner (pm_autotune) or set
-// explicitly.  x pass: ky columns per CTA and maximum radix (0: radix 8
-// from 768 up, else 16; -1: the other of the two).  Green pass: lines per
-// CTA, maximum radix and the resident CTAs per SM the kernel is
-// register-limited to.  The Green default is the fastest shape measured at
-// 384 and 768; for the x pass the tuner picks 16 columns (variant 2) there,
-// ahead of the 8-column default.
+// explicitly.  x pass: ky columns per CTA and maximum radix (fx_cfg).  Green
+// pass: lines per CTA, maximum radix and the resident CTAs per SM the kernel
+// is register-limited to.  The Green default is the fastest shape measured
+// at 384 and 768.
 constexpr int MIN_TUNED_N = 256;
 // Variants compiled at size N.  The 8-line Green variants stop at 768: at
 // 1024 they would spill registers.
@@ -456,9 +455,19 @@ __host__ __device__ constexpr int n_fx_variants(int N) {
 __host__ __device__ constexpr int n_green_variants(int N) {
   return N >= MIN_TUNED_N && N <= 768 ? PM_NUM_GREEN_VARIANTS : 1;
 }
+// x pass by mesh size.  Default: 16 columns (128-byte rows) from 256 to 768,
+// where the twiddles sit in shared memory and the 16-column form fits 2 CTAs
+// per SM; 8 columns at 1024, where they do not and it would fit one; 8 below
+// 256, where 16 would leave fewer CTAs than SMs have room for.  One inverse
+// launch, ms, as {16 columns radix 16, 8 columns radix 16, 8 columns radix 8}:
+// 256: 0.024, 0.029, 0.029; 384: 0.079, 0.084, 0.097; 512: 0.183, 0.193,
+// 0.182; 768: 0.566, 0.654, 0.734; 1024: 2.04, 1.53, 1.81.
 struct FxCfg { int tk, rm; };
+__host__ __device__ constexpr FxCfg fx_cfg(int N, int v) {
+  const bool wide = N >= 256 && N < 1024;
+  return v == 1 ? FxCfg{8, 8} : ((v == 0) == wide ? FxCfg{16, 16} : FxCfg{8, 16});
+}
 struct GreenCfg { int byg, rm, minb, thr; };
-constexpr FxCfg kFxCfg[PM_NUM_FX_VARIANTS] = {{8, 0}, {8, -1}, {16, 16}};
 // (lines per CTA, maximum radix, CTAs per SM, threads): at 768 a radix-16
 // stage has 48 butterflies per line, so 8 lines fill 384 threads, 4 lines
 // 192 and 2 lines 96 once each; 2 lines on 128 threads split the radix-3
@@ -469,11 +478,6 @@ constexpr FxCfg kFxCfg[PM_NUM_FX_VARIANTS] = {{8, 0}, {8, -1}, {16, 16}};
 constexpr GreenCfg kGreenCfg[PM_NUM_GREEN_VARIANTS] = {
     {2, 16, 7, 128}, {8, 8, 2, 256}, {8, 16, 2, 384}, {4, 16, 4, 192}, {2, 16, 8, 96},
     {2, 16, 8, 128}, {4, 16, 3, 256}};
-__host__ __device__ constexpr int rm_x_default(int N) { return N >= 768 ? 8 : 16; }
-__host__ __device__ constexpr int fx_rm(int N, int v) {
-  return kFxCfg[v].rm == 0 ? rm_x_default(N)
-                           : (kFxCfg[v].rm < 0 ? 24 - rm_x_default(N) : kFxCfg[v].rm);
-}
 
 // FZ: r2c along z of R (TY z-lines (x, y0..y0+TY-1) per CTA) through a
 // complex FFT of length H = N/2 on (x_2m + i x_2m+1):
@@ -838,6 +842,12 @@ template <int TKV> struct SwTile;
 template <> struct SwTile<8> { using type = cgfft::SmemSw8; };
 template <> struct SwTile<16> { using type = cgfft::SmemSw16; };
 
+// n_x as a float by exact integer and float additions (|n_x| < 2^22), which
+// run at the full rate where a conversion runs at a quarter of it.
+__device__ __forceinline__ float signed_index(int n, int N) {
+  return __fsub_rn(__int_as_float(0x4b400000 + (n <= N / 2 ? n : n - N)), 12582912.0f);
+}
+
 // Shared tile element scaled on load like GmemScaled (SCALE 1: n_x or the
 // gradient table at n; 2: the plane's n_z).
 template <class S, int SCALE>
@@ -848,26 +858,24 @@ struct SmemScaled {
   const float* g;
   __device__ __forceinline__ cplx ld(int b, int n) const {
     const cplx v = t.ld(b, n);
-    const float f = SCALE == 1 ? (g ? __ldg(g + n) : (float)(n <= N / 2 ? n : n - N)) : fz;
+    const float f = SCALE == 1 ? (g ? __ldg(g + n) : signed_index(n, N)) : fz;
     return cplx{__fmul_rn(v.x, f), __fmul_rn(v.y, f)};
   }
   __device__ __forceinline__ void st(int b, int n, cplx v) const { t.st(b, n, v); }
   static constexpr bool kShared = true;
 };
 
-template <int N, int DIR, int SCALE, int TKV, int RMX>
-__global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap tm,
-                                             float2* out, const float2* __restrict__ twN,
-                                             const float* __restrict__ gtab,
+// The gather of one CTA of the TMA x pass: columns 2 TKV bx .. of plane kz of
+// the spectrum behind tm into the swizzled tile at `base`, the twiddle pack
+// copied meanwhile; every thread waits, bounded.  False when the loads did
+// not complete.
+template <int N, int TKV, int RMX>
+__device__ __forceinline__ bool fx_sw_gather(const CUtensorMap& tm, unsigned char* base, int bx,
+                                             int kz, const float2* __restrict__ twN,
                                              unsigned* __restrict__ err) {
   static_assert(N % fx_nbox<N>() == 0 && fx_krows<N>() % 8 == 0, "box rows");
   constexpr int KR = fx_krows<N>(), NB = fx_nbox<N>();
   constexpr unsigned kBytes = (unsigned)(sizeof(float2) * N * TKV);
-  extern __shared__ __align__(16) unsigned char smraw[];
-  unsigned char* base =
-      smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
-  using Tile = typename SwTile<TKV>::type;
-  const Tile t{reinterpret_cast<cplx*>(base)};
   const unsigned bar = (unsigned)__cvta_generic_to_shared(base + kBytes);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
@@ -883,22 +891,17 @@ __global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap
       asm volatile(
           "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
           " [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst0 + (unsigned)(sizeof(float2) * TKV * KR * h)),
-          "l"(reinterpret_cast<unsigned long long>(&tm)), "r"((int)(2 * TKV * blockIdx.x)),
-          "r"(h * KR), "r"((int)blockIdx.y), "r"(bar)
+          "l"(reinterpret_cast<unsigned long long>(&tm)), "r"(2 * TKV * bx),
+          "r"(h * KR), "r"(kz), "r"(bar)
           : "memory");
     }
   }
   // the stages' twiddles into shared memory while the tensor loads land
-  using TP = cgfft::TwPack<N, RMX, false, false>;
-  float2* tws = reinterpret_cast<float2*>(base + kBytes + 16);
   if constexpr (tw_in_smem<N>()) {
-    TP::template copy<T>(tws, twN);
+    cgfft::TwPack<N, RMX, false, false>::template copy<T>(
+        reinterpret_cast<float2*>(base + kBytes + 16), twN);
     __syncthreads();
   }
-  const auto tw = [&] {
-    if constexpr (tw_in_smem<N>()) return TP{tws};
-    else return twN;
-  }();
   unsigned done = 0;
   for (int it = 0; it < (1 << 22) && !done; it++) {
     asm volatile(
@@ -906,18 +909,75 @@ __global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap
         " selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done) : "r"(bar) : "memory");
   }
-  if (!done) {
-    if (threadIdx.x == 0) atomicOr(err, (unsigned)CG_ERR_TMA_WAIT);
-    return;
-  }
-  const size_t off = (size_t)blockIdx.y * N * N + blockIdx.x * TKV;
-  const cgfft::GmemC<1, N> go{out + off};
-  if constexpr (SCALE == 0) {
-    cgfft::fft_io<N, TKV, T, false, DIR, RMX>(t, t, go, tw);
+  if (!done && threadIdx.x == 0) atomicOr(err, (unsigned)CG_ERR_TMA_WAIT);
+  return done != 0;
+}
+
+// The twiddles of that CTA: the pack after the tile, or the table.
+template <int N, int TKV, int RMX>
+__device__ __forceinline__ auto fx_sw_twiddles(unsigned char* base,
+                                               const float2* __restrict__ twN) {
+  if constexpr (tw_in_smem<N>())
+    return cgfft::TwPack<N, RMX, false, false>{
+        reinterpret_cast<float2*>(base + sizeof(float2) * N * TKV + 16)};
+  else
+    return twN;
+}
+
+__device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
+  return p + ((1024u - ((unsigned)__cvta_generic_to_shared(p) & 1023u)) & 1023u);
+}
+
+// Forward x pass, in place.
+template <int N, int TKV, int RMX>
+__global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap tm,
+                                             float2* out, const float2* __restrict__ twN,
+                                             unsigned* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  unsigned char* base = align1024(smraw);
+  if (!fx_sw_gather<N, TKV, RMX>(tm, base, (int)blockIdx.x, (int)blockIdx.y, twN, err)) return;
+  using Tile = typename SwTile<TKV>::type;
+  const Tile t{reinterpret_cast<cplx*>(base)};
+  const cgfft::GmemC<1, N> go{out + (size_t)blockIdx.y * N * N + blockIdx.x * TKV};
+  cgfft::fft_io<N, TKV, T, false, -1, RMX>(t, t, go, fx_sw_twiddles<N, TKV, RMX>(base, twN));
+}
+
+// Inverse x passes of the force components c0 + blockIdx.z (all three in one
+// launch, or one).  x (0) and z (2) read the shared spectrum (`shared`), scaled
+// by n_x or n_z, into their own outputs; y (1) is transformed in place.  One
+// launch of the three, one after the other, in us against three launches: 192:
+// 40, 49; 384: 214, 246; 512: 535, 562; 768: 1729, 1762; 1024: 5133, 5475 (the
+// components side by side, so that x and z read a tile together, took 41, 237,
+// 556, 1806 and 5387: the three output streams cost more than the shared reads
+// gain).
+struct FxInvArgs {
+  int c0;
+  float2* out[3];
+  const float* gtab;        // gradient table (NULL: the signed index)
+};
+
+template <int N, int TKV, int RMX>
+__global__ void __launch_bounds__(T) k_fx_inv_sw(const __grid_constant__ CUtensorMap shared,
+                                                 const __grid_constant__ CUtensorMap tmy,
+                                                 const __grid_constant__ FxInvArgs a,
+                                                 const float2* __restrict__ twN,
+                                                 unsigned* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  unsigned char* base = align1024(smraw);
+  const int c = a.c0 + (int)blockIdx.z, bx = (int)blockIdx.x, kz = (int)blockIdx.y;
+  if (!fx_sw_gather<N, TKV, RMX>(c == 1 ? tmy : shared, base, bx, kz, twN, err)) return;
+  using Tile = typename SwTile<TKV>::type;
+  const Tile t{reinterpret_cast<cplx*>(base)};
+  const auto tw = fx_sw_twiddles<N, TKV, RMX>(base, twN);
+  const cgfft::GmemC<1, N> go{a.out[c] + (size_t)kz * N * N + bx * TKV};
+  if (c == 1) {
+    cgfft::fft_io<N, TKV, T, false, 1, RMX>(t, t, go, tw);
+  } else if (c == 0) {
+    const SmemScaled<Tile, 1> ts{t, N, 0.0f, a.gtab};
+    cgfft::fft_io<N, TKV, T, false, 1, RMX>(ts, t, go, tw);
   } else {
-    const float fz = SCALE == 2 && gtab ? __ldg(gtab + blockIdx.y) : (float)blockIdx.y;
-    const SmemScaled<Tile, SCALE> ts{t, N, fz, gtab};
-    cgfft::fft_io<N, TKV, T, false, DIR, RMX>(ts, t, go, tw);
+    const SmemScaled<Tile, 2> ts{t, N, a.gtab ? __ldg(a.gtab + kz) : (float)kz, a.gtab};
+    cgfft::fft_io<N, TKV, T, false, 1, RMX>(ts, t, go, tw);
   }
 }
 
@@ -1016,13 +1076,12 @@ __device__ __noinline__ void fft_tile_y(const First f, const Mid m, const Last l
 //   g1 = IFFT_y(i f1 n_y/|n|^2 delta)       the y component
 //   g2 = IFFT_y(i f1/|n|^2 delta)           the x and z components before
 // their factor n_x / n_z, which is constant along a y line and is applied
-// by the inverse x pass as it loads g2 (k_fx, SCALE 1 and 2): one inverse
-// transform serves both components.  BG lines (kz, kx0 .. kx0+BG-1) per
+// by the inverse x pass as it loads g2 (k_fx_inv_sw; k_fx, SCALE 1 and 2):
+// one inverse transform serves both components.  BG lines (kz, kx0 .. kx0+BG-1) per
 // CTA of TG threads; N is a multiple of BG so the lines of a CTA share kz.
 template <int N, int BG, int RMG, int MINB, int TG, bool MODS>
-__global__ void __launch_bounds__(TG, MINB) k_green(const float2* __restrict__ spec,
-                                                         float2* __restrict__ g1,
-                                                         float2* __restrict__ g2,
+__global__ void __launch_bounds__(TG, MINB) k_green(float2* spec, float2* __restrict__ g1,
+                                                    float2* g2,
                                                          const float2* __restrict__ twN,
                                                          float f1, GreenMods gm) {
   constexpr int P = cgfft::line_pitch<N>();
@@ -1033,7 +1092,9 @@ __global__ void __launch_bounds__(TG, MINB) k_green(const float2* __restrict__ s
   const int kz = (int)(l0 / N) + gm.kz0;
   const int kx0 = (int)(l0 % N);
   const size_t off = l0 * N;
-  const cgfft::GmemC<N, 1> gin{const_cast<float2*>(spec) + off};
+  // g2 may be spec itself (a CTA reads its lines before it writes them), so
+  // they are read by plain loads
+  const cgfft::GmemC<N, 1, false> gin{spec + off};
   const SmemLine<P> d{D}, w{W};
   fft_tile_y<N, BG, RMG, TG, -1>(gin, d, d, twN);
   // the y component's load also leaves the shared x/z value in D
@@ -1280,9 +1341,15 @@ __device__ __forceinline__ void zsw_halfcomplex(const cgfft::SmemSw16& t,
   }
 }
 
+// blockIdx.z: the component, of the spectra and meshes in `a` (one launch for
+// all three where they follow one another, one component alone otherwise).
+struct ZiArgs {
+  CUtensorMap tm[3];
+  float* out[3];
+};
+
 template <int N>
-__global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_constant__ CUtensorMap tm,
-                                             float* __restrict__ out,
+__global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_constant__ ZiArgs a,
                                              const float2* __restrict__ twH,
                                              const float2* __restrict__ twN,
                                              unsigned* __restrict__ err) {
@@ -1306,7 +1373,7 @@ __global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_cons
   // memory while the tensor loads land
   using TP = ZswPack<N>;
   float2* tws = reinterpret_cast<float2*>(base + kBytes + 16);
-  if (!zsw_gather<N>(tm, base, bar, 0, x, y0, [&] {
+  if (!zsw_gather<N>(a.tm[blockIdx.z], base, bar, 0, x, y0, [&] {
         if constexpr (zsw_pack<N>()) TP::template copy<T>(tws, twH);
       })) {
     if (threadIdx.x == 0) atomicOr(err, (unsigned)CG_ERR_TMA_WAIT);
@@ -1314,7 +1381,7 @@ __global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_cons
   }
   zsw_halfcomplex<N>(t, twN);
   __syncthreads();
-  const cgfft::GmemC<H, 1> gout{reinterpret_cast<float2*>(out) + ((size_t)x * N + y0) * H};
+  const cgfft::GmemC<H, 1> gout{reinterpret_cast<float2*>(a.out[blockIdx.z]) + ((size_t)x * N + y0) * H};
   if constexpr (zsw_pack<N>())
     cgfft::fft_io<H, TY, T, false, 1, 16, true>(t, t, gout, TP{tws});
   else
@@ -1594,17 +1661,15 @@ struct MeshKernels {
   void (*fxi)(const float2*, float2*, const float2*, const float*);
   void (*fxi_x)(const float2*, float2*, const float2*, const float*);   // input times n_x
   void (*fxi_z)(const float2*, float2*, const float2*, const float*);   // input times n_z
-  // the same four with the TMA gather (k_fx_sw)
-  void (*fxf_sw)(CUtensorMap, float2*, const float2*, const float*, unsigned*);
-  void (*fxi_sw)(CUtensorMap, float2*, const float2*, const float*, unsigned*);
-  void (*fxi_x_sw)(CUtensorMap, float2*, const float2*, const float*, unsigned*);
-  void (*fxi_z_sw)(CUtensorMap, float2*, const float2*, const float*, unsigned*);
+  // the forward pass and the three inverse ones with the TMA gather
+  void (*fxf_sw)(CUtensorMap, float2*, const float2*, unsigned*);
+  void (*fxi3_sw)(CUtensorMap, CUtensorMap, FxInvArgs, const float2*, unsigned*);
   size_t sm_fx_sw;
-  void (*green)(const float2*, float2*, float2*, const float2*, float, GreenMods);
-  void (*green_mods)(const float2*, float2*, float2*, const float2*, float, GreenMods);
+  void (*green)(float2*, float2*, float2*, const float2*, float, GreenMods);
+  void (*green_mods)(float2*, float2*, float2*, const float2*, float, GreenMods);
   void (*zi)(const float2*, float*, const float2*, const float2*);
   void (*zi_tma)(CUtensorMap, float*, const float2*, const float2*, unsigned*);
-  void (*zi_sw)(CUtensorMap, float*, const float2*, const float2*, unsigned*);
+  void (*zi_sw)(ZiArgs, const float2*, const float2*, unsigned*);
   void (*zip)(CUtensorMap, const float2*, const float4*, const unsigned*, float*, float*,
               const float2*, const float2*, float, unsigned*);
   size_t sm_fz, sm_fy, sm_fx, sm_green, sm_zi, sm_zi_tma, sm_zi_sw;
@@ -1615,15 +1680,13 @@ struct MeshKernels {
 
 template <int N, int V>
 void set_fx(MeshKernels* k) {
-  constexpr int TKV = kFxCfg[V].tk, RMX = fx_rm(N, V);
+  constexpr int TKV = fx_cfg(N, V).tk, RMX = fx_cfg(N, V).rm;
   k->fxf = k_fx<N, -1, 0, TKV, RMX>;
   k->fxi = k_fx<N, 1, 0, TKV, RMX>;
   k->fxi_x = k_fx<N, 1, 1, TKV, RMX>;
   k->fxi_z = k_fx<N, 1, 2, TKV, RMX>;
-  k->fxf_sw = k_fx_sw<N, -1, 0, TKV, RMX>;
-  k->fxi_sw = k_fx_sw<N, 1, 0, TKV, RMX>;
-  k->fxi_x_sw = k_fx_sw<N, 1, 1, TKV, RMX>;
-  k->fxi_z_sw = k_fx_sw<N, 1, 2, TKV, RMX>;
+  k->fxf_sw = k_fx_sw<N, TKV, RMX>;
+  k->fxi3_sw = k_fx_inv_sw<N, TKV, RMX>;
   k->sm_fx_sw = fx_sw_smem<N, TKV, RMX>();
   k->sm_fx = sizeof(cplx) * cgfft::col_tile_elems<N, TKV>();
   k->tk = TKV;
@@ -1728,9 +1791,7 @@ cudaError_t set_all_smem(int N) {
     if (e == cudaSuccess) e = set_smem((const void*)k.fxi_x, k.sm_fx);
     if (e == cudaSuccess) e = set_smem((const void*)k.fxi_z, k.sm_fx);
     if (e == cudaSuccess) e = set_smem((const void*)k.fxf_sw, k.sm_fx_sw);
-    if (e == cudaSuccess) e = set_smem((const void*)k.fxi_sw, k.sm_fx_sw);
-    if (e == cudaSuccess) e = set_smem((const void*)k.fxi_x_sw, k.sm_fx_sw);
-    if (e == cudaSuccess) e = set_smem((const void*)k.fxi_z_sw, k.sm_fx_sw);
+    if (e == cudaSuccess) e = set_smem((const void*)k.fxi3_sw, k.sm_fx_sw);
     if (e == cudaSuccess) e = set_smem((const void*)k.green, k.sm_green);
     if (e == cudaSuccess) e = set_smem((const void*)k.green_mods, k.sm_green);
     if (e == cudaSuccess) e = set_smem((const void*)k.zi, k.sm_zi);
@@ -1997,8 +2058,9 @@ cudaError_t pm_autotune(PmPlan* p, cudaStream_t st, MeshSched* best, float* ms_g
       const bool sw = x_maps_for(p, k.tk);
       prof_mark(st, CG_ST_OTHER);
       if (sw)
-        k.fxi_x_sw<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx_sw, st>>>(p->xtm[2], p->gsp[0],
-                                                                     p->twN, nullptr, p->err);
+        k.fxi3_sw<<<dim3(N / k.tk, N / 2 + 1, 3), T, k.sm_fx_sw, st>>>(
+            p->xtm[0], p->xtm[1], FxInvArgs{0, {p->gsp[0], p->gsp[1], p->gsp[2]}, nullptr},
+            p->twN, p->err);
       else
         k.fxi_x<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->gsp[2], p->gsp[0], p->twN,
                                                                nullptr);
@@ -2252,7 +2314,7 @@ void launch_fx_fwd(PmPlan* p, const MeshKernels& k, cudaStream_t st) {
   prof_mark(st, CG_ST_FX_FWD);
   if (x_maps_for(p, k.tk))
     k.fxf_sw<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx_sw, st>>>(p->xtm[0], p->spec, p->twN,
-                                                               nullptr, p->err);
+                                                               p->err);
   else
     k.fxf<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->spec, p->spec, p->twN, nullptr);
 }
@@ -2272,7 +2334,7 @@ cudaError_t pm_r2c(PmPlan* p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-void launch_zi(const PmPlan* p, const MeshKernels& k, int a, cudaStream_t st);
+void launch_zi(const PmPlan* p, const MeshKernels& k, int a, int n, cudaStream_t st);
 
 // The column bins of the particles' clouds for this force step: counts with
 // warp-aggregated ranks, their prefix sum, the entries.  With f, the
@@ -2349,22 +2411,33 @@ cudaError_t pm_force_mesh(PmPlan* p, int a, cudaStream_t st) {
   if (!p->fmesh_stale) return cudaSuccess;
   MeshKernels k;
   get_kernels(p->N, &k);
-  prof_mark(st, CG_ST_ZI);
-  launch_zi(p, k, a, st);
+  launch_zi(p, k, a, 1, st);
   return cudaGetLastError();
 }
 
-// z c2r of component a: gsp[a] -> fmesh[a], by the TMA gather where the
-// plan holds its tensor maps
-void launch_zi(const PmPlan* p, const MeshKernels& k, int a, cudaStream_t st) {
+// z c2r of components a .. a + n - 1: gsp -> fmesh, by the TMA gather where
+// the plan holds its tensor maps
+void launch_zi(const PmPlan* p, const MeshKernels& k, int a, int n, cudaStream_t st) {
   const int N = p->N;
   const dim3 gz(N / TY, N);
-  if (p->zsw_ok)
-    k.zi_sw<<<gz, T, k.sm_zi_sw, st>>>(p->ztm[a], p->fmesh[a], p->twH, p->twN, p->err);
-  else if (p->ztm_ok)
-    k.zi_tma<<<gz, T, k.sm_zi_tma, st>>>(p->ztm[a], p->fmesh[a], p->twH, p->twN, p->err);
-  else
-    k.zi<<<gz, T, k.sm_zi, st>>>(p->gsp[a], p->fmesh[a], p->twH, p->twN);
+  if (p->zsw_ok) {
+    ZiArgs z;
+    for (int i = 0; i < 3; i++) {
+      const int c = a + (i < n ? i : 0);
+      z.tm[i] = p->ztm[c];
+      z.out[i] = p->fmesh[c];
+    }
+    prof_mark(st, CG_ST_ZI);
+    k.zi_sw<<<dim3(N / TY, N, n), T, k.sm_zi_sw, st>>>(z, p->twH, p->twN, p->err);
+    return;
+  }
+  for (int c = a; c < a + n; c++) {
+    prof_mark(st, CG_ST_ZI);
+    if (p->ztm_ok)
+      k.zi_tma<<<gz, T, k.sm_zi_tma, st>>>(p->ztm[c], p->fmesh[c], p->twH, p->twN, p->err);
+    else
+      k.zi<<<gz, T, k.sm_zi, st>>>(p->gsp[c], p->fmesh[c], p->twH, p->twN);
+  }
 }
 
 // Tensor maps of the three spectra for k_zi_tma or (swizzled) k_zi_sw (see
@@ -2401,7 +2474,7 @@ bool encode_zi_maps(PmPlan* p, bool swizzled) {
   return true;
 }
 
-// Tensor maps of the x pass's inputs (spec, gsp[1], gsp[2]) for k_fx_sw
+// Tensor maps of the x pass's inputs (spec, gsp[1]) for k_fx_sw / k_fx_inv_sw
 // with tk columns per CTA: floats (2N, N, N/2+1), box (2 tk, N / nbox, 1),
 // swizzled like the tile.
 bool encode_x_maps(PmPlan* p, int tk) {
@@ -2421,8 +2494,8 @@ bool encode_x_maps(PmPlan* p, int tk) {
   const cuuint64_t strides[2] = {(cuuint64_t)N * 8, (cuuint64_t)N * N * 8};
   const cuuint32_t box[3] = {(cuuint32_t)(2 * tk), (cuuint32_t)(N / nb), 1};
   const cuuint32_t es[3] = {1, 1, 1};
-  float2* const src[3] = {p->spec, p->gsp[1], p->gsp[2]};
-  for (int a = 0; a < 3; a++) {
+  float2* const src[2] = {p->spec, p->gsp[1]};
+  for (int a = 0; a < 2; a++) {
     if (enc(&p->xtm[a], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)src[a], dims, strides, box,
             es, CU_TENSOR_MAP_INTERLEAVE_NONE,
             tk == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
@@ -2444,49 +2517,40 @@ bool x_maps_for(PmPlan* p, int tk) {
   return true;
 }
 
-// The Green pass and the inverse x passes; with zi, each component's z c2r
-// into its force mesh after its x pass.
+// The Green pass and the inverse x passes into gsp[0..2]; with zi, the z c2r
+// of the three into the force meshes.  The shared x/z spectrum replaces the
+// density's in p->spec, so no component's output overwrites an input that
+// another still reads.
 static cudaError_t green_x_zi(PmPlan* p, cudaStream_t st, bool zi) {
   MeshKernels k;
   get_kernels(p->N, &k);
   const int N = p->N;
-  // gsp[1] <- y component, gsp[2] <- the shared x/z spectrum
   prof_mark(st, CG_ST_GREEN);
   const GreenMods gm{p->kfilt_cur >= 0 ? p->kfilt + (size_t)p->kfilt_cur * p->kfilt_n : nullptr,
                      p->kfilt_n, p->kfilt_inv_dn, p->ktab};
   (gm.t || gm.tab ? k.green_mods : k.green)<<<(N / 2 + 1) * N / k.byg, k.tg, k.sm_green, st>>>(
-      p->spec, p->gsp[1], p->gsp[2], p->twN, p->f1, gm);
+      p->spec, p->gsp[1], p->spec, p->twN, p->f1, gm);
   const dim3 gx(N / k.tk, N / 2 + 1);
   const bool xsw = x_maps_for(p, k.tk);
-  // x: n_x * gsp[2] -> gsp[0] (gsp[2] is still needed for z)
-  prof_mark(st, CG_ST_FX_INV);
-  if (xsw)
-    k.fxi_x_sw<<<gx, T, k.sm_fx_sw, st>>>(p->xtm[2], p->gsp[0], p->twN, p->ktab, p->err);
-  else
-    k.fxi_x<<<gx, T, k.sm_fx, st>>>(p->gsp[2], p->gsp[0], p->twN, p->ktab);
-  if (zi) {
-    prof_mark(st, CG_ST_ZI);
-    launch_zi(p, k, 0, st);
-  }
-  // y: in place
-  prof_mark(st, CG_ST_FX_INV);
-  if (xsw)
-    k.fxi_sw<<<gx, T, k.sm_fx_sw, st>>>(p->xtm[1], p->gsp[1], p->twN, nullptr, p->err);
-  else
-    k.fxi<<<gx, T, k.sm_fx, st>>>(p->gsp[1], p->gsp[1], p->twN, nullptr);
-  if (zi) {
-    prof_mark(st, CG_ST_ZI);
-    launch_zi(p, k, 1, st);
-  }
-  // z: n_z * gsp[2], in place
-  prof_mark(st, CG_ST_FX_INV);
-  if (xsw)
-    k.fxi_z_sw<<<gx, T, k.sm_fx_sw, st>>>(p->xtm[2], p->gsp[2], p->twN, p->ktab, p->err);
-  else
-    k.fxi_z<<<gx, T, k.sm_fx, st>>>(p->gsp[2], p->gsp[2], p->twN, p->ktab);
-  if (zi) {
-    prof_mark(st, CG_ST_ZI);
-    launch_zi(p, k, 2, st);
+  // Components per launch.  All three at once, except where one spectrum stays
+  // in L2 from its x pass to its z c2r but three do not (256: 68 MB each): one
+  // after the other there (all at once: 30 us of 380 a force slower).
+  const int nc = zi && xsw && p->spec_bytes < kL2Bytes && 3 * p->spec_bytes > kL2Bytes ? 1 : 3;
+  for (int c = 0; c < 3; c += nc) {
+    if (xsw) {
+      prof_mark(st, CG_ST_FX_INV);
+      k.fxi3_sw<<<dim3(gx.x, gx.y, nc), T, k.sm_fx_sw, st>>>(
+          p->xtm[0], p->xtm[1], FxInvArgs{c, {p->gsp[0], p->gsp[1], p->gsp[2]}, p->ktab}, p->twN,
+          p->err);
+    } else {
+      prof_mark(st, CG_ST_FX_INV);
+      k.fxi_x<<<gx, T, k.sm_fx, st>>>(p->spec, p->gsp[0], p->twN, p->ktab);
+      prof_mark(st, CG_ST_FX_INV);
+      k.fxi<<<gx, T, k.sm_fx, st>>>(p->gsp[1], p->gsp[1], p->twN, nullptr);
+      prof_mark(st, CG_ST_FX_INV);
+      k.fxi_z<<<gx, T, k.sm_fx, st>>>(p->spec, p->gsp[2], p->twN, p->ktab);
+    }
+    if (zi) launch_zi(p, k, c, nc, st);
   }
   return cudaGetLastError();
 }

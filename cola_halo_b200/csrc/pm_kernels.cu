@@ -1609,40 +1609,87 @@ int z_gather_mode(int N, bool* explicit_choice) {
 // conjugate), 1 on the kz = 0 and kz = N/2 planes.  Optional division by the
 // CIC window prod_i sinc^2(pi n_i / N) squared.  acc = [sum w, sum w |n|,
 // sum w |S|^2] per bin, accumulated in double.
-__global__ void __launch_bounds__(T) k_pk_bin(const float2* __restrict__ spec, int N, int nbins,
-                                              int deconv, double* __restrict__ acc) {
-  extern __shared__ double sb[];
+//
+// k_fy_pk is the forward y pass that ends in these sums instead of storing
+// the spectrum, which nothing reads afterwards: one read of the spectrum where
+// a y pass and a separate binning kernel made two reads and a write.  The
+// modes ky and -ky share |n| and are added first.  Along ky the shells follow
+// one another, so the lanes of a warp that fall into one shell are
+// neighbours: their sums meet by shuffles, and each shell takes one
+// shared-memory addition per warp (atomics on doubles, a compare-and-swap
+// loop each, had every lane of a shell wait for the others: 512^3, 0.96 ms for
+// the binning alone).  CTAs are persistent, so the shells leave a CTA once.
+__device__ __forceinline__ double cic_window2(int n, int N) {
+  if (n == 0) return 1.0;
+  const double x = M_PI * n / N;
+  const double sc = sin(x) / x;
+  return sc * sc;
+}
+
+template <int N>
+__global__ void __launch_bounds__(T) k_fy_pk(const float2* __restrict__ spec,
+                                             const float2* __restrict__ twN, int nbins,
+                                             int deconv, double* __restrict__ acc) {
+  constexpr int P = cgfft::line_pitch<N>();
+  constexpr int TILES = (N / 2 + 1) * N / BY;
+  constexpr int SEG = (N / 2 + 1 + 31) / 32;      // warp segments of a line's modes 0 .. N/2
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const SmemLine<P> mid{reinterpret_cast<cplx*>(smraw)};
+  double* sb = reinterpret_cast<double*>(smraw + sizeof(cplx) * BY * P);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < 3 * nbins; i += T) sb[i] = 0.0;
-  __syncthreads();
-  const size_t total = (size_t)(N / 2 + 1) * N * N;
-  for (size_t t = (size_t)blockIdx.x * T + threadIdx.x; t < total; t += (size_t)gridDim.x * T) {
-    const int kz = (int)(t / ((size_t)N * N));
-    const int i = (int)((t / N) % N);
-    const int j = (int)(t % N);
-    const int si = i <= N / 2 ? i : i - N;
-    const int sj = j <= N / 2 ? j : j - N;
-    const double n2 = (double)si * si + (double)sj * sj + (double)kz * kz;
-    const double nm = sqrt(n2);
-    const int b = (int)floor(nm + 0.5) - 1;
-    if (b < 0 || b >= nbins) continue;
-    const double w = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-    const float2 s = spec[t];
-    double p = (double)s.x * s.x + (double)s.y * s.y;
-    if (deconv) {
-      double win = 1.0;
-      const int ns[3] = {si, sj, kz};
-      for (int a = 0; a < 3; a++) {
-        if (ns[a] != 0) {
-          const double x = M_PI * ns[a] / N;
-          const double sc = sin(x) / x;
-          win *= sc * sc;
+  for (int tile = blockIdx.x; tile < TILES; tile += gridDim.x) {
+    const cgfft::GmemC<N, 1> g{const_cast<float2*>(spec) + (size_t)tile * BY * N};
+    __syncthreads();              // the last tile's modes are added
+    cgfft::fft_io<N, BY, T, true, -1>(g, mid, mid, twN);
+    const int kz = tile * BY / N, i0 = tile * BY % N;
+    for (int q = warp; q < BY * SEG; q += T / 32) {
+      const int b = q / SEG, j = (q % SEG) * 32 + lane;
+      const int i = i0 + b, si = i <= N / 2 ? i : i - N;
+      int bin = -1, w = 0;
+      double wn = 0.0, wp = 0.0;
+      if (j <= N / 2) {
+        const double n2 = (double)si * si + (double)j * j + (double)kz * kz;
+        const double nm = sqrt(n2);
+        bin = (int)floor(nm + 0.5) - 1;
+        if (bin >= nbins) bin = -1;
+        if (bin >= 0) {
+          const cplx s = mid.ld(b, j);
+          double p = (double)s.x * s.x + (double)s.y * s.y;
+          w = (kz == 0 || kz == N / 2) ? 1 : 2;
+          wp = w * p;
+          if (j > 0 && j < N / 2) {
+            const cplx m = mid.ld(b, N - j);
+            wp += w * ((double)m.x * m.x + (double)m.y * m.y);
+            w *= 2;
+          }
+          if (deconv) {
+            const double win = cic_window2(si, N) * cic_window2(j, N) * cic_window2(kz, N);
+            wp /= win * win;
+          }
+          wn = w * nm;
         }
       }
-      p /= win * win;
+      // |n| grows with j: equal shells are consecutive lanes (-1, no shell, at
+      // the start for the mean mode and at the end)
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int ob = __shfl_up_sync(0xffffffffu, bin, o), ow = __shfl_up_sync(0xffffffffu, w, o);
+        const double on = __shfl_up_sync(0xffffffffu, wn, o);
+        const double op = __shfl_up_sync(0xffffffffu, wp, o);
+        if (lane >= o && ob == bin) {
+          w += ow;
+          wn += on;
+          wp += op;
+        }
+      }
+      const int next = __shfl_down_sync(0xffffffffu, bin, 1);
+      if (bin >= 0 && (lane == 31 || next != bin)) {
+        atomicAdd(&sb[bin], (double)w);
+        atomicAdd(&sb[nbins + bin], wn);
+        atomicAdd(&sb[2 * nbins + bin], wp);
+      }
     }
-    atomicAdd(&sb[b], w);
-    atomicAdd(&sb[nbins + b], w * nm);
-    atomicAdd(&sb[2 * nbins + b], w * p);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 3 * nbins; i += T)
@@ -1657,6 +1704,7 @@ struct MeshKernels {
               float, float);
   void (*fyf)(float2*, const float2*);
   void (*fyi)(float2*, const float2*);
+  void (*fypk)(const float2*, const float2*, int, int, double*);
   void (*fxf)(const float2*, float2*, const float2*, const float*);
   void (*fxi)(const float2*, float2*, const float2*, const float*);
   void (*fxi_x)(const float2*, float2*, const float2*, const float*);   // input times n_x
@@ -1710,6 +1758,7 @@ MeshKernels make_kernels(MeshSched s) {
   k.dfz = k_dfz<N, 4>;
   k.fyf = k_fy<N, -1>;
   k.fyi = k_fy<N, 1>;
+  k.fypk = k_fy_pk<N>;
   k.zi = k_zi<N>;
   k.zi_tma = k_zi_tma<N>;
   k.sm_zi_tma = zi_tma_smem<N>();
@@ -1786,6 +1835,7 @@ cudaError_t set_all_smem(int N) {
     if (e == cudaSuccess) e = set_smem((const void*)k.dfz, k.sm_fz);
     if (e == cudaSuccess) e = set_smem((const void*)k.fyf, k.sm_fy);
     if (e == cudaSuccess) e = set_smem((const void*)k.fyi, k.sm_fy);
+    if (e == cudaSuccess) e = set_smem((const void*)k.fypk, k.sm_fy + sizeof(double) * 3 * N);
     if (e == cudaSuccess) e = set_smem((const void*)k.fxf, k.sm_fx);
     if (e == cudaSuccess) e = set_smem((const void*)k.fxi, k.sm_fx);
     if (e == cudaSuccess) e = set_smem((const void*)k.fxi_x, k.sm_fx);
@@ -2773,13 +2823,12 @@ cudaError_t pm_power_spectrum(PmPlan* p, const float* const x[3], long long n, i
   cudaMemsetAsync(p->dsum, 0, sizeof(double), st);
   prof_mark(st, CG_ST_FZ);
   k.fz<<<dim3(N / TY, N), T, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
-  prof_mark(st, CG_ST_FX_FWD);
-  k.fxf<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->spec, p->spec, p->twN, nullptr);
-  prof_mark(st, CG_ST_OTHER);
-  k.fyf<<<(N / 2 + 1) * N / BY, T, k.sm_fy, st>>>(p->spec, p->twN);
+  launch_fx_fwd(p, k, st);
   cudaMemsetAsync(acc, 0, sizeof(double) * 3 * nbins, st);
+  const size_t sm = k.sm_fy + sizeof(double) * 3 * nbins;
+  const int tiles = (N / 2 + 1) * N / BY;
+  const int cap = cg_sm_count() * std::max(1, std::min(4, (int)((size_t)220 * 1024 / (sm + 1024))));
   prof_mark(st, CG_ST_OTHER);
-  k_pk_bin<<<grid_for((long long)(N / 2 + 1) * N * N), T, sizeof(double) * 3 * nbins, st>>>(
-      p->spec, N, nbins, deconv, acc);
+  k.fypk<<<std::min(tiles, cap), T, sm, st>>>(p->spec, p->twN, nbins, deconv, acc);
   return cudaGetLastError();
 }

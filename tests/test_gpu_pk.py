@@ -48,3 +48,33 @@ def test_pk_shot_noise_and_bins(gpu_lib, bbks_table):
     # the two deposits differ only by float32 atomic ordering
     np.testing.assert_allclose(p1 - p2, L ** 3 / nc ** 3, rtol=0, atol=1e-6 * np.abs(p1).max())
     assert np.all(np.diff(k1) > 0) and abs(k1[0] - 2 * math.pi / L) < 0.5 * 2 * math.pi / L
+
+
+@pytest.mark.parametrize("N", [16, 48, 144, 192])
+@pytest.mark.parametrize("deconv", [False, True])
+def test_pk_shells_of_all_meshes(gpu_lib, N, deconv):
+    """One shell, shells to the Nyquist wavenumber and shells past the corner of
+    the spectrum, for lines of less than one to several warps of modes: equal
+    mode counts and mean |k|, and the power of a Poisson field.  A float
+    transform's modes are off by a few 2^-24 log2(N^3) of their rms: 2e-5 of the
+    largest power, undivided by the window, covers twice that."""
+    from cola_halo_b200 import PARTICLE_DTYPE, Simulation
+    nc, L = 16, 100.0
+    p = np.zeros(nc ** 3, dtype=PARTICLE_DTYPE)
+    p["x"] = np.random.default_rng(N).uniform(0, L, (nc ** 3, 3))
+    sim = Simulation(nc, N, L, OM)
+    sim.set_particles(p, 1.0, 1.0)
+    sim.move()
+    x = R.wrap(p["x"], L)
+    dens = R.cic_deposit(x, N, L, N / nc)
+    for nbins in (1, N // 2, N):
+        k, pk, modes = sim.power_spectrum(nbins=nbins, deconvolve_cic=deconv)
+        ko, po, co = R.power_spectrum(dens, L, nbins=nbins, deconvolve_cic=deconv)
+        _, flat, _ = R.power_spectrum(dens, L, nbins=nbins, deconvolve_cic=False)
+        np.testing.assert_array_equal(modes, co)
+        ok = co > 0
+        np.testing.assert_allclose(k[ok], ko[ok], rtol=1e-12)
+        # the window divides a shell's power and its error alike
+        gain = po[ok] / flat[ok]
+        assert np.all(np.abs(pk[ok] - po[ok]) <= 2e-5 * flat[ok].max() * gain)
+    sim.close()

@@ -444,8 +444,7 @@ using cgfft::SmemLine;
 // and chosen per mesh size by the autotuner (pm_autotune) or set
 // explicitly.  x pass: ky columns per CTA and maximum radix (fx_cfg).  Green
 // pass: lines per CTA, maximum radix and the resident CTAs per SM the kernel
-// is register-limited to.  The Green default is the fastest shape measured
-// at 384 and 768.
+// is register-limited to (green_cfg).
 constexpr int MIN_TUNED_N = 256;
 // Variants compiled at size N.  The 8-line Green variants stop at 768: at
 // 1024 they would spill registers.
@@ -468,16 +467,29 @@ __host__ __device__ constexpr FxCfg fx_cfg(int N, int v) {
   return v == 1 ? FxCfg{8, 8} : ((v == 0) == wide ? FxCfg{16, 16} : FxCfg{8, 16});
 }
 struct GreenCfg { int byg, rm, minb, thr; };
-// (lines per CTA, maximum radix, CTAs per SM, threads): at 768 a radix-16
-// stage has 48 butterflies per line, so 8 lines fill 384 threads, 4 lines
-// 192 and 2 lines 96 once each; 2 lines on 128 threads split the radix-3
-// stage's 512 butterflies evenly.  The default, 2 lines on 128 threads at 7
-// CTAs per SM, keeps a barrier to 4 warps (768^3: 1.39 ms; 4 lines on 256
-// threads, the earlier default: 1.64 ms; 2 lines on 96 threads: 1.62 ms; 2
-// on 128 at 8 or 6 CTAs per SM: 1.41 and 1.42 ms).
+// The tuned shapes of the Green pass (entry 0 stands for green_cfg's default).
 constexpr GreenCfg kGreenCfg[PM_NUM_GREEN_VARIANTS] = {
     {2, 16, 7, 128}, {8, 8, 2, 256}, {8, 16, 2, 384}, {4, 16, 4, 192}, {2, 16, 8, 96},
     {2, 16, 8, 128}, {4, 16, 3, 256}};
+// (lines per CTA, maximum radix, CTAs per SM, threads).  Variant 0, the default
+// by mesh size: lines and threads such that the radix-16 stages (N / 16
+// butterflies a line) give most threads one each -- 2 lines of 48 on 128 threads
+// at 768, which keep a barrier to 4 warps and split the radix-3 stage evenly
+// (1.38 ms; 2 on 96 threads 1.63, 1 on 64 1.50, 4 on 256 1.64), and more
+// lines on fewer threads below, where the 768 shape leaves most threads
+// without a butterfly and one thread with a serial chain of 16 elements.
+// Alone, us, as {768 shape, this one}: 512: 440, 400; 384: 211, 201; 256: 66,
+// 46; 192: 37, 29; 128: 14.8, 10.5; 96: 10.5, 8.4; with force-kernel tables and
+// a transfer function 256: 149, 92 (4 lines on 64); 192: 85, 50; 128: 37, 17.
+__host__ __device__ constexpr GreenCfg green_cfg(int N, int v) {
+  if (v != 0) return kGreenCfg[v];
+  if (N >= 768) return GreenCfg{2, 16, 7, 128};
+  if (N >= 512) return GreenCfg{2, 16, 8, 64};
+  if (N >= 384) return GreenCfg{4, 16, 7, 128};
+  if (N >= 256) return GreenCfg{4, 16, 8, 96};
+  if (N > 128) return GreenCfg{4, 16, 8, 64};
+  return GreenCfg{8, 16, 8, 64};
+}
 
 // FZ: r2c along z of R (TY z-lines (x, y0..y0+TY-1) per CTA) through a
 // complex FFT of length H = N/2 on (x_2m + i x_2m+1):
@@ -1742,7 +1754,7 @@ void set_fx(MeshKernels* k) {
 
 template <int N, int V>
 void set_green(MeshKernels* k) {
-  constexpr GreenCfg c = kGreenCfg[V];
+  constexpr GreenCfg c = green_cfg(N, V);
   k->green = k_green<N, c.byg, c.rm, c.minb, c.thr, false>;
   k->green_mods = k_green<N, c.byg, c.rm, c.minb, c.thr, true>;
   k->tg = c.thr;

@@ -504,17 +504,29 @@ __host__ __device__ constexpr GreenCfg green_cfg(int N, int v) {
 // nor __restrict__ there.
 template <bool RESET> using DensPtr = typename std::conditional<RESET, float*, const float*>::type;
 
+// Threads of the z r2c and of the TMA x passes by mesh size: those whose
+// radix-16 stages (TY N / 32 butterflies a CTA in z, N / 16 per column in x)
+// fill them in whole rounds.  us with 256 threads and with these: z r2c 512:
+// 275, 261; 384: 134, 119; 128: 10.4, 8.7; x inverse (three components) 1024:
+// 4709, 4408; 192: 34, 31; 144: 16.9, 14.8; 96: 8.3, 6.7.
+__host__ __device__ constexpr int fz_threads(int N) {
+  return N == 128 || N == 144 || (N >= 256 && N <= 512) ? 128 : 256;
+}
+__host__ __device__ constexpr int fx_threads(int N, int tk, int rm) {
+  return N <= 192 || (N >= 1024 && tk == 8 && rm == 16) ? 128 : 256;
+}
+
 // The split of k_fz (after the H-point transform of the TY lines in `mid`):
 // X_k for k = 0..H stored transposed into S[kz][x][y0 + b], and the lines'
 // sum Re Z_0 + Im Z_0 added to *dsum in double.
-template <int N>
+template <int N, int TT>
 __device__ __forceinline__ void fz_split_store(const SmemLine<cgfft::line_pitch<N / 2>()>& mid,
                                                int x, int y0, float2* __restrict__ spec,
                                                const float2* __restrict__ twN,
                                                double* __restrict__ dsum) {
   constexpr int H = N / 2;
   double acc = 0.0;
-  for (int idx = threadIdx.x; idx < (H + 1) * TY; idx += T) {
+  for (int idx = threadIdx.x; idx < (H + 1) * TY; idx += TT) {
     const int b = idx % TY, k = idx / TY;
     const cplx zk = mid.ld(b, k == H ? 0 : k);
     const cplx zc0 = mid.ld(b, k == 0 ? 0 : H - k);
@@ -532,25 +544,25 @@ __device__ __forceinline__ void fz_split_store(const SmemLine<cgfft::line_pitch<
 }
 
 template <int N, bool RESET>
-__global__ void __launch_bounds__(T) k_fz(DensPtr<RESET> dens,
+__global__ void __launch_bounds__(fz_threads(N)) k_fz(DensPtr<RESET> dens,
                                           float2* __restrict__ spec,
                                           const float2* __restrict__ twH,
                                           const float2* __restrict__ twN,
                                           double* __restrict__ dsum) {
-  constexpr int H = N / 2;
+  constexpr int H = N / 2, TT = fz_threads(N);
   extern __shared__ __align__(16) unsigned char smraw[];
   const SmemLine<cgfft::line_pitch<H>()> mid{reinterpret_cast<cplx*>(smraw)};
   const int x = blockIdx.y;
   const int y0 = blockIdx.x * TY;
   const cgfft::GmemC<H, 1> gin{reinterpret_cast<float2*>(const_cast<float*>(dens)) +
                               ((size_t)x * N + y0) * H};
-  cgfft::fft_io<H, TY, T, true, -1>(gin, mid, mid, twH);
+  cgfft::fft_io<H, TY, TT, true, -1>(gin, mid, mid, twH);
   if constexpr (RESET) {
     __syncthreads();    // every thread's loads of the lines are done
     float4* line = reinterpret_cast<float4*>(dens + ((size_t)x * N + y0) * N);
-    for (int i = threadIdx.x; i < TY * N / 4; i += T) line[i] = make_float4(-1.f, -1.f, -1.f, -1.f);
+    for (int i = threadIdx.x; i < TY * N / 4; i += TT) line[i] = make_float4(-1.f, -1.f, -1.f, -1.f);
   }
-  fz_split_store<N>(mid, x, y0, spec, twN, dsum);
+  fz_split_store<N, TT>(mid, x, y0, spec, twN, dsum);
 }
 
 // ------------------------------------------------- column-binned deposit
@@ -771,7 +783,7 @@ __global__ void __launch_bounds__(T, MINB) k_dfz(const float4* __restrict__ ent,
   }
   __syncthreads();
   cgfft::fft_io<H, TY, T, true, -1>(mid, mid, mid, twH);
-  fz_split_store<N>(mid, x, y0, spec, twN, dsum);
+  fz_split_store<N, T>(mid, x, y0, spec, twN, dsum);
 }
 
 // FY: c2c along ky, BY contiguous lines per CTA, in place.
@@ -910,7 +922,7 @@ __device__ __forceinline__ bool fx_sw_gather(const CUtensorMap& tm, unsigned cha
   }
   // the stages' twiddles into shared memory while the tensor loads land
   if constexpr (tw_in_smem<N>()) {
-    cgfft::TwPack<N, RMX, false, false>::template copy<T>(
+    cgfft::TwPack<N, RMX, false, false>::template copy<fx_threads(N, TKV, RMX)>(
         reinterpret_cast<float2*>(base + kBytes + 16), twN);
     __syncthreads();
   }
@@ -942,7 +954,7 @@ __device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
 
 // Forward x pass, in place.
 template <int N, int TKV, int RMX>
-__global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap tm,
+__global__ void __launch_bounds__(fx_threads(N, TKV, RMX)) k_fx_sw(const __grid_constant__ CUtensorMap tm,
                                              float2* out, const float2* __restrict__ twN,
                                              unsigned* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -951,7 +963,7 @@ __global__ void __launch_bounds__(T) k_fx_sw(const __grid_constant__ CUtensorMap
   using Tile = typename SwTile<TKV>::type;
   const Tile t{reinterpret_cast<cplx*>(base)};
   const cgfft::GmemC<1, N> go{out + (size_t)blockIdx.y * N * N + blockIdx.x * TKV};
-  cgfft::fft_io<N, TKV, T, false, -1, RMX>(t, t, go, fx_sw_twiddles<N, TKV, RMX>(base, twN));
+  cgfft::fft_io<N, TKV, fx_threads(N, TKV, RMX), false, -1, RMX>(t, t, go, fx_sw_twiddles<N, TKV, RMX>(base, twN));
 }
 
 // Inverse x passes of the force components c0 + blockIdx.z (all three in one
@@ -969,7 +981,7 @@ struct FxInvArgs {
 };
 
 template <int N, int TKV, int RMX>
-__global__ void __launch_bounds__(T) k_fx_inv_sw(const __grid_constant__ CUtensorMap shared,
+__global__ void __launch_bounds__(fx_threads(N, TKV, RMX)) k_fx_inv_sw(const __grid_constant__ CUtensorMap shared,
                                                  const __grid_constant__ CUtensorMap tmy,
                                                  const __grid_constant__ FxInvArgs a,
                                                  const float2* __restrict__ twN,
@@ -983,13 +995,13 @@ __global__ void __launch_bounds__(T) k_fx_inv_sw(const __grid_constant__ CUtenso
   const auto tw = fx_sw_twiddles<N, TKV, RMX>(base, twN);
   const cgfft::GmemC<1, N> go{a.out[c] + (size_t)kz * N * N + bx * TKV};
   if (c == 1) {
-    cgfft::fft_io<N, TKV, T, false, 1, RMX>(t, t, go, tw);
+    cgfft::fft_io<N, TKV, fx_threads(N, TKV, RMX), false, 1, RMX>(t, t, go, tw);
   } else if (c == 0) {
     const SmemScaled<Tile, 1> ts{t, N, 0.0f, a.gtab};
-    cgfft::fft_io<N, TKV, T, false, 1, RMX>(ts, t, go, tw);
+    cgfft::fft_io<N, TKV, fx_threads(N, TKV, RMX), false, 1, RMX>(ts, t, go, tw);
   } else {
     const SmemScaled<Tile, 2> ts{t, N, a.gtab ? __ldg(a.gtab + kz) : (float)kz, a.gtab};
-    cgfft::fft_io<N, TKV, T, false, 1, RMX>(ts, t, go, tw);
+    cgfft::fft_io<N, TKV, fx_threads(N, TKV, RMX), false, 1, RMX>(ts, t, go, tw);
   }
 }
 
@@ -1269,7 +1281,7 @@ __global__ void __launch_bounds__(T, 2) k_zi_tma(const __grid_constant__ CUtenso
 // ((N/2+1) x 128 B rounded up to whole boxes: 51 KB at 768^3, four CTAs per
 // SM).  ZSW_NB boxes of ZSW_KR rows (a multiple of 8, so every box starts on
 // a 1024-byte boundary of the tile; rows past N/2 are filled with zeros and
-// never read).  The half-complex combination runs in place on the tile, the
+// never read).  The half-complex combination is the first stage's load, the
 // inner stages map consecutive threads to consecutive lines (conflict-free
 // on the swizzled rows) and the last stage to consecutive butterflies of a
 // line (coalesced stores).  Same arithmetic as k_zi; bounded wait, error
@@ -1360,13 +1372,46 @@ struct ZiArgs {
   float* out[3];
 };
 
+// The half-complex combination as the first stage's load: Z_n of line b from
+// rows n and H - n, zsw_halfcomplex's arithmetic (its expression for row H - n
+// is the one for row n with the rows exchanged).  The rows are read twice, but
+// the combined tile is neither written nor read back, and one barrier goes.
+template <int H>
+struct HalfComplexLoad {
+  cgfft::SmemSw16 t;
+  const float2* __restrict__ twN;
+  __device__ __forceinline__ cplx ld(int b, int n) const {
+    const cplx a = t.ld(b, n), c = t.ld(b, H - n);
+    if (n == 0) return cplx{a.x + c.x, a.x - c.x};
+    const float2 w = __ldg(twN + n);
+    const cplx sm = {a.x + c.x, a.y - c.y}, d = {a.x - c.x, a.y + c.y};
+    const cplx r = {d.x * w.x + d.y * w.y, d.y * w.x - d.x * w.y};
+    return cplx{sm.x - r.y, sm.y + r.x};
+  }
+  static constexpr bool kShared = true;
+};
+
+// Threads and CTAs per SM by mesh size.  us for the three components, with the
+// separate combination on 256 threads (4 CTAs per SM, 3 from 768) and this: 96:
+// 8.9, 6.8; 128: 15.1, 10.9; 192: 38, 31; 256: 81, 62; 384: 282, 233; 512: 605,
+// 488; 768: 2227, 1914; 1024: 5651, 4911.
+struct ZiCfg { int thr, minb; };
+__host__ __device__ constexpr ZiCfg zi_cfg(int N) {
+  return N <= 128   ? ZiCfg{64, 12}
+         : N <= 256 ? ZiCfg{128, 8}
+         : N == 384 ? ZiCfg{192, 5}
+         : N == 512 ? ZiCfg{256, 5}
+         : N == 768 ? ZiCfg{256, 3}
+                    : ZiCfg{256, 2};
+}
+
 template <int N>
-__global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_constant__ ZiArgs a,
+__global__ void __launch_bounds__(zi_cfg(N).thr, zi_cfg(N).minb) k_zi_sw(const __grid_constant__ ZiArgs a,
                                              const float2* __restrict__ twH,
                                              const float2* __restrict__ twN,
                                              unsigned* __restrict__ err) {
   static_assert(TY == 16, "the swizzled tile holds 16 lines per 128-byte row");
-  constexpr int H = N / 2;
+  constexpr int H = N / 2, TT = zi_cfg(N).thr;
   constexpr int KR = zsw_krows<N>(), NB = zsw_nbox<N>();
   constexpr unsigned kBytes = 128u * NB * KR;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1386,18 +1431,17 @@ __global__ void __launch_bounds__(T, N >= 768 ? 3 : 4) k_zi_sw(const __grid_cons
   using TP = ZswPack<N>;
   float2* tws = reinterpret_cast<float2*>(base + kBytes + 16);
   if (!zsw_gather<N>(a.tm[blockIdx.z], base, bar, 0, x, y0, [&] {
-        if constexpr (zsw_pack<N>()) TP::template copy<T>(tws, twH);
+        if constexpr (zsw_pack<N>()) TP::template copy<TT>(tws, twH);
       })) {
     if (threadIdx.x == 0) atomicOr(err, (unsigned)CG_ERR_TMA_WAIT);
     return;
   }
-  zsw_halfcomplex<N>(t, twN);
-  __syncthreads();
   const cgfft::GmemC<H, 1> gout{reinterpret_cast<float2*>(a.out[blockIdx.z]) + ((size_t)x * N + y0) * H};
+  const HalfComplexLoad<H> hc{t, twN};
   if constexpr (zsw_pack<N>())
-    cgfft::fft_io<H, TY, T, false, 1, 16, true>(t, t, gout, TP{tws});
+    cgfft::fft_io<H, TY, TT, false, 1, 16, true>(hc, t, gout, TP{tws});
   else
-    cgfft::fft_io<H, TY, T, false, 1, 16, true>(t, t, gout, twH);
+    cgfft::fft_io<H, TY, TT, false, 1, 16, true>(hc, t, gout, twH);
 }
 
 // ------------------------------------------ z c2r fused with interpolation
@@ -1736,6 +1780,7 @@ struct MeshKernels {
   int tk;    // ky columns per CTA of the x pass
   int byg;   // lines per CTA of the Green pass
   int tg;    // threads per CTA of the Green pass
+  int tfz, tfx, tzi;   // of the z r2c, the TMA x passes, the TMA z c2r
 };
 
 template <int N, int V>
@@ -1748,6 +1793,7 @@ void set_fx(MeshKernels* k) {
   k->fxf_sw = k_fx_sw<N, TKV, RMX>;
   k->fxi3_sw = k_fx_inv_sw<N, TKV, RMX>;
   k->sm_fx_sw = fx_sw_smem<N, TKV, RMX>();
+  k->tfx = fx_threads(N, TKV, RMX);
   k->sm_fx = sizeof(cplx) * cgfft::col_tile_elems<N, TKV>();
   k->tk = TKV;
 }
@@ -1767,6 +1813,7 @@ MeshKernels make_kernels(MeshSched s) {
   MeshKernels k;
   k.fz = k_fz<N, false>;
   k.fz_reset = k_fz<N, true>;
+  k.tfz = fz_threads(N);
   k.dfz = k_dfz<N, 4>;
   k.fyf = k_fy<N, -1>;
   k.fyi = k_fy<N, 1>;
@@ -1775,6 +1822,7 @@ MeshKernels make_kernels(MeshSched s) {
   k.zi_tma = k_zi_tma<N>;
   k.sm_zi_tma = zi_tma_smem<N>();
   k.zi_sw = k_zi_sw<N>;
+  k.tzi = zi_cfg(N).thr;
   k.sm_zi_sw = zsw_smem<N>() + (zsw_pack<N>() ? ZswPack<N>::bytes : 0);
   k.zip = k_zi_interp<N>;
   k.sm_fz = sizeof(cplx) * TY * cgfft::line_pitch<N / 2>();
@@ -2120,7 +2168,7 @@ cudaError_t pm_autotune(PmPlan* p, cudaStream_t st, MeshSched* best, float* ms_g
       const bool sw = x_maps_for(p, k.tk);
       prof_mark(st, CG_ST_OTHER);
       if (sw)
-        k.fxi3_sw<<<dim3(N / k.tk, N / 2 + 1, 3), T, k.sm_fx_sw, st>>>(
+        k.fxi3_sw<<<dim3(N / k.tk, N / 2 + 1, 3), k.tfx, k.sm_fx_sw, st>>>(
             p->xtm[0], p->xtm[1], FxInvArgs{0, {p->gsp[0], p->gsp[1], p->gsp[2]}, nullptr},
             p->twN, p->err);
       else
@@ -2248,7 +2296,7 @@ cudaError_t mesh_r2c(const MeshFFT* f, const float* real, float2* spec, cudaStre
   if (!get_kernels(f->N, &k)) return cudaErrorInvalidValue;
   const int N = f->N;
   prof_mark(st, CG_ST_FZ);
-  k.fz<<<dim3(N / TY, N), T, k.sm_fz, st>>>(real, spec, f->twH, f->twN, f->dsum);
+  k.fz<<<dim3(N / TY, N), k.tfz, k.sm_fz, st>>>(real, spec, f->twH, f->twN, f->dsum);
   prof_mark(st, CG_ST_OTHER);
   k.fyf<<<(N / 2 + 1) * N / BY, T, k.sm_fy, st>>>(spec, f->twN);
   prof_mark(st, CG_ST_FX_FWD);
@@ -2375,7 +2423,7 @@ void launch_fx_fwd(PmPlan* p, const MeshKernels& k, cudaStream_t st) {
   const int N = p->N;
   prof_mark(st, CG_ST_FX_FWD);
   if (x_maps_for(p, k.tk))
-    k.fxf_sw<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx_sw, st>>>(p->xtm[0], p->spec, p->twN,
+    k.fxf_sw<<<dim3(N / k.tk, N / 2 + 1), k.tfx, k.sm_fx_sw, st>>>(p->xtm[0], p->spec, p->twN,
                                                                p->err);
   else
     k.fxf<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->spec, p->spec, p->twN, nullptr);
@@ -2388,9 +2436,9 @@ cudaError_t pm_r2c(PmPlan* p, cudaStream_t st) {
   cudaMemsetAsync(p->dsum, 0, sizeof(double), st);
   prof_mark(st, CG_ST_FZ);
   if (p->keep_dens)
-    k.fz<<<dim3(N / TY, N), T, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
+    k.fz<<<dim3(N / TY, N), k.tfz, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
   else
-    k.fz_reset<<<dim3(N / TY, N), T, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
+    k.fz_reset<<<dim3(N / TY, N), k.tfz, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
   p->dens_reset = !p->keep_dens;
   launch_fx_fwd(p, k, st);
   return cudaGetLastError();
@@ -2490,7 +2538,7 @@ void launch_zi(const PmPlan* p, const MeshKernels& k, int a, int n, cudaStream_t
       z.out[i] = p->fmesh[c];
     }
     prof_mark(st, CG_ST_ZI);
-    k.zi_sw<<<dim3(N / TY, N, n), T, k.sm_zi_sw, st>>>(z, p->twH, p->twN, p->err);
+    k.zi_sw<<<dim3(N / TY, N, n), k.tzi, k.sm_zi_sw, st>>>(z, p->twH, p->twN, p->err);
     return;
   }
   for (int c = a; c < a + n; c++) {
@@ -2601,7 +2649,7 @@ static cudaError_t green_x_zi(PmPlan* p, cudaStream_t st, bool zi) {
   for (int c = 0; c < 3; c += nc) {
     if (xsw) {
       prof_mark(st, CG_ST_FX_INV);
-      k.fxi3_sw<<<dim3(gx.x, gx.y, nc), T, k.sm_fx_sw, st>>>(
+      k.fxi3_sw<<<dim3(gx.x, gx.y, nc), k.tfx, k.sm_fx_sw, st>>>(
           p->xtm[0], p->xtm[1], FxInvArgs{c, {p->gsp[0], p->gsp[1], p->gsp[2]}, p->ktab}, p->twN,
           p->err);
     } else {
@@ -2689,7 +2737,7 @@ cudaError_t pm_slab_density(PmPlan* p, int x0, int nx, const float* const x[3], 
   }
   cudaMemsetAsync(p->dsum, 0, sizeof(double), st);
   prof_mark(st, CG_ST_FZ);
-  k.fz<<<dim3(N / TY, nx), T, k.sm_fz, st>>>(p->dens + x0 * plane, p->spec + (size_t)x0 * N,
+  k.fz<<<dim3(N / TY, nx), k.tfz, k.sm_fz, st>>>(p->dens + x0 * plane, p->spec + (size_t)x0 * N,
                                              p->twH, p->twN, p->dsum);
   p->dens_reset = false;
   p->dens_stale = true;       // only this slab's planes hold the density
@@ -2834,7 +2882,7 @@ cudaError_t pm_power_spectrum(PmPlan* p, const float* const x[3], long long n, i
   if (e != cudaSuccess) return e;
   cudaMemsetAsync(p->dsum, 0, sizeof(double), st);
   prof_mark(st, CG_ST_FZ);
-  k.fz<<<dim3(N / TY, N), T, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
+  k.fz<<<dim3(N / TY, N), k.tfz, k.sm_fz, st>>>(p->dens, p->spec, p->twH, p->twN, p->dsum);
   launch_fx_fwd(p, k, st);
   cudaMemsetAsync(acc, 0, sizeof(double) * 3 * nbins, st);
   const size_t sm = k.sm_fy + sizeof(double) * 3 * nbins;

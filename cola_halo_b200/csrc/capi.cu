@@ -696,11 +696,13 @@ extern "C" int cg_net_num_params(void) { return CNET_PARAMS; }
 // (already scaled), out3 = [v][3] raw network output, grad3 = dL/dout.
 static int net_load_input(cg_net* h, const float* in2) {
   const size_t nv = (size_t)h->n.N * h->n.N * h->n.N;
-  std::vector<__nv_bfloat16> b(nv * CNET_C, __float2bfloat16_rn(0.0f));
+  std::vector<__nv_bfloat16> b(nv * CNET_C, __float2bfloat16_rn(0.0f)), p(nv * 2);
   for (size_t v = 0; v < nv; v++) {
-    b[v * CNET_C] = __float2bfloat16_rn(in2[2 * v]);
-    b[v * CNET_C + 1] = __float2bfloat16_rn(in2[2 * v + 1]);
+    for (int c = 0; c < 2; c++)
+      p[2 * v + c] = b[v * CNET_C + c] = __float2bfloat16_rn(in2[2 * v + c]);
   }
+  CG_CHECK(cudaMemcpyAsync(h->n.feat, p.data(), p.size() * sizeof(__nv_bfloat16),
+                           cudaMemcpyHostToDevice, h->st), "upload input");
   CG_CHECK(cudaMemcpyAsync(h->n.act[0], b.data(), b.size() * sizeof(__nv_bfloat16),
                            cudaMemcpyHostToDevice, h->st), "upload input");
   CG_CHECK(cudaStreamSynchronize(h->st), "sync");
@@ -760,7 +762,7 @@ extern "C" int cg_net_train_step(cg_net* h, cg_sim* coarse, cg_sim* fine, float 
   const float* x[3] = {coarse->ps.x[0], coarse->ps.x[1], coarse->ps.x[2]};
   const float* ff[3] = {fine->ps.f[0], fine->ps.f[1], fine->ps.f[2]};
   const float* fc[3] = {coarse->ps.f[0], coarse->ps.f[1], coarse->ps.f[2]};
-  CG_CHECK(cnet_features(&h->n, coarse->pm.dens, st), "features");
+  CG_CHECK(cnet_features(&h->n, coarse->pm.dens, true, st), "features");
   CG_CHECK(cnet_target(&h->n, x, coarse->ps.n, coarse->L, ff, fc, st), "target");
   CG_CHECK(cnet_forward(&h->n, st, false), "forward");
   CG_CHECK(cnet_loss_grad(&h->n, 1.0 / (double)coarse->ps.n, st), "loss");
@@ -781,7 +783,7 @@ extern "C" int cg_net_forces(cg_net* h, cg_sim* coarse) {
   if (rc) return rc;
   cudaStream_t st = coarse->st;   // stay on the realization's stream
   const float* x[3] = {coarse->ps.x[0], coarse->ps.x[1], coarse->ps.x[2]};
-  CG_CHECK(cnet_features(&h->n, coarse->pm.dens, st), "features");
+  CG_CHECK(cnet_features(&h->n, coarse->pm.dens, false, st), "features");
   CG_CHECK(cnet_forward(&h->n, st, false), "forward");
   CG_CHECK(cnet_apply(&h->n, x, coarse->ps.n, coarse->L, coarse->ps.f, st), "apply");
   return CG_OK;

@@ -218,18 +218,19 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ gr, floa
   }
 }
 
-// Features: channel 0 = delta, channel 1 = phi (both on the coarse mesh).
+// Features: channel 0 = delta, channel 1 = phi (both on the coarse mesh), as
+// pairs and, with wide, in the 16-channel layout.
 __global__ void k_features(const float* __restrict__ delta, const float* __restrict__ phi,
-                           size_t nv, float sd, float sp, __nv_bfloat16* __restrict__ f) {
+                           size_t nv, float sd, float sp, __nv_bfloat162* __restrict__ f,
+                           __nv_bfloat16* __restrict__ wide) {
   for (size_t v = (size_t)blockIdx.x * T + threadIdx.x; v < nv; v += (size_t)gridDim.x * T) {
-    __nv_bfloat16 h[C];
-#pragma unroll
-    for (int c = 0; c < C; c++) h[c] = __float2bfloat16_rn(0.0f);
-    h[0] = __float2bfloat16_rn(delta[v] * sd);
-    h[1] = __float2bfloat16_rn(phi[v] * sp);
-    uint4* d = reinterpret_cast<uint4*>(f + v * C);
-    d[0] = *reinterpret_cast<const uint4*>(&h[0]);
-    d[1] = *reinterpret_cast<const uint4*>(&h[8]);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(delta[v] * sd, phi[v] * sp);
+    f[v] = h;
+    if (wide) {
+      uint4* d = reinterpret_cast<uint4*>(wide + v * C);
+      d[0] = make_uint4(*reinterpret_cast<const unsigned*>(&h), 0, 0, 0);
+      d[1] = make_uint4(0, 0, 0, 0);
+    }
   }
 }
 
@@ -328,6 +329,7 @@ cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed) {
   CN_TRY(cudaMalloc(&n->trainable, sizeof(int) * P));
   CN_TRY(cudaMalloc(&n->wb, sizeof(__nv_bfloat16) * 3 * WSZ));
   for (int l = 0; l < 3; l++) CN_TRY(cudaMalloc(&n->act[l], sizeof(__nv_bfloat16) * nv * C));
+  CN_TRY(cudaMalloc(&n->feat, sizeof(__nv_bfloat162) * nv));
   CN_TRY(cudaMalloc(&n->out, sizeof(float) * nv * C));
   CN_TRY(cudaMalloc(&n->out4, sizeof(float4) * nv));
   CN_TRY(cudaMalloc(&n->g0, sizeof(float) * nv * C));
@@ -378,7 +380,7 @@ void cnet_free(CNet* n) {
   cudaFree(n->params); cudaFree(n->grads); cudaFree(n->m1); cudaFree(n->m2);
   cudaFree(n->trainable); cudaFree(n->wb);
   for (int l = 0; l < 3; l++) cudaFree(n->act[l]);
-  cudaFree(n->out); cudaFree(n->out4); cudaFree(n->g0); cudaFree(n->g1); cudaFree(n->gb);
+  cudaFree(n->feat); cudaFree(n->out); cudaFree(n->out4); cudaFree(n->g0); cudaFree(n->g1); cudaFree(n->gb);
   cudaFree(n->resid); cudaFree(n->loss); cudaFree(n->phi);
   cudaFree(n->spec);
   mesh_fft_free(&n->fft);
@@ -415,10 +417,16 @@ static cudaError_t conv(const CNet* n, const __nv_bfloat16* in, const __nv_bfloa
   return cudaGetLastError();
 }
 
+bool cnet_narrow_input(const CNet* n) { return n->use_tc && n->N % 128 == 0; }
+
 cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full) {
   cudaError_t e;
   const float* P = n->params;
-  if ((e = conv(n, n->act[0], n->wb, P + WSZ, 1, nullptr, n->act[1], false, st))) return e;
+  if (cnet_narrow_input(n))
+    e = conv_tc_features(n->feat, n->N, n->wb, P + WSZ, 1, n->act[1], st);
+  else
+    e = conv(n, n->act[0], n->wb, P + WSZ, 1, nullptr, n->act[1], false, st);
+  if (e) return e;
   if ((e = conv(n, n->act[1], n->wb + WSZ, P + (WSZ + C) + WSZ, 1, nullptr, n->act[2], false, st)))
     return e;
   return conv(n, n->act[2], n->wb + 2 * WSZ, P + 2 * (WSZ + C) + WSZ, 0, full ? n->out : nullptr,
@@ -491,7 +499,7 @@ cudaError_t cnet_adam(CNet* n, float lr, cudaStream_t st) {
 }
 
 // Input features from a coarse PM plan whose density mesh holds delta.
-cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st) {
+cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
   cudaError_t e = mesh_r2c(&n->fft, delta, n->spec, st);
@@ -500,8 +508,9 @@ cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st) {
   k_potential<<<grid_for((long long)(N / 2 + 1) * N * N), T, 0, st>>>(n->spec, N);
   if ((e = mesh_c2r(&n->fft, n->spec, n->phi, st)) != cudaSuccess) return e;
   prof_mark(st, CG_ST_OTHER);
-  k_features<<<grid_for((long long)nv), T, 0, st>>>(delta, n->phi, nv, n->in_scale[0],
-                                                    n->in_scale[1], n->act[0]);
+  k_features<<<grid_for((long long)nv), T, 0, st>>>(
+      delta, n->phi, nv, n->in_scale[0], n->in_scale[1], n->feat,
+      wide || !cnet_narrow_input(n) ? n->act[0] : nullptr);
   return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@ struct CNet {
   int* trainable;              // 1 for live weights (masked channels stay 0)
   __nv_bfloat16* wb;           // bf16 weights used by the kernels, 3 x 27*16*16
   __nv_bfloat16* act[3];       // layer inputs: features, hidden 1, hidden 2 [v][16]
+  __nv_bfloat162* feat;        // the features' two live channels [v] (tensor-core first layer)
   float* out;                  // network output [v][16] (channels 0-2 used)
   float4* out4;                // its channels 0-3 packed [v]: what the interpolation reads
   float* g0;                   // gradient buffers [v][16]
@@ -39,7 +40,11 @@ struct CNet {
 cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed);
 void cnet_free(CNet* n);
 cudaError_t cnet_sync_bf16(CNet* n, cudaStream_t st);
-cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st);
+// features of delta into feat; wide: into act[0] as well (the weight gradient
+// reads it, and the CUDA-core first layer, which then always gets it)
+cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st);
+// the first layer reads feat instead of act[0]
+bool cnet_narrow_input(const CNet* n);
 // full: also write the [v][16] output that the loss and the host API read
 // (the packed out4 is always written)
 cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true);
@@ -59,6 +64,9 @@ cudaError_t cnet_apply(const CNet* n, const float* const x[3], long long np, flo
 cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
                             const float* bias, int act, float* out_f, __nv_bfloat16* out_b,
                             float4* out4, cudaStream_t st);
+// The first layer from the features' two live channels, into out_b.
+cudaError_t conv_tc_features(const __nv_bfloat162* in, int N, const __nv_bfloat16* w,
+                             const float* bias, int act, __nv_bfloat16* out_b, cudaStream_t st);
 // gate (or NULL): the layer below's output, whose leaky-ReLU backward scales
 // the result; out_b (or NULL): a bf16 copy
 cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bfloat16* w,

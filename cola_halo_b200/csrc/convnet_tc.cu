@@ -495,6 +495,140 @@ cudaError_t launch_sweep(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
   return cudaGetLastError();
 }
 
+// The first layer, whose input has two live channels (density, potential):
+// the 27 taps' pairs of one voxel are gathered into one row of 54 + 10 zeros, so
+// a tile of 128 voxels is 4 MMAs of K = 16 on a 128 x 64 operand where the
+// 16-channel layout needs 27 (9 in the sweep) of mostly zeros; and the features
+// take 4 bytes a voxel instead of 32.  Thread r copies voxel r's 27 words from
+// the nine input lines in shared memory (consecutive lanes, consecutive words)
+// into seven 16-byte groups of four taps, K-major: group g of row r sits at g *
+// 2048 + r * 16.  The next tile's lines arrive by cp.async meanwhile.
+constexpr int IN_LINE = (TILE_M + 8) * 4;        // z0 - 4 .. z0 + 131, 4 bytes a voxel
+constexpr int IN_LINES = 9 * IN_LINE;
+constexpr int IN_A = 8 * TILE_M * 16;            // 64 K values
+constexpr int IN_B = 8 * C * 16;
+constexpr int IN_CPS = 6;
+constexpr int in_smem_bytes() { return 2 * IN_LINES + IN_A + IN_B + 64; }
+
+__device__ __forceinline__ void gather_in(const __nv_bfloat162* __restrict__ in, int N, int tile,
+                                          uint8_t* dst) {
+  const int per_line = N / TILE_M;
+  const int line = tile / per_line, z0 = tile % per_line * TILE_M;
+  const int x = line / N, y = line % N;
+  for (int i = threadIdx.x; i < 9 * (IN_LINE / 16); i += THREADS) {
+    const int L = i / (IN_LINE / 16), q = i % (IN_LINE / 16);
+    int xx = x + L / 3 - 1, yy = y + L % 3 - 1, zz = z0 - 4 + 4 * q;
+    xx = xx < 0 ? xx + N : (xx >= N ? xx - N : xx);
+    yy = yy < 0 ? yy + N : (yy >= N ? yy - N : yy);
+    zz = zz < 0 ? zz + N : (zz >= N ? zz - N : zz);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                 :: "r"(smem_u32(dst + L * IN_LINE + q * 16)),
+                    "l"(in + ((size_t)xx * N + yy) * N + zz) : "memory");
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, IN_CPS)
+    k_conv_in(const __nv_bfloat162* __restrict__ in, int N, const __nv_bfloat16* __restrict__ w,
+              const float* __restrict__ bias, int act, __nv_bfloat16* __restrict__ out_b) {
+  extern __shared__ __align__(1024) uint8_t sm[];
+  uint8_t* const sA = sm;
+  uint8_t* const sB = sA + IN_A;
+  uint8_t* const lines = sB + IN_B;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(lines + 2 * IN_LINES);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
+  const int tid = threadIdx.x, warp = tid >> 5;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(tslot)), "r"(32) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(mbar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // B: element (n = output channel, k = 2 tap + input channel); zeros past tap 26
+  for (int i = tid; i < 64 * C; i += THREADS) {
+    const int n = i / 64, k = i % 64;
+    const __nv_bfloat16 v =
+        k < 54 ? w[(k / 2 * C + k % 2) * C + n] : __float2bfloat16_rn(0.0f);
+    *reinterpret_cast<__nv_bfloat16*>(sB + (k / 8) * (C * 16) + n * 16 + (k % 8) * 2) = v;
+  }
+  *reinterpret_cast<uint4*>(sA + 7 * TILE_M * 16 + tid * 16) = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tslot;
+  const uint32_t bar = smem_u32(mbar);
+  const int ntiles = N * N * (N / TILE_M);
+  uint32_t phase = 0;
+  bool ok = true;
+  int tile = blockIdx.x;
+  if (tile < ntiles) gather_in(in, N, tile, lines);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int it = 0; tile < ntiles && ok; tile += gridDim.x, it++) {
+    const int next = tile + gridDim.x;
+    // the other line buffer was read before the last tile's MMAs
+    if (next < ntiles) gather_in(in, N, next, lines + ((it + 1) & 1) * IN_LINES);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(lines + (it & 1) * IN_LINES) + tid + 3;
+#pragma unroll
+    for (int g = 0; g < 7; g++) {
+      uint32_t q[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int t = 4 * g + j;
+        q[j] = t < 27 ? src[(t / 3) * (IN_LINE / 4) + t % 3] : 0u;
+      }
+      *reinterpret_cast<uint4*>(sA + g * (TILE_M * 16) + tid * 16) =
+          make_uint4(q[0], q[1], q[2], q[3]);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0) {
+      for (int k = 0; k < 4; k++) {
+        const uint64_t da = umma_desc(smem_u32(sA) + (uint32_t)(2 * k * TILE_M * 16),
+                                      TILE_M * 16, 128);
+        const uint64_t db = umma_desc(smem_u32(sB) + (uint32_t)(2 * k * C * 16), C * 16, 128);
+        const uint32_t acc = k > 0 ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+            :: "r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(acc)
+            : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                   :: "r"(bar) : "memory");
+    }
+    const bool got = mbar_wait(bar, phase);
+    ok = __syncthreads_and(got ? 1 : 0) != 0;
+    if (!ok && tid == 0) atomicOr(&g_tc_err, 1u);
+    phase ^= 1u;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok) {
+      const int per_line = N / TILE_M;
+      uint32_t r[16];
+      tmem_ld16(r, tmem + ((uint32_t)(warp * 32) << 16));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      store_voxel(r, (size_t)(tile / per_line) * N + tile % per_line * TILE_M + tid, bias, act,
+                  nullptr, nullptr, out_b, nullptr);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  // copies still in flight (a prefetch after a timeout) finish before exit
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(32)
+                 : "memory");
+}
+
 template <bool FLIP, int STAGES, int CPS>
 cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const float* bias,
                      int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
@@ -546,6 +680,19 @@ cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16*
                             const float* bias, int act, float* out_f, __nv_bfloat16* out_b,
                             float4* out4, cudaStream_t st) {
   return launch<false>(in, N, w, bias, act, nullptr, out_f, out_b, out4, st);
+}
+
+cudaError_t conv_tc_features(const __nv_bfloat162* in, int N, const __nv_bfloat16* w,
+                             const float* bias, int act, __nv_bfloat16* out_b, cudaStream_t st) {
+  if (N < TILE_M || N % TILE_M) return cudaErrorNotSupported;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_conv_in, cudaFuncAttributeMaxDynamicSharedMemorySize, in_smem_bytes());
+  if (attr != cudaSuccess) return attr;
+  const int ntiles = N * N * (N / TILE_M), cap = IN_CPS * cg_sm_count();
+  prof_mark(st, CG_ST_OTHER);
+  k_conv_in<<<ntiles < cap ? ntiles : cap, THREADS, in_smem_bytes(), st>>>(in, N, w, bias, act,
+                                                                          out_b);
+  return cudaGetLastError();
 }
 
 cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bfloat16* w,

@@ -215,3 +215,23 @@ def test_conv_sweep_two_tiles_per_line(gpu_lib):
         gpu_lib.cg_net_set_conv_variant(-1)
         net.close()
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n,taps", [(128, (0, 13, 26)), (128, (2, 9, 20)), (256, (6, 17, 24))])
+def test_first_layer_from_packed_features(gpu_lib, n, taps):
+    """The first layer reads the two live input channels as pairs: weights that
+    pick one tap and channel each (tile and line ends, all three periodic faces)
+    give the shifted inputs back exactly, the other layers passing them on."""
+    net, p = _net(n)
+    p = np.zeros_like(p)
+    w = p.reshape(3, CR.LAYER)[:, :CR.WSZ].reshape(3, 27, 16, 16)
+    for c, t in enumerate(taps):
+        w[0, t, c % 2, c] = w[1, 13, c, c] = w[2, 13, c, c] = 1.0
+    net.set_params(p)
+    net.tensor_cores(True)
+    # whole numbers below 256 are bf16 values; no channel is ever negative
+    x = np.random.default_rng(n).integers(0, 256, (n, n, n, 2)).astype(np.float32)
+    got = net.forward_host(x)
+    for c, t in enumerate(taps):
+        want = np.roll(x[..., c % 2], (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2))
+        np.testing.assert_array_equal(got[..., c], want)

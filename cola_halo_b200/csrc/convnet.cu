@@ -459,7 +459,9 @@ cudaError_t cnet_backward(CNet* n, cudaStream_t st, bool gb_ready) {
   for (int l = 2; l >= 0; l--) {
     float* dw = n->grads + l * (WSZ + C);
     cudaError_t ew = cudaErrorNotSupported;
-    if (n->use_tc) ew = conv_wgrad_tc(n->act[l], g, N, dw, dw + WSZ, st);
+    if (n->use_tc)
+      ew = l == 0 ? conv_wgrad_in(n->feat, g, N, dw, dw + WSZ, st)
+                  : conv_wgrad_tc(n->act[l], g, N, l == 2, dw, dw + WSZ, st);
     if (ew == cudaErrorNotSupported) {
       prof_mark(st, CG_ST_OTHER);
       k_conv_wgrad<<<cg_sm_count() * 2, T, wgrad_smem, st>>>(n->act[l], g, N, dw, dw + WSZ);
@@ -499,7 +501,7 @@ cudaError_t cnet_adam(CNet* n, float lr, cudaStream_t st) {
 }
 
 // Input features from a coarse PM plan whose density mesh holds delta.
-cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st) {
+cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
   cudaError_t e = mesh_r2c(&n->fft, delta, n->spec, st);
@@ -510,7 +512,7 @@ cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t s
   prof_mark(st, CG_ST_OTHER);
   k_features<<<grid_for((long long)nv), T, 0, st>>>(
       delta, n->phi, nv, n->in_scale[0], n->in_scale[1], n->feat,
-      wide || !cnet_narrow_input(n) ? n->act[0] : nullptr);
+      cnet_narrow_input(n) ? nullptr : n->act[0]);
   return cudaGetLastError();
 }
 

@@ -40,9 +40,8 @@ struct CNet {
 cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed);
 void cnet_free(CNet* n);
 cudaError_t cnet_sync_bf16(CNet* n, cudaStream_t st);
-// features of delta into feat; wide: into act[0] as well (the weight gradient
-// reads it, and the CUDA-core first layer, which then always gets it)
-cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st);
+// features of delta into feat, and into act[0] where the first layer reads that
+cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st);
 // the first layer reads feat instead of act[0]
 bool cnet_narrow_input(const CNet* n);
 // full: also write the [v][16] output that the loss and the host API read
@@ -73,8 +72,12 @@ cudaError_t conv_tc_backward_data(const __nv_bfloat16* g, int N, const __nv_bflo
                                   const __nv_bfloat16* gate, float* out_f, __nv_bfloat16* out_b,
                                   cudaStream_t st);
 // Weight gradient on tensor cores (convnet_wgrad.cu), added to dw [27][16][16]
-// and db [16]; cudaErrorNotSupported when N is no multiple of 16.
-cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, float* dw, float* db,
+// and db [16]; cudaErrorNotSupported when N is no multiple of 16.  last: only
+// the first eight channels of g are not zero.
+cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, bool last, float* dw,
+                          float* db, cudaStream_t st);
+// The same for the first layer, from the features' two live channels.
+cudaError_t conv_wgrad_in(const __nv_bfloat162* in, const float* g, int N, float* dw, float* db,
                           cudaStream_t st);
 // Device error word of the tensor-core kernels (bounded waits that gave up).
 unsigned conv_tc_error_word();

@@ -235,3 +235,30 @@ def test_first_layer_from_packed_features(gpu_lib, n, taps):
     for c, t in enumerate(taps):
         want = np.roll(x[..., c % 2], (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2))
         np.testing.assert_array_equal(got[..., c], want)
+
+
+@pytest.mark.parametrize("n", [16, 48, 128, 144])
+def test_weight_gradients_of_every_layer_exact(gpu_lib, n):
+    """All three layers' weight gradients where every partial sum is a whole
+    number below 2^24, so that float32 sums are exact in any order: the layers
+    pass small positive inputs through, and the output gradient is -1, 0 or 1."""
+    net, p = _net(n)
+    p = np.zeros_like(p)
+    w = p.reshape(3, CR.LAYER)[:, :CR.WSZ].reshape(3, 27, 16, 16)
+    for c in range(3):
+        w[0, 13, c % 2, c] = w[1, 13, c, c] = w[2, 13, c, c] = 1.0
+    net.set_params(p)
+    net.tensor_cores(True)
+    rng = np.random.default_rng(n)
+    x = rng.integers(1, 4, (n, n, n, 2)).astype(np.float32)
+    g = rng.integers(-1, 2, (n, n, n, 3)).astype(np.float32)
+    got = net.backward_host(x, g).reshape(3, CR.LAYER)
+    gm = g.reshape(-1, 3).astype(np.float64)
+    for layer in range(3):
+        chans = (0, 1) if layer == 0 else (0, 1, 0)
+        want = np.zeros((27, 16, 16))
+        for t in range(27):
+            a = np.roll(x, (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2))
+            want[t, :len(chans), :3] = a.reshape(-1, 2)[:, list(chans)].T.astype(np.float64) @ gm
+        np.testing.assert_array_equal(got[layer][:CR.WSZ].reshape(27, 16, 16), want, str(layer))
+        np.testing.assert_array_equal(got[layer][CR.WSZ:CR.WSZ + 3], gm.sum(axis=0))

@@ -419,10 +419,10 @@ static cudaError_t conv(const CNet* n, const __nv_bfloat16* in, const __nv_bfloa
 
 bool cnet_narrow_input(const CNet* n) { return n->use_tc && n->N % 128 == 0; }
 
-cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full) {
+cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full, bool wide) {
   cudaError_t e;
   const float* P = n->params;
-  if (cnet_narrow_input(n))
+  if (!wide && cnet_narrow_input(n))
     e = conv_tc_features(n->feat, n->N, n->wb, P + WSZ, 1, n->act[1], st);
   else
     e = conv(n, n->act[0], n->wb, P + WSZ, 1, nullptr, n->act[1], false, st);
@@ -501,7 +501,7 @@ cudaError_t cnet_adam(CNet* n, float lr, cudaStream_t st) {
 }
 
 // Input features from a coarse PM plan whose density mesh holds delta.
-cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st) {
+cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
   cudaError_t e = mesh_r2c(&n->fft, delta, n->spec, st);
@@ -512,7 +512,7 @@ cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st) {
   prof_mark(st, CG_ST_OTHER);
   k_features<<<grid_for((long long)nv), T, 0, st>>>(
       delta, n->phi, nv, n->in_scale[0], n->in_scale[1], n->feat,
-      cnet_narrow_input(n) ? nullptr : n->act[0]);
+      wide || !cnet_narrow_input(n) ? n->act[0] : nullptr);
   return cudaGetLastError();
 }
 

@@ -40,13 +40,17 @@ struct CNet {
 cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed);
 void cnet_free(CNet* n);
 cudaError_t cnet_sync_bf16(CNet* n, cudaStream_t st);
-// features of delta into feat, and into act[0] where the first layer reads that
-cudaError_t cnet_features(CNet* n, const float* delta, cudaStream_t st);
-// the first layer reads feat instead of act[0]
+// features of delta into feat, and into act[0] if wide or where the first layer
+// reads nothing else
+cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t st);
+// the first layer can read feat instead of act[0]
 bool cnet_narrow_input(const CNet* n);
 // full: also write the [v][16] output that the loss and the host API read
-// (the packed out4 is always written)
-cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true);
+// (the packed out4 is always written).  wide: the first layer from act[0], whose
+// sums run in the order of the other pipeline variants.  A training step takes it
+// (36 us more at 128^3): a few voxels decide its loss, where one bf16 rounding of a
+// hidden value shows at 1e-5, so that a step stays the same on every variant.
+cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true, bool wide = false);
 // loss and dL/dout (g0 and its bf16 copy gb) from out4 and the residual sums
 cudaError_t cnet_loss_grad(CNet* n, double inv_msum, cudaStream_t st);
 // gb_ready: gb holds g0 in bf16 already

@@ -12,7 +12,7 @@
 // buffer started dz rows further on: the z shift costs no copy.  B_t are the
 // tap weights in the no-swizzle core-matrix layout (LBO 128 B, SBO 256 B).
 //
-// k_conv_sweep, the default, reuses the lines along y (below).  In k_conv_tc
+// k_conv_sweep, the default, reuses the lines along x (below).  In k_conv_tc
 // CTAs are persistent over tiles, 4 per SM with one line buffer each: one
 // thread issues the tile's 27 MMAs (M=128, N=16, K=16), tcgen05.commit
 // arrives on an mbarrier, the cp.async gather of the next tile starts, and
@@ -166,14 +166,12 @@ __global__ void __launch_bounds__(THREADS, CPS)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0) {
-      for (int k = 0; k < 27; k++) {
-        // tap (dx, dy, dz), in the order dy, dx, dz (k_conv_sweep's): line t / 3,
-        // started dz = t % 3 rows on
-        const int t = (k / 3 % 3) * 9 + (k / 9) * 3 + k % 3;
+      for (int t = 0; t < 27; t++) {
+        // tap (dx, dy, dz): line t / 3, started dz = t % 3 rows on
         const uint64_t da =
             umma_desc(smem_u32(s + (t / 3) * LINE_BYTES + (t % 3) * 16), HALF_BYTES, 128);
         const uint64_t db = umma_desc(smem_u32(sB + t * B_BYTES), 128, 256);
-        const uint32_t acc = k > 0 ? 1u : 0u;
+        const uint32_t acc = t > 0 ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
@@ -247,21 +245,21 @@ __global__ void __launch_bounds__(THREADS, CPS)
                  : "memory");
 }
 
-// The same convolution, sweeping along y with every input row used once.  A
-// CTA owns the z tiles (x0, y, z0) and (x0 + 1, y, z0) for a run of y.  Input
-// row y' (the four lines x0-1 .. x0+2) adds to the outputs of rows y'-1, y'
-// and y'+1 at once: one MMA of M = 128 voxels, N = 48 columns (the three
-// rows' 16 output channels, with the weights of dy = +1, 0, -1) and K = 16
-// per output line, dx and dz.  The A operand (128 rows of 32 bytes from shared
+// The same convolution, sweeping along x with every input row used once.  A
+// CTA owns the z tiles (x, y0, z0) and (x, y0 + 1, z0) for a run of x.  Input
+// row x' (the four lines y0-1 .. y0+2) adds to the outputs of rows x'-1, x'
+// and x'+1 at once: one MMA of M = 128 voxels, N = 48 columns (the three
+// rows' 16 output channels, with the weights of dx = +1, 0, -1) and K = 16
+// per output line, dy and dz.  The A operand (128 rows of 32 bytes from shared
 // memory) is what an MMA of N <= 64 waits for, so this does 9 reads of it per
 // output line where one tile at a time (N = 16) needs 27; and the lines come
 // from L2 twice per output line instead of three (k_conv_ring before this) or
 // nine times.
 //
-// The three accumulators of an output column x sit in tensor-memory slots o
-// mod 3 (o the output row counted from the run's start).  The rows y'-1, y',
-// y'+1 take every slot once, in a cyclic order that moves by one per row, so
-// the B operand of a tap pair (dx, dz) is stored as five blocks of 16 channels, dy
+// The three accumulators of an output column y sit in tensor-memory slots o
+// mod 3 (o the output row counted from the run's start).  The rows x'-1, x',
+// x'+1 take every slot once, in a cyclic order that moves by one per row, so
+// the B operand of a tap pair (dy, dz) is stored as five blocks of 16 channels, dx
 // = +1, 0, -1, +1, 0, and the row's window of three starts at block 2, 1 or 0.
 // After a row's MMAs the slot of output o = i - 2 (i the row) is complete: its
 // threads read it, set it to zero for output o + 3 and hand the tensor memory
@@ -269,10 +267,10 @@ __global__ void __launch_bounds__(THREADS, CPS)
 // next row's lines arrive by cp.async meanwhile.  4 CTAs per SM (57 KB, 128
 // tensor-memory columns each).
 //
-// Per output the products are added in the order dy, dx, dz, as in k_conv_tc:
-// bit-identical.
+// Per output the products are added in the order dx, dy, dz, as in k_conv_tc:
+// bit-identical.  (A sweep along y is as fast but adds in another order.)
 constexpr int SROW_BYTES = 4 * LINE_BYTES;       // four lines of one input row
-constexpr int SB_BYTES = 5 * B_BYTES;            // five 16-channel blocks per (dx, dz)
+constexpr int SB_BYTES = 5 * B_BYTES;            // five 16-channel blocks per (dy, dz)
 constexpr int SLOTS = 3;
 __host__ __device__ constexpr int sweep_smem_bytes() {
   return 2 * SROW_BYTES + 9 * SB_BYTES + 64;
@@ -280,17 +278,17 @@ __host__ __device__ constexpr int sweep_smem_bytes() {
 constexpr int SWEEP_CPS = 4;
 constexpr uint32_t kIdesc48 = (kIdesc & ~(0x3Fu << 17)) | ((48u >> 3) << 17);
 
-// cp.async of row y (periodic) of the lines x0-1 .. x0+2, voxels z0 - 1 ..
+// cp.async of row x (periodic) of the lines y0-1 .. y0+2, voxels z0 - 1 ..
 // z0 + 128, into a row buffer.
-__device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in, int N, int x0,
-                                           int y, int z0, uint8_t* row) {
-  y = y < 0 ? y + N : (y >= N ? y - N : y);
+__device__ __forceinline__ void gather_row(const __nv_bfloat16* __restrict__ in, int N, int y0,
+                                           int x, int z0, uint8_t* row) {
+  x = x < 0 ? x + N : (x >= N ? x - N : x);
   for (int i = threadIdx.x; i < 4 * ROWS * 2; i += THREADS) {
     const int h = i & 1, j = (i >> 1) % ROWS, L = (i >> 1) / ROWS;
-    int xx = x0 + L - 1, zz = z0 + j - 1;
-    xx = xx < 0 ? xx + N : (xx >= N ? xx - N : xx);
+    int yy = y0 + L - 1, zz = z0 + j - 1;
+    yy = yy < 0 ? yy + N : (yy >= N ? yy - N : yy);
     zz = zz < 0 ? zz + N : (zz >= N ? zz - N : zz);
-    const __nv_bfloat16* src = in + (((size_t)xx * N + y) * N + zz) * C + h * 8;
+    const __nv_bfloat16* src = in + (((size_t)x * N + yy) * N + zz) * C + h * 8;
     const uint32_t dst = smem_u32(row + L * LINE_BYTES + h * HALF_BYTES + j * 16);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
   }
@@ -374,11 +372,11 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(mbar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // B of (dx, dz): blocks dy = +1, 0, -1, +1, 0; element (n = output channel,
+  // B of (dy, dz): blocks dx = +1, 0, -1, +1, 0; element (n = output channel,
   // k = input channel) of tap t
   for (int i = tid; i < 9 * 5 * C * C; i += THREADS) {
     const int k = i % C, n = i / C % C, b = i / (C * C) % 5, p = i / (5 * C * C);
-    const int t = (p / 3) * 9 + (2 - b % 3) * 3 + p % 3;
+    const int t = (2 - b % 3) * 9 + p;
     const __nv_bfloat16 v = FLIP ? w[((26 - t) * C + n) * C + k] : w[(t * C + k) * C + n];
     *reinterpret_cast<__nv_bfloat16*>(sB + p * SB_BYTES + cm_off(b * C + n, k)) = v;
   }
@@ -389,7 +387,7 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
   const uint32_t tmem = *tslot;
   const uint32_t mine = tmem + ((uint32_t)(warp * 32) << 16);
   const uint32_t bar = smem_u32(mbar);
-  // output rows in the order (x pair, z tile, y); a CTA takes a contiguous range
+  // output rows in the order (y pair, z tile, x); a CTA takes a contiguous range
   const int nz = N / TILE_M;
   const int nrows = N / 2 * nz * N;
   const int per = (nrows + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -397,19 +395,19 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
   uint32_t phase = 0;
   bool ok = true;
   for (int l = (int)blockIdx.x * per; l < l1 && ok;) {
-    const int y0 = l % N, z0 = (l / N) % nz * TILE_M, x0 = l / (N * nz) * 2;
-    const int run = min(l1 - l, N - y0);
-    gather_row(in, N, x0, y0 - 1, z0, sm);
+    const int x0 = l % N, z0 = (l / N) % nz * TILE_M, y0 = l / (N * nz) * 2;
+    const int run = min(l1 - l, N - x0);
+    gather_row(in, N, y0, x0 - 1, z0, sm);
     asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
     for (int q = 0; q < 2 * SLOTS; q++) tmem_zero16(mine + 16 * q);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     uint32_t r[2][16];
-    // row i holds y' = y0 - 1 + i
+    // row i holds x' = x0 - 1 + i
     for (int i = 0; i <= run + 1 && ok; i++) {
       // the other buffer's row i - 1 has been multiplied
-      if (i <= run) gather_row(in, N, x0, y0 + i, z0, sm + ((i + 1) & 1) * SROW_BYTES);
+      if (i <= run) gather_row(in, N, y0, x0 + i, z0, sm + ((i + 1) & 1) * SROW_BYTES);
       asm volatile("cp.async.commit_group;" ::: "memory");
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -418,17 +416,17 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
       if (tid == 0) {
         const uint32_t row = smem_u32(sm + (i & 1) * SROW_BYTES);
         const uint32_t b0 = smem_u32(sB) + (uint32_t)((2 - i % 3) * B_BYTES);
-        for (int xo = 0; xo < 2; xo++) {
+        for (int yo = 0; yo < 2; yo++) {
           for (int p = 0; p < 9; p++) {
-            // (dx, dz) = (p / 3, p % 3): line xo + dx, started dz rows on
+            // (dy, dz) = (p / 3, p % 3): line yo + dy, started dz rows on
             const uint64_t da = umma_desc(
-                row + (uint32_t)((xo + p / 3) * LINE_BYTES + (p % 3) * 16), HALF_BYTES, 128);
+                row + (uint32_t)((yo + p / 3) * LINE_BYTES + (p % 3) * 16), HALF_BYTES, 128);
             const uint64_t db = umma_desc(b0 + (uint32_t)(p * SB_BYTES), 128, 256);
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, %4, 0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                :: "r"(tmem + (uint32_t)(16 * SLOTS * xo)), "l"(da), "l"(db), "r"(kIdesc48),
+                :: "r"(tmem + (uint32_t)(16 * SLOTS * yo)), "l"(da), "l"(db), "r"(kIdesc48),
                    "r"(1u)
                 : "memory");
           }
@@ -439,9 +437,9 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
       }
       // the output that row i - 1 completed, beside this row's MMAs
       if (i >= 3) {
-        const size_t v = ((size_t)x0 * N + y0 + i - 3) * N + z0 + tid;
+        const size_t v = ((size_t)(x0 + i - 3) * N + y0) * N + z0 + tid;
         store_voxel(r[0], v, bias, act, gate, out_f, out_b, out4);
-        store_voxel(r[1], v + (size_t)N * N, bias, act, gate, out_f, out_b, out4);
+        store_voxel(r[1], v + N, bias, act, gate, out_f, out_b, out4);
       }
       const bool got = mbar_wait(bar, phase);
       ok = __syncthreads_and(got ? 1 : 0) != 0;
@@ -458,9 +456,9 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     if (ok) {
-      const size_t v = ((size_t)x0 * N + y0 + run - 1) * N + z0 + tid;
+      const size_t v = ((size_t)(x0 + run - 1) * N + y0) * N + z0 + tid;
       store_voxel(r[0], v, bias, act, gate, out_f, out_b, out4);
-      store_voxel(r[1], v + (size_t)N * N, bias, act, gate, out_f, out_b, out4);
+      store_voxel(r[1], v + N, bias, act, gate, out_f, out_b, out4);
     }
     // every copy has landed and every MMA has completed: the buffers are free
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -649,7 +647,7 @@ cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, con
   return cudaGetLastError();
 }
 
-// pipeline variant: 2 (the default) = the sweep along y (k_conv_sweep); 1 =
+// pipeline variant: 2 (the default) = the sweep along x (k_conv_sweep); 1 =
 // one tile at a time, one stage, 4 CTAs/SM; 0 = two stages, 2 CTAs/SM.
 // COLAGPU_CONV_VARIANT=0/1/2 selects one.
 int g_conv_variant = -1;      // conv_tc_set_variant

@@ -86,5 +86,5 @@ cudaError_t conv_wgrad_in(const __nv_bfloat162* in, const float* g, int N, float
 // Device error word of the tensor-core kernels (bounded waits that gave up).
 unsigned conv_tc_error_word();
 // Pipeline of the tensor-core convolutions: -1 by mesh size, 0 two stages,
-// 1 one stage, 2 the sweep along y (the default).  -1 returned on a bad value.
+// 1 one stage, 2 the sweep along x (the default).  -1 returned on a bad value.
 int conv_tc_set_variant(int v);

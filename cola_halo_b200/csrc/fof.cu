@@ -11,7 +11,8 @@
 //   1. wrap positions (move_particles2_min, fof.c:1042) and bin them on a
 //      grid of cells no smaller than ll (counting sort: count with ranks,
 //      scan, scatter); from here on a particle is its slot in cell order
-//   2. the particles of crowded cells are put in the order of their sub-cells
+//   2. the particles of crowded cells are put in the order of their sub-cells,
+//      and those of a block of 32 slots that hang together are joined
 //   3. each particle tests the later particles of the cells within ll of it;
 //      a link joins the two sets of a lock-free union-find over the slots
 //      (hooking one root under the other with atomicCAS, in a scrambled order
@@ -25,10 +26,11 @@
 // error word.
 //
 // 256^3 particles, L = 600, ll = 0.2 spacings, a third of them in halos: the
-// link kernel takes 5.8 ms (12.4 with all 27 neighbour cells and a union-find
+// link kernel takes 5.3 ms (12.4 with all 27 neighbour cells and a union-find
 // over the original indices; 8.8 with one candidate at a time), and the whole call
 // 10.2 ms (26.6).  The link kernel is bound by its chains of dependent L2 loads:
-// cell starts, candidates, parents.
+// cell starts, candidates, parents; two thirds of it are the slots outside
+// clumps.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -83,18 +85,15 @@ __global__ void k_fof_bin(const PMin* __restrict__ p, long long n, float L, floa
   }
 }
 
-// Wrapped position and original index at the particle's slot; the slot starts
-// as a set of its own.
+// Wrapped position and original index at the particle's slot.
 __global__ void k_fof_scatter(const PMin* __restrict__ p, const unsigned* __restrict__ key,
                               const unsigned* __restrict__ rank, long long n, float L,
-                              const unsigned* __restrict__ start, float4* __restrict__ pos,
-                              int* __restrict__ parent) {
+                              const unsigned* __restrict__ start, float4* __restrict__ pos) {
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < n;
        i += (long long)gridDim.x * T) {
     const float4 q = *reinterpret_cast<const float4*>(p + i);
     const unsigned slot = start[key[i]] + rank[i];
     pos[slot] = make_float4(wrap1(q.x, L), wrap1(q.y, L), wrap1(q.z, L), __int_as_float((int)i));
-    parent[i] = (int)i;
   }
 }
 
@@ -228,24 +227,49 @@ __global__ void __launch_bounds__(kSubThreads) k_fof_subsort(
 }
 
 // Bounding boxes of the blocks of 32 slots: box[2 b] the lower corner, box[2 b +
-// 1] the upper one.
-__global__ void k_fof_boxes(const float4* __restrict__ pos, long long n,
-                            float4* __restrict__ box) {
+// 1] the upper one; and their first sets.  In halos, where a block is a clump of
+// at most two cells across (marked in the lower corner's w), the slots that hang
+// together within it go under the first of them: 32 broadcasts and votes in
+// registers, where the link kernel would join them one pair after another through
+// L2 while other warps meet 32 sets in place of one (256^3: 5.8 to 5.3 ms of
+// link, for 0.15 here).  Other slots start as sets of their own.
+__global__ void k_fof_blocks(const float4* __restrict__ pos, long long n, float inv, float L,
+                             float ll2, float4* __restrict__ box, int* __restrict__ parent) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const float half = 0.5f * L;
   const int lane = threadIdx.x & 31;
   for (long long base = (long long)blockIdx.x * T + (threadIdx.x & ~31); base < n;
        base += (long long)gridDim.x * T) {
-    const float4 a = pos[min(base + lane, n - 1)];
+    const bool live = base + lane < n;
+    const float4 a = pos[live ? base + lane : n - 1];
     float lo[3] = {a.x, a.y, a.z}, hi[3] = {a.x, a.y, a.z};
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+        lo[k] = fminf(lo[k], __shfl_xor_sync(kAll, lo[k], o));
+        hi[k] = fmaxf(hi[k], __shfl_xor_sync(kAll, hi[k], o));
       }
+    // (the warp's lanes hold the same corners)
+    const bool clump =
+        fmaxf(fmaxf(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]) * inv <= 2.0f;
     if (lane == 0) {
-      box[base / 16] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+      box[base / 16] = make_float4(lo[0], lo[1], lo[2], clump ? 1.0f : 0.0f);
       box[base / 16 + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
     }
+    unsigned set = 1u << lane;      // the lanes that hang together with this one
+    if (clump)
+      for (int j = 0; j < 32; j++) {
+        float4 d;
+        d.x = __shfl_sync(kAll, a.x, j);
+        d.y = __shfl_sync(kAll, a.y, j);
+        d.z = __shfl_sync(kAll, a.z, j);
+        const bool linked = base + j < n && live && (lane == j || dist2(a, d, L, half) < ll2);
+        const unsigned near = __ballot_sync(kAll, linked);
+        // every set with a lane near j becomes one
+        const unsigned all = __ballot_sync(kAll, (set & near) != 0);
+        if (set & near) set = all;
+      }
+    if (live) parent[base + lane] = (int)base + __ffs(set) - 1;
   }
 }
 
@@ -254,14 +278,14 @@ __global__ void k_fof_boxes(const float4* __restrict__ pos, long long n,
 // consecutive in z, so a row is one range of slots, or two across the
 // periodic face, and rows before the particle's own hold no later slot.
 //
-// In halos, where a warp's 32 slots are a clump of at most two cells across,
-// its lanes take the same ranges (the cells within ll of the clump) and skip the
-// blocks of 32 candidates whose box is further than ll from the clump's.  Of a
-// block that is left each lane loads one candidate and finds its root.  Once the
-// clump is one set, candidates of that set drop out by one vote, and a link
-// takes all candidates of the set it joins out too, so that most blocks of a
-// halo cost two loads and no distance.  Elsewhere the few candidates are each
-// lane's own; their parents are loaded four at a time.
+// In a clump (k_fof_blocks), whose own pairs are done, the lanes take the same
+// ranges (the cells within ll of the clump) and skip the blocks of 32 candidates
+// whose box is further than ll from the clump's.  Of a block that is left each
+// lane loads one candidate and finds its root.  Once the clump is one set,
+// candidates of that set drop out by one vote, and a link takes all candidates
+// of the set it joins out too, so that most blocks of a halo cost two loads and
+// no distance.  Elsewhere the few candidates are each lane's own; their parents
+// are loaded four at a time.
 //
 // ra is an ancestor of s: a candidate whose parent or root it is belongs to the
 // set already, for sets never split.
@@ -280,15 +304,14 @@ __global__ void __launch_bounds__(T, 5) k_fof_link(const float4* __restrict__ po
     const float4 a = pos[s];
     float4 lo = box[base / 16], hi = box[base / 16 + 1];
     unsigned own = (unsigned)cell_of(a.x, inv, nc) * nc + cell_of(a.y, inv, nc);
-    const float wide = fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * inv;
-    const bool clump = wide <= 2.0f;
+    const bool clump = lo.w != 0.0f;
     if (clump) own = __reduce_min_sync(kAll, own);
     else lo = hi = a;
     int xl, xh, yl, yh, zl, zh;
     cells_within(lo.x, hi.x, reach, L, inv, nc, xl, xh);
     cells_within(lo.y, hi.y, reach, L, inv, nc, yl, yh);
     cells_within(lo.z, hi.z, reach, L, inv, nc, zl, zh);
-    int ra = (int)s;
+    int ra = clump ? __ldcg(parent + s) : (int)s;
     // slots t .. end - 1, each lane its own
     const auto test = [&](unsigned t, unsigned end) {
       t = max(t, s + 1);
@@ -334,7 +357,7 @@ __global__ void __launch_bounds__(T, 5) k_fof_link(const float4* __restrict__ po
     };
     // slots of the cells z0 .. z1 of a row; `near`: no periodic face in between
     const auto range = [&](unsigned row, int z0, int z1, bool near) {
-      unsigned t = max(start[row * nc + z0], (unsigned)base + 1);
+      unsigned t = max(start[row * nc + z0], (unsigned)base + (clump ? 32 : 1));
       const unsigned end = start[row * nc + z1 + 1];
       if (!clump) {
         test(t, end);
@@ -574,7 +597,7 @@ extern "C" int cg_fof(const void* pmin, long long np, float boxsize, float ll, i
     k_fof_bin<<<g, T, 0, st>>>(d_p, np, boxsize, inv, (int)nc, key, rank, start);
     cgscan::exclusive(start, start, ncells + 1, bsum, nullptr, CG_ST_OTHER, st);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_scatter<<<g, T, 0, st>>>(d_p, key, rank, np, boxsize, start, pos, parent);
+    k_fof_scatter<<<g, T, 0, st>>>(d_p, key, rank, np, boxsize, start, pos);
     // (the list of dense cells goes where the ranks were)
     prof_mark(st, CG_ST_OTHER);
     k_fof_dense<<<g, T, 0, st>>>(pos, np, start, (int)nc, inv, rank, word + 2);
@@ -582,7 +605,7 @@ extern "C" int cg_fof(const void* pmin, long long np, float boxsize, float ll, i
     k_fof_subsort<<<cg_grid(np, 4), kSubThreads, 0, st>>>(pos, start, (int)nc, inv, rank,
                                                           word + 2);
     prof_mark(st, CG_ST_OTHER);
-    k_fof_boxes<<<g, T, 0, st>>>(pos, np, box);
+    k_fof_blocks<<<g, T, 0, st>>>(pos, np, inv, boxsize, ll * ll, box, parent);
     prof_mark(st, CG_ST_OTHER);
     k_fof_link<<<g, T, 0, st>>>(pos, np, box, start, (int)nc, inv, boxsize, ll * ll, reach,
                                 parent, word + 1);

@@ -182,8 +182,9 @@ def dist_setup(args):
 
 
 def algorithmic_bytes(stage, N, npart, reset=True):
-    """Algorithmic bytes per launch of each stage (each tensor counted once):
-    the deposit reads the positions and writes the mesh once; the z r2c reads
+    """Algorithmic bytes per launch of each stage (each tensor counted once;
+    the inverse x and z passes per force component, launch_parts): the
+    deposit reads the positions and writes the mesh once; the z r2c reads
     the mesh, writes the half spectrum and (reset) writes -1 back over the
     mesh for the next deposit."""
     Mr = 4.0 * N ** 3
@@ -202,6 +203,14 @@ def algorithmic_bytes(stage, N, npart, reset=True):
         "drift": 60.0 * npart,
         "kick_drift": 84.0 * npart,
     }.get(stage)
+
+
+def launch_parts(name, stages):
+    """Force components per launch of the inverse x and z passes (one launch
+    for all three, or one each), 1 for every other stage."""
+    if name not in ("fx_inv", "zi_c2r") or "green_y" not in stages:
+        return 1
+    return 3 * stages["green_y"]["launches"] // stages[name]["launches"]
 
 
 def load_traffic():
@@ -497,8 +506,10 @@ def run_b200(args, cfg):
     hbm, peak_kind = peaks()
     dom = max(stages, key=lambda k: stages[k]["ms"])
     per_launch_ms = stages[dom]["ms"] / stages[dom]["launches"]
-    ab = algorithmic_bytes(dom, N, npart)
+    parts = launch_parts(dom, stages)
+    ab = algorithmic_bytes(dom, N, npart) * parts
     traffic = load_traffic().get("%s@%d" % (dom, N))
+    traffic = traffic and traffic * parts
     roofline = {"kernel": dom, "bound": "hbm",
                 "achieved": ab / (per_launch_ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                 "frac": ab / (per_launch_ms / 1e3) / 1e9 / hbm, "traffic": traffic,
@@ -509,6 +520,7 @@ def run_b200(args, cfg):
         b = algorithmic_bytes(name, N, npart)
         if b is None or not st["launches"]:
             continue
+        b *= launch_parts(name, stages)
         t = st["ms"] / st["launches"] / 1e3
         stage_roofline[name] = {"ms_per_launch": round(t * 1e3, 4),
                                 "gbs": round(b / t / 1e9, 1), "frac": round(b / t / 1e9 / hbm, 3)}

@@ -103,8 +103,8 @@ cudaError_t mesh_r2c(const MeshFFT* f, const float* real, float2* spec, cudaStre
 cudaError_t mesh_c2r(const MeshFFT* f, float2* spec, float* real, cudaStream_t st);
 
 // Schedule of the FFT passes of one mesh size: which compiled variant of the
-// strided x pass and of the fused Green pass runs (pm_kernels.cu fx_cfg,
-// green_cfg).  Variants other than 0 exist from 256 up (Green: up to 768).
+// strided x pass and of the fused Green pass runs (fx_shapes.h,
+// pm_kernels.cu green_cfg).  Variants other than 0 exist from 256 up (Green: up to 768).
 #define PM_NUM_FX_VARIANTS 3
 #define PM_NUM_GREEN_VARIANTS 7
 #define PM_NUM_DEP_VARIANTS 6

@@ -36,10 +36,17 @@
 #include <mutex>
 
 #include "fft_core.cuh"
+#include "fx_shapes.h"
 #include "internal.h"
 #include "scan.cuh"
 
 using cgfft::cplx;
+using cgfx::FxCfg;
+using cgfx::FxDirectCfg;
+using cgfx::MIN_TUNED_N;
+using cgfx::fx_cfg;
+using cgfx::fx_direct_cfg;
+using cgfx::fx_threads;
 
 // TMA maps of the x pass for tk columns per CTA (encoded on demand).
 bool x_maps_for(PmPlan* p, int tk);
@@ -439,13 +446,9 @@ using cgfft::Gmem;
 using cgfft::SmemCol;
 using cgfft::SmemLine;
 
-// Schedules of the strided x pass and the fused y Green pass.  Variant 0
-// is the default; the others are compiled for meshes from MIN_TUNED_N up
-// and chosen per mesh size by the autotuner (pm_autotune) or set
-// explicitly.  x pass: ky columns per CTA and maximum radix (fx_cfg).  Green
-// pass: lines per CTA, maximum radix and the resident CTAs per SM the kernel
-// is register-limited to (green_cfg).
-constexpr int MIN_TUNED_N = 256;
+// Schedules of the strided x pass (fx_shapes.h) and the fused y Green pass:
+// lines per CTA, maximum radix and the resident CTAs per SM the kernel is
+// register-limited to (green_cfg).
 // Variants compiled at size N.  The 8-line Green variants stop at 768: at
 // 1024 they would spill registers.
 __host__ __device__ constexpr int n_fx_variants(int N) {
@@ -453,18 +456,6 @@ __host__ __device__ constexpr int n_fx_variants(int N) {
 }
 __host__ __device__ constexpr int n_green_variants(int N) {
   return N >= MIN_TUNED_N && N <= 768 ? PM_NUM_GREEN_VARIANTS : 1;
-}
-// x pass by mesh size.  Default: 16 columns (128-byte rows) from 256 to 768,
-// where the twiddles sit in shared memory and the 16-column form fits 2 CTAs
-// per SM; 8 columns at 1024, where they do not and it would fit one; 8 below
-// 256, where 16 would leave fewer CTAs than SMs have room for.  One inverse
-// launch, ms, as {16 columns radix 16, 8 columns radix 16, 8 columns radix 8}:
-// 256: 0.024, 0.029, 0.029; 384: 0.079, 0.084, 0.097; 512: 0.183, 0.193,
-// 0.182; 768: 0.566, 0.654, 0.734; 1024: 2.04, 1.53, 1.81.
-struct FxCfg { int tk, rm; };
-__host__ __device__ constexpr FxCfg fx_cfg(int N, int v) {
-  const bool wide = N >= 256 && N < 1024;
-  return v == 1 ? FxCfg{8, 8} : ((v == 0) == wide ? FxCfg{16, 16} : FxCfg{8, 16});
 }
 struct GreenCfg { int byg, rm, minb, thr; };
 // The tuned shapes of the Green pass (entry 0 stands for green_cfg's default).
@@ -504,18 +495,12 @@ __host__ __device__ constexpr GreenCfg green_cfg(int N, int v) {
 // nor __restrict__ there.
 template <bool RESET> using DensPtr = typename std::conditional<RESET, float*, const float*>::type;
 
-// Threads of the z r2c and of the TMA x passes by mesh size: those whose
-// radix-16 stages (TY N / 32 butterflies a CTA in z, N / 16 per column in x)
-// fill them in whole rounds.  us with 256 threads and with these: z r2c 512:
-// 275, 261; 384: 134, 119; 128: 10.4, 8.7; x inverse (three components) 1024:
-// 4709, 4408; 192: 34, 31; 144: 16.9, 14.8; 96: 8.3, 6.7.
+// Threads of the z r2c by mesh size: those whose radix-16 stages (TY N / 32
+// butterflies a CTA) fill them in whole rounds.  us with 256 threads and with these: 512:
+// 275, 261; 384: 134, 119; 128: 10.4, 8.7.
 __host__ __device__ constexpr int fz_threads(int N) {
   return N == 128 || N == 144 || (N >= 256 && N <= 512) ? 128 : 256;
 }
-__host__ __device__ constexpr int fx_threads(int N, int tk, int rm) {
-  return N <= 192 || (N >= 1024 && tk == 8 && rm == 16) ? 128 : 256;
-}
-
 // The split of k_fz (after the H-point transform of the TY lines in `mid`):
 // X_k for k = 0..H stored transposed into S[kz][x][y0 + b], and the lines'
 // sum Re Z_0 + Im Z_0 added to *dsum in double.
@@ -821,21 +806,21 @@ struct GmemScaled {
 // (the same array for an in-place pass).  SCALE 0: plain; 1 / 2: the input
 // is first multiplied by n_x / n_z (GmemScaled; gtab: the gradient table or
 // NULL, unused by SCALE 0).
-template <int N, int DIR, int SCALE, int TKV, int RMX>
-__global__ void __launch_bounds__(T) k_fx(const float2* in, float2* out,
-                                          const float2* __restrict__ twN,
-                                          const float* __restrict__ gtab) {
+template <int N, int DIR, int SCALE, int TKV, int RMX, int TT, int MINB>
+__global__ void __launch_bounds__(TT, MINB) k_fx(const float2* in, float2* out,
+                                                 const float2* __restrict__ twN,
+                                                 const float* __restrict__ gtab) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const SmemCol<TKV> mid{reinterpret_cast<cplx*>(smraw)};
   const size_t off = (size_t)blockIdx.y * N * N + blockIdx.x * TKV;
   const cgfft::GmemC<1, N> go{out + off};
   if constexpr (SCALE == 0) {
     const cgfft::GmemC<1, N> gi{const_cast<float2*>(in) + off};
-    cgfft::fft_io<N, TKV, T, false, DIR, RMX>(gi, mid, go, twN);
+    cgfft::fft_io<N, TKV, TT, false, DIR, RMX>(gi, mid, go, twN);
   } else {
     const float fz = SCALE == 2 && gtab ? __ldg(gtab + blockIdx.y) : (float)blockIdx.y;
     const GmemScaled<SCALE> gi{in + off, (size_t)N, N, fz, gtab};
-    cgfft::fft_io<N, TKV, T, false, DIR, RMX>(gi, mid, go, twN);
+    cgfft::fft_io<N, TKV, TT, false, DIR, RMX>(gi, mid, go, twN);
   }
 }
 
@@ -1806,7 +1791,8 @@ struct MeshKernels {
   void (*zip)(CUtensorMap, const float2*, const float4*, const unsigned*, float*, float*,
               const float2*, const float2*, float, unsigned*);
   size_t sm_fz, sm_fy, sm_fx, sm_green, sm_zi, sm_zi_tma, sm_zi_sw;
-  int tk;    // ky columns per CTA of the x pass
+  int tk;    // ky columns per CTA of the TMA x pass
+  int tkd, tfd;   // those of the direct x pass, and its threads
   int byg;   // lines per CTA of the Green pass
   int tg;    // threads per CTA of the Green pass
   int tfz, tfx, tzi;   // of the z r2c, the TMA x passes, the TMA z c2r
@@ -1815,15 +1801,18 @@ struct MeshKernels {
 template <int N, int V>
 void set_fx(MeshKernels* k) {
   constexpr int TKV = fx_cfg(N, V).tk, RMX = fx_cfg(N, V).rm;
-  k->fxf = k_fx<N, -1, 0, TKV, RMX>;
-  k->fxi = k_fx<N, 1, 0, TKV, RMX>;
-  k->fxi_x = k_fx<N, 1, 1, TKV, RMX>;
-  k->fxi_z = k_fx<N, 1, 2, TKV, RMX>;
+  constexpr FxDirectCfg d = fx_direct_cfg(N, V);
+  k->fxf = k_fx<N, -1, 0, d.tk, d.rm, d.thr, d.minb>;
+  k->fxi = k_fx<N, 1, 0, d.tk, d.rm, d.thr, d.minb>;
+  k->fxi_x = k_fx<N, 1, 1, d.tk, d.rm, d.thr, d.minb>;
+  k->fxi_z = k_fx<N, 1, 2, d.tk, d.rm, d.thr, d.minb>;
+  k->sm_fx = sizeof(cplx) * cgfft::col_tile_elems<N, d.tk>();
+  k->tkd = d.tk;
+  k->tfd = d.thr;
   k->fxf_sw = k_fx_sw<N, TKV, RMX>;
   k->fxi3_sw = k_fx_inv_sw<N, TKV, RMX>;
   k->sm_fx_sw = fx_sw_smem<N, TKV, RMX>();
   k->tfx = fx_threads(N, TKV, RMX);
-  k->sm_fx = sizeof(cplx) * cgfft::col_tile_elems<N, TKV>();
   k->tk = TKV;
 }
 
@@ -2201,8 +2190,8 @@ cudaError_t pm_autotune(PmPlan* p, cudaStream_t st, MeshSched* best, float* ms_g
             p->xtm[0], p->xtm[1], FxInvArgs{0, {p->gsp[0], p->gsp[1], p->gsp[2]}, nullptr},
             p->twN, p->err);
       else
-        k.fxi_x<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->gsp[2], p->gsp[0], p->twN,
-                                                               nullptr);
+        k.fxi_x<<<dim3(N / k.tkd, N / 2 + 1), k.tfd, k.sm_fx, st>>>(p->gsp[2], p->gsp[0], p->twN,
+                                                                    nullptr);
     }, tx);
   if (e != cudaSuccess) return e;
   float tbest = 1e30f;
@@ -2329,7 +2318,7 @@ cudaError_t mesh_r2c(const MeshFFT* f, const float* real, float2* spec, cudaStre
   prof_mark(st, CG_ST_OTHER);
   k.fyf<<<(N / 2 + 1) * N / BY, T, k.sm_fy, st>>>(spec, f->twN);
   prof_mark(st, CG_ST_FX_FWD);
-  k.fxf<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(spec, spec, f->twN, nullptr);
+  k.fxf<<<dim3(N / k.tkd, N / 2 + 1), k.tfd, k.sm_fx, st>>>(spec, spec, f->twN, nullptr);
   return cudaGetLastError();
 }
 
@@ -2338,7 +2327,7 @@ cudaError_t mesh_c2r(const MeshFFT* f, float2* spec, float* real, cudaStream_t s
   if (!get_kernels(f->N, &k)) return cudaErrorInvalidValue;
   const int N = f->N;
   prof_mark(st, CG_ST_FX_INV);
-  k.fxi<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(spec, spec, f->twN, nullptr);
+  k.fxi<<<dim3(N / k.tkd, N / 2 + 1), k.tfd, k.sm_fx, st>>>(spec, spec, f->twN, nullptr);
   prof_mark(st, CG_ST_OTHER);
   k.fyi<<<(N / 2 + 1) * N / BY, T, k.sm_fy, st>>>(spec, f->twN);
   prof_mark(st, CG_ST_ZI);
@@ -2455,7 +2444,7 @@ void launch_fx_fwd(PmPlan* p, const MeshKernels& k, cudaStream_t st) {
     k.fxf_sw<<<dim3(N / k.tk, N / 2 + 1), k.tfx, k.sm_fx_sw, st>>>(p->xtm[0], p->spec, p->twN,
                                                                p->err);
   else
-    k.fxf<<<dim3(N / k.tk, N / 2 + 1), T, k.sm_fx, st>>>(p->spec, p->spec, p->twN, nullptr);
+    k.fxf<<<dim3(N / k.tkd, N / 2 + 1), k.tfd, k.sm_fx, st>>>(p->spec, p->spec, p->twN, nullptr);
 }
 
 cudaError_t pm_r2c(PmPlan* p, cudaStream_t st) {
@@ -2669,8 +2658,8 @@ static cudaError_t green_x_zi(PmPlan* p, cudaStream_t st, bool zi) {
                      p->kfilt_n, p->kfilt_inv_dn, p->ktab};
   (gm.t || gm.tab ? k.green_mods : k.green)<<<(N / 2 + 1) * N / k.byg, k.tg, k.sm_green, st>>>(
       p->spec, p->gsp[1], p->spec, p->twN, p->f1, gm);
-  const dim3 gx(N / k.tk, N / 2 + 1);
   const bool xsw = x_maps_for(p, k.tk);
+  const dim3 gx(N / (xsw ? k.tk : k.tkd), N / 2 + 1);
   // Components per launch.  All three at once, except where one spectrum stays
   // in L2 from its x pass to its z c2r but three do not (256: 68 MB each): one
   // after the other there (all at once: 30 us of 380 a force slower).
@@ -2683,11 +2672,11 @@ static cudaError_t green_x_zi(PmPlan* p, cudaStream_t st, bool zi) {
           p->err);
     } else {
       prof_mark(st, CG_ST_FX_INV);
-      k.fxi_x<<<gx, T, k.sm_fx, st>>>(p->spec, p->gsp[0], p->twN, p->ktab);
+      k.fxi_x<<<gx, k.tfd, k.sm_fx, st>>>(p->spec, p->gsp[0], p->twN, p->ktab);
       prof_mark(st, CG_ST_FX_INV);
-      k.fxi<<<gx, T, k.sm_fx, st>>>(p->gsp[1], p->gsp[1], p->twN, nullptr);
+      k.fxi<<<gx, k.tfd, k.sm_fx, st>>>(p->gsp[1], p->gsp[1], p->twN, nullptr);
       prof_mark(st, CG_ST_FX_INV);
-      k.fxi_z<<<gx, T, k.sm_fx, st>>>(p->spec, p->gsp[2], p->twN, p->ktab);
+      k.fxi_z<<<gx, k.tfd, k.sm_fx, st>>>(p->spec, p->gsp[2], p->twN, p->ktab);
     }
     if (zi) launch_zi(p, k, c, nc, st);
   }
@@ -2783,20 +2772,20 @@ cudaError_t pm_slab_kspace(PmPlan* p, int kz0, int nkz, cudaStream_t st) {
   cudaError_t e = sgn_table(p, &sgn);
   if (e != cudaSuccess) return e;
   const size_t off = (size_t)kz0 * N * N;
-  const dim3 gx(N / k.tk, nkz);
+  const dim3 gx(N / k.tkd, nkz);
   prof_mark(st, CG_ST_FX_FWD);
-  k.fxf<<<gx, T, k.sm_fx, st>>>(p->spec + off, p->spec + off, p->twN, nullptr);
+  k.fxf<<<gx, k.tfd, k.sm_fx, st>>>(p->spec + off, p->spec + off, p->twN, nullptr);
   prof_mark(st, CG_ST_GREEN);
   GreenMods gm{p->kfilt_cur >= 0 ? p->kfilt + (size_t)p->kfilt_cur * p->kfilt_n : nullptr,
                p->kfilt_n, p->kfilt_inv_dn, p->ktab, kz0};
   (gm.t || gm.tab ? k.green_mods : k.green)<<<nkz * N / k.byg, k.tg, k.sm_green, st>>>(
       p->spec + off, p->gsp[1] + off, p->gsp[2] + off, p->twN, p->f1, gm);
   prof_mark(st, CG_ST_FX_INV);
-  k.fxi_x<<<gx, T, k.sm_fx, st>>>(p->gsp[2] + off, p->gsp[0] + off, p->twN, p->ktab);
+  k.fxi_x<<<gx, k.tfd, k.sm_fx, st>>>(p->gsp[2] + off, p->gsp[0] + off, p->twN, p->ktab);
   prof_mark(st, CG_ST_FX_INV);
-  k.fxi<<<gx, T, k.sm_fx, st>>>(p->gsp[1] + off, p->gsp[1] + off, p->twN, nullptr);
+  k.fxi<<<gx, k.tfd, k.sm_fx, st>>>(p->gsp[1] + off, p->gsp[1] + off, p->twN, nullptr);
   prof_mark(st, CG_ST_FX_INV);
-  k.fxi_z<<<gx, T, k.sm_fx, st>>>(p->gsp[2] + off, p->gsp[2] + off, p->twN,
+  k.fxi_z<<<gx, k.tfd, k.sm_fx, st>>>(p->gsp[2] + off, p->gsp[2] + off, p->twN,
                                   (p->ktab ? p->ktab : sgn) + kz0);
   return cudaGetLastError();
 }

@@ -9,6 +9,9 @@
 // COLAGPU_TUNE_CACHE names a file, appended to it as one line
 //   <device name> TAB <ngrid> TAB <green variant> TAB <x variant>
 // so that later processes on the same kind of GPU reuse it without timing.
+// The numbers stand for the shapes of one build: they count only below a line
+// kShapes, which the first entry of a build that changed the shapes writes; what
+// stands above it, or below another such line, is timed again.
 // A cached or installed schedule also makes runs reproducible: variants
 // differ in rounding (different radix orders), not in the algorithm.
 #include <cuda_runtime.h>
@@ -48,21 +51,40 @@ std::string device_name() {
   return s;
 }
 
-// The last line of the cache file for (device, N), if any.
+// Names the shapes (fx_cfg, green_cfg) that the numbers refer to; another name for
+// every change of them.
+constexpr char kShapesTag[] = "#shapes";
+constexpr char kShapes[] = "#shapes 2026-12";
+bool is_shapes(const char* line, const char* want) {
+  const size_t n = strlen(want);
+  return strncmp(line, want, n) == 0 && (!line[n] || strchr(" \r\n", line[n]));
+}
+
+// Whether the entries at the end of the cache file are of these shapes.
+bool cache_current(FILE* f) {
+  char line[512];
+  bool ours = false;
+  while (fgets(line, sizeof(line), f))
+    if (is_shapes(line, kShapesTag)) ours = is_shapes(line, kShapes);
+  return ours;
+}
+
+// The last line of the cache file for (device, N) of these shapes, if any.
 bool cache_lookup(const std::string& dev, int N, MeshSched* out) {
   const char* path = getenv("COLAGPU_TUNE_CACHE");
   if (!path || !*path) return false;
   FILE* f = fopen(path, "r");
   if (!f) return false;
   char line[512];
-  bool found = false;
+  bool found = false, ours = false;
   while (fgets(line, sizeof(line), f)) {
+    if (is_shapes(line, kShapesTag)) ours = is_shapes(line, kShapes);
     char* tab = strchr(line, '\t');
     if (!tab) continue;
     *tab = 0;
     int n = 0, g = 0, x = 0;
     if (sscanf(tab + 1, "%d\t%d\t%d", &n, &g, &x) != 3) continue;
-    if (dev == line && n == N) {
+    if (ours && dev == line && n == N) {
       out->green = g;
       out->fx = x;
       found = true;
@@ -75,8 +97,14 @@ bool cache_lookup(const std::string& dev, int N, MeshSched* out) {
 void cache_store(const std::string& dev, int N, MeshSched s) {
   const char* path = getenv("COLAGPU_TUNE_CACHE");
   if (!path || !*path) return;
+  bool ours = false;
+  if (FILE* r = fopen(path, "r")) {
+    ours = cache_current(r);
+    fclose(r);
+  }
   FILE* f = fopen(path, "a");
   if (!f) return;
+  if (!ours) fprintf(f, "%s\n", kShapes);
   fprintf(f, "%s\t%d\t%d\t%d\n", dev.c_str(), N, s.green, s.fx);
   fclose(f);
 }

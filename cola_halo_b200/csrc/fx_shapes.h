@@ -11,7 +11,9 @@ namespace cgfx {
 // autotuner (pm_autotune) or set explicitly.
 constexpr int MIN_TUNED_N = 256;
 
-// TMA form.  Default: 16 columns (128-byte rows) from 256 to 768, where the
+// TMA form.  A variant's number keeps its shape from one build to the next (cached
+// and saved schedules hold numbers): 0 the default, 1 8 columns at radix 8 (16
+// from 768 up), 2 16 columns at radix 16.  Default: 16 columns (128-byte rows) from 256 to 768, where the
 // twiddles sit in shared memory and the 16-column form fits 2 CTAs per SM; 8
 // columns at 1024, where they do not and it would fit one; 8 below 256, where
 // 16 would leave fewer CTAs than SMs have room for.  One inverse launch, ms, as
@@ -20,8 +22,13 @@ constexpr int MIN_TUNED_N = 256;
 // 0.182; 768: 0.566, 0.654, 0.734; 1024: 2.04, 1.53, 1.81.
 struct FxCfg { int tk, rm; };
 constexpr FxCfg fx_cfg(int N, int v) {
-  const bool wide = N >= 256 && N < 1024;
-  return v == 1 ? FxCfg{8, 8} : ((v == 0) == wide ? FxCfg{16, 16} : FxCfg{8, 16});
+  if (v == 1) return FxCfg{8, N >= 768 ? 16 : 8};
+  return v == 2 || (N >= 256 && N < 1024) ? FxCfg{16, 16} : FxCfg{8, 16};
+}
+// The first variant of v's shape (the default is one of the others).
+constexpr int fx_first(int N, int v) {
+  const FxCfg a = fx_cfg(N, 0), b = fx_cfg(N, v);
+  return a.tk == b.tk && a.rm == b.rm ? 0 : v;
 }
 
 // Threads of the TMA form by mesh size: those whose radix-16 stages (N / 16

@@ -2194,6 +2194,9 @@ cudaError_t pm_autotune(PmPlan* p, cudaStream_t st, MeshSched* best, float* ms_g
                                                                     nullptr);
     }, tx);
   if (e != cudaSuccess) return e;
+  // one shape, one time: the default stands for the variant of its shape
+  for (int v = 1; v < nf; v++)
+    if (cgfx::fx_first(N, v) == 0) tx[0] = tx[v] = std::min(tx[0], tx[v]);
   float tbest = 1e30f;
   for (int v = 0; v < ng; v++) {
     if (ms_green) ms_green[v] = tg[v];

@@ -325,7 +325,9 @@ int cg_sim_write_gadget(cg_sim* s, double aout, float omega_m, float h, const ch
  * the best time of every variant when they were timed.  CG_TUNE_FORCE
  * re-times.  The variants agree to float rounding; a fixed schedule
  * (cached, or set with cg_set_schedule) makes runs bit-reproducible.
- * Variant 0 is the default; sizes below 256 have only variant 0.  Tune
+ * Variant 0 is the default, whose shape may change from build to build; the
+ * other numbers keep theirs (x pass: 1 is 8 columns, 2 is 16).  Cached entries
+ * of other shapes are not used.  Sizes below 256 have only variant 0.  Tune
  * outside stream capture. */
 #define CG_TUNE_FORCE 1
 int cg_autotune(int ngrid, int flags, float* ms_green, float* ms_fx);

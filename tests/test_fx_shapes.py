@@ -53,3 +53,14 @@ def test_direct_form_has_its_own_shape(shapes):
         assert n % tk == 0 and n % dtk == 0 and thr % 32 == 0, (n, v)
         if rm == 16:
             assert n // 16 * dtk <= 2 * thr, (n, v)
+
+
+def test_variant_numbers_keep_their_shapes(shapes):
+    """Saved schedules hold variant numbers: 1 is 8 columns at radix 8 (16 from 768
+    up) and 2 is 16 columns at radix 16 on every mesh that has them; the default
+    is one of the shapes that were timed, and no mesh lists a shape twice but
+    for the default."""
+    for n in MESHES[MESHES.index(256):]:
+        assert shapes[n, 1][:2] == (8, 16 if n >= 768 else 8), n
+        assert shapes[n, 2][:2] == (16, 16), n
+        assert shapes[n, 0][:2] in ((16, 16), (8, 16)), n

@@ -99,3 +99,27 @@ def test_autotune_times_installs_and_caches(gpu_lib, tmp_path):
             os.environ["COLAGPU_TUNE_CACHE"] = old
         gpu_lib.cg_set_schedule(384, 0, 0)
         gpu_lib.cg_set_schedule(512, 0, 0)
+
+
+def test_cached_entries_of_other_shapes_are_timed_again(gpu_lib, tmp_path, monkeypatch):
+    """A line that no line of this build's shapes precedes (an older build's file),
+    and one below another build's, hold numbers of other shapes: the mesh is
+    timed, and the choice goes below a line of its own."""
+    import torch
+    dev = torch.cuda.get_device_name(0)
+    cache = tmp_path / "schedules.txt"
+    cache.write_text("%s\t256\t1\t1\n#shapes of another build\n%s\t256\t2\t1\n" % (dev, dev))
+    monkeypatch.setenv("COLAGPU_TUNE_CACHE", str(cache))
+    ng, nf = _variants(gpu_lib, 256)
+    mg, mf = (ctypes.c_float * ng)(), (ctypes.c_float * nf)()
+    try:
+        assert gpu_lib.cg_autotune(256, 0, mg, mf) == 0, gpu_lib.cg_last_error()
+        assert all(t > 0 for t in mg) and all(t > 0 for t in mf)
+        g, f = _schedule(gpu_lib, 256)
+        lines = cache.read_text().splitlines()
+        assert lines[-2].startswith("#shapes ") and lines[-2] != lines[1]
+        assert lines[-1] == "%s\t256\t%d\t%d" % (dev, g, f)
+        # one shape, one time
+        assert f != 2 and mf[2] == mf[0]
+    finally:
+        gpu_lib.cg_set_schedule(256, 0, 0)

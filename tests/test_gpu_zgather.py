@@ -60,10 +60,11 @@ def test_z_gathers_bit_identical(gpu_lib, bbks_table, nc, L):
 
 
 @pytest.mark.parametrize("nc,L,fxv", [(16, 100.0, None), (32, 200.0, None), (128, 300.0, 0),
-                                      (128, 300.0, 2)])
+                                      (128, 300.0, 1), (128, 300.0, 2)])
 def test_x_gathers_bit_identical(gpu_lib, bbks_table, nc, L, fxv):
-    """fxv: the x-pass schedule variant (0: 8 columns per CTA, 64-byte rows;
-    2: 16 columns, 128-byte rows), None below 256 where only one exists."""
+    """fxv: the x-pass schedule variant (1: 8 columns per CTA, 64-byte rows;
+    2, and 0 here: 16 columns, 128-byte rows), None below 256 where only one
+    exists."""
     try:
         runs = [_force_run(gpu_lib, 2, nc, L, bbks_table, True, xmode=m, fx_variant=fxv)
                 for m in (0, 1)]

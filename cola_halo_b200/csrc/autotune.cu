@@ -151,7 +151,7 @@ extern "C" int cg_get_deposit_variant(int ngrid) {
 }
 
 extern "C" int cg_set_deposit_variant(int ngrid, int variant) {
-  if (!pm_supported_mesh(ngrid) || variant < 0 || variant >= PM_NUM_DEP_VARIANTS)
+  if (!pm_supported_mesh(ngrid) || variant < 0 || variant > PM_NUM_DEP_VARIANTS)
     return cg_set_error_from_lpt(CG_EINVAL, "cg_set_deposit_variant: bad arguments");
   MeshSched s = pm_get_schedule(ngrid);
   s.dep = variant;

@@ -111,7 +111,8 @@ cudaError_t mesh_c2r(const MeshFFT* f, float2* spec, float* real, cudaStream_t s
 struct MeshSched {
   int green = 0;
   int fx = 0;
-  int dep = 0;   // deposit shape (pm_kernels.cu kDepCfg)
+  int dep = PM_NUM_DEP_VARIANTS;   // deposit shape (pm_kernels.cu kDepCfg), or by the
+                                   // particles' order and number
 };
 
 // pm_kernels.cu

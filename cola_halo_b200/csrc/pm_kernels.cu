@@ -240,11 +240,11 @@ __global__ void __launch_bounds__(T) k_deposit(const float* __restrict__ x0,
 // Shapes of the box deposit (particles per CTA, box cells of shared memory),
 // a schedule parameter per mesh size chosen by cg_sim_tune_deposit on the
 // particles of a run; chunk 0: every cloud takes the global atomics
-// (k_deposit).  Variant 0 (the default) is the first box for particles in cell
-// order, where a chunk in a halo covers few cells; in lattice order a chunk
-// spans the box along z whatever its particles do, no box fits, and variant 0
-// takes k_deposit, which merges neighbours along z (us, boxes against that:
-// halos formed, 128^3 on 128^3 76, 53; 256^3 on 512^3 594, 504; on 768^3 895, 813;
+// (k_deposit).  Until one is set or tuned (deposit_choice), particles in cell
+// order take the first box, for a chunk in a halo covers few cells; in lattice
+// order a chunk spans the box along z whatever its particles do, no box fits,
+// and they take k_deposit, which merges neighbours along z (us, boxes against
+// that: halos formed, 128^3 on 128^3 76, 53; 256^3 on 512^3 594, 504; on 768^3 895, 813;
 // lattice, 256^3 on 512^3 333, 266; on 768^3 424, 374; 512^3 on 1024^3 2620, 2080).
 struct DepCfg { int chunk, vmax; };
 constexpr DepCfg kDepCfg[PM_NUM_DEP_VARIANTS] = {
@@ -2079,18 +2079,17 @@ void launch_deposit(PmPlan* p, const float* const x[3], long long n, int v, cuda
   }
 }
 
-// The deposit variant of the schedule; 0 leaves the choice to the order of
-// the particles (kDepCfg), and to their number: below kMergeFrom the one-pass
+// The deposit variant of the schedule or, where none was set or tuned, the one
+// for the order of the particles (kDepCfg) and their number: below kMergeFrom the one-pass
 // deposit is a fraction of a wave and as long as its atomics' latency, and the
 // boxes take no longer (32^3 on 96^3: 31.0 us a force with boxes, 31.3 without;
 // 128^3 on 128^3: 214 and 190) and add each particle's share in one order from
 // run to run.
 constexpr long long kMergeFrom = 1 << 17;
-int deposit_by_order(const PmPlan* p, long long n, int v) {
-  return v == 0 && !p->cell_order && n >= kMergeFrom ? PM_NUM_DEP_VARIANTS - 1 : v;
-}
 int deposit_choice(const PmPlan* p, long long n) {
-  return deposit_by_order(p, n, sched_for(p->N).dep);
+  const int v = sched_for(p->N).dep;
+  if (v < PM_NUM_DEP_VARIANTS) return v;
+  return !p->cell_order && n >= kMergeFrom ? PM_NUM_DEP_VARIANTS - 1 : 0;
 }
 
 bool pm_supported_mesh(int N) {
@@ -2871,7 +2870,7 @@ cudaError_t pm_tune_deposit(PmPlan* p, const float* const x[3], long long n, cud
       prof_mark(st, CG_ST_FILL);
       k_fill<<<grid_for((long long)n4), T, 0, st>>>(reinterpret_cast<float4*>(p->dens), n4, -1.0f);
       cudaEventRecord(a, st);
-      launch_deposit(p, x, n, deposit_by_order(p, n, v), st);
+      launch_deposit(p, x, n, v, st);
       cudaEventRecord(b, st);
       e = cudaEventSynchronize(b);
       float tr = 0.0f;

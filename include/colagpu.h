@@ -399,13 +399,14 @@ int cg_sim_slab_interp(cg_sim* s, int x0, int nx, const float* bx, long long nb,
  * sets the particles per CTA and the shared-memory box (512 / 3,072 cells,
  * 256 / 3,072, 1,024 / 6,144, 2,048 / 12,288, 512 / 6,144, or global
  * atomics only, the sums of neighbouring particles merged in the warp).
- * Variant 0, the default, is that box for particles in cell order and for few
- * particles, and global atomics otherwise.  cg_sim_tune_deposit times every variant on the handle's
- * current particles (best of 3 CUDA-event timings), installs the fastest
- * for the handle's mesh size and returns it (or a negative CG_E* code); ms
- * (may be NULL) receives each variant's time.  It wraps the positions into
- * the box first (move_particles2's wrap) and leaves a deposit of them in
- * the density mesh.  All variants give the same density to float
+ * Until one is set or tuned, particles in cell order and few particles take
+ * the first, others the last; cg_get_deposit_variant is then
+ * cg_deposit_variants(), and setting that number goes back to it.
+ * cg_sim_tune_deposit times every variant on the handle's current particles
+ * (best of 3 CUDA-event timings), installs the fastest for the handle's mesh
+ * size and returns it (or a negative CG_E* code); ms (may be NULL) receives
+ * each variant's time.  It wraps the positions into the box first
+ * (move_particles2's wrap) and leaves a deposit of them in the density mesh.  All variants give the same density to float
  * rounding. */
 int cg_deposit_variants(void);
 int cg_get_deposit_variant(int ngrid);

@@ -185,3 +185,36 @@ def test_merged_deposit_runs(gpu_lib, N, n):
         sim.close()
     finally:
         gpu_lib.cg_set_deposit_variant(N, old)
+
+
+def test_box_deposit_can_be_asked_for(gpu_lib):
+    """Variant 0 is the 512-particle box whatever the order and number of the
+    particles, and a mesh without a choice reports, and can be given back, the
+    rule.  All particles sit at one point, so that a shape adds equal numbers and
+    gives the same bits in every run: the two boxes of 512 particles agree, and
+    the merge in the warp (sums of 32 first) differs from them."""
+    from cola_halo_b200 import PARTICLE_DTYPE, Simulation
+    N, n = 64, 1 << 17
+    p = np.zeros(n, dtype=PARTICLE_DTYPE)
+    p["x"] = (20.3, 30.7, 40.1)
+    nv = gpu_lib.cg_deposit_variants()
+    old = gpu_lib.cg_get_deposit_variant(N)
+    sim = Simulation(N, N, float(N), OM)
+    sim.keep_density(True)
+    sim.set_particles(p, 0.1, 0.1)
+
+    def density(v):
+        assert gpu_lib.cg_set_deposit_variant(N, v) == 0
+        assert gpu_lib.cg_get_deposit_variant(N) == v
+        assert gpu_lib.cg_sim_forces(sim.h, None) == 0
+        return sim.get_mesh(0)
+
+    try:
+        box, other, merged, rule = density(0), density(4), density(nv - 1), density(nv)
+        np.testing.assert_array_equal(box, other)
+        assert (box != merged).any()
+        np.testing.assert_array_equal(rule, merged)      # not in cell order
+        assert gpu_lib.cg_set_deposit_variant(N, nv + 1) != 0
+    finally:
+        gpu_lib.cg_set_deposit_variant(N, old)
+        sim.close()

@@ -322,6 +322,11 @@ cudaError_t cnet_alloc(CNet* n, int N, unsigned long long seed) {
   const int P = CNET_PARAMS;
   cudaError_t e = cudaSuccess;
 #define CN_TRY(x) do { if (e == cudaSuccess) e = (x); } while (0)
+  // shared-memory limits belong to a device, so every net sets them on its own
+  CN_TRY(conv_tc_set_smem());
+  CN_TRY(conv_wgrad_set_smem());
+  CN_TRY(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              200 * 1024));
   CN_TRY(cudaMalloc(&n->params, sizeof(float) * P));
   CN_TRY(cudaMalloc(&n->grads, sizeof(float) * P));
   CN_TRY(cudaMalloc(&n->m1, sizeof(float) * P));
@@ -442,11 +447,6 @@ cudaError_t cnet_backward(CNet* n, cudaStream_t st, bool gb_ready) {
   const int N = n->N;
   const size_t nv = (size_t)N * N * N;
   const size_t wgrad_smem = sizeof(float) * (9 * (N + 2) * C + N * C);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
   cudaMemsetAsync(n->grads, 0, sizeof(float) * CNET_PARAMS, st);
   float* g = n->g0;
   float* gnext = n->g1;

@@ -62,6 +62,11 @@ cudaError_t cnet_target(CNet* n, const float* const x[3], long long np, float bo
 cudaError_t cnet_apply(const CNet* n, const float* const x[3], long long np, float boxsize,
                        float* const f[3], cudaStream_t st);
 
+// Shared-memory limits of the convolution kernels (convnet_tc.cu) and of the
+// weight gradients (convnet_wgrad.cu) on the current device.
+cudaError_t conv_tc_set_smem();
+cudaError_t conv_wgrad_set_smem();
+
 // tcgen05 convolutions (convnet_tc.cu); cudaErrorNotSupported when the mesh
 // is not a multiple of the 128-voxel tile.
 cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,

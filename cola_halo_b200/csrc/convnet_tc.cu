@@ -477,14 +477,6 @@ template <bool FLIP>
 cudaError_t launch_sweep(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
                          const float* bias, int act, const __nv_bfloat16* gate, float* of,
                          __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv_sweep<FLIP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         sweep_smem_bytes());
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
   const int nrows = N / 2 * (N / TILE_M) * N;
   const int cap = SWEEP_CPS * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);
@@ -630,14 +622,6 @@ __global__ void __launch_bounds__(THREADS, IN_CPS)
 template <bool FLIP, int STAGES, int CPS>
 cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const float* bias,
                      int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv_tc<FLIP, STAGES, CPS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem_bytes(STAGES));
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
   const int ntiles = N * N * (N / TILE_M);
   const int sms = cg_sm_count();
   const int grid = ntiles < CPS * sms ? ntiles : CPS * sms;
@@ -672,7 +656,25 @@ cudaError_t launch(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const
   return launch_v<FLIP, 2, 2>(in, N, w, bias, act, gate, of, ob, o4, st);
 }
 
+// The kernels of one direction.
+template <bool FLIP>
+cudaError_t set_smem() {
+  constexpr auto kMax = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_conv_sweep<FLIP>, kMax, sweep_smem_bytes());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_conv_tc<FLIP, 1, 4>, kMax, smem_bytes(1));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_conv_tc<FLIP, 2, 2>, kMax, smem_bytes(2));
+  return e;
+}
+
 }  // namespace
+
+cudaError_t conv_tc_set_smem() {
+  cudaError_t e = cudaFuncSetAttribute(k_conv_in, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       in_smem_bytes());
+  if (e == cudaSuccess) e = set_smem<false>();
+  if (e == cudaSuccess) e = set_smem<true>();
+  return e;
+}
 
 cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16* w,
                             const float* bias, int act, float* out_f, __nv_bfloat16* out_b,
@@ -683,9 +685,6 @@ cudaError_t conv_tc_forward(const __nv_bfloat16* in, int N, const __nv_bfloat16*
 cudaError_t conv_tc_features(const __nv_bfloat162* in, int N, const __nv_bfloat16* w,
                              const float* bias, int act, __nv_bfloat16* out_b, cudaStream_t st) {
   if (N < TILE_M || N % TILE_M) return cudaErrorNotSupported;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_conv_in, cudaFuncAttributeMaxDynamicSharedMemorySize, in_smem_bytes());
-  if (attr != cudaSuccess) return attr;
   const int ntiles = N * N * (N / TILE_M), cap = IN_CPS * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);
   k_conv_in<<<ntiles < cap ? ntiles : cap, THREADS, in_smem_bytes(), st>>>(in, N, w, bias, act,

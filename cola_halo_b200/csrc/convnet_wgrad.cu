@@ -380,12 +380,17 @@ __global__ void __launch_bounds__(IN_THREADS, IN_CPS)
 
 }  // namespace
 
+cudaError_t conv_wgrad_set_smem() {
+  constexpr auto kMax = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_wgrad_in, kMax, IN_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_conv_wgrad_tc<1>, kMax, SMEM_BYTES);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_conv_wgrad_tc<2>, kMax, SMEM_BYTES);
+  return e;
+}
+
 cudaError_t conv_wgrad_in(const __nv_bfloat162* in, const float* g, int N, float* dw, float* db,
                           cudaStream_t st) {
   if (N % 16) return cudaErrorNotSupported;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_wgrad_in, cudaFuncAttributeMaxDynamicSharedMemorySize, IN_SMEM);
-  if (attr != cudaSuccess) return attr;
   const int nruns = N * N * ((N + RUN - 1) / RUN), cap = IN_CPS * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);
   k_wgrad_in<<<nruns < cap ? nruns : cap, IN_THREADS, IN_SMEM, st>>>(in, g, N, dw, db);
@@ -395,13 +400,6 @@ cudaError_t conv_wgrad_in(const __nv_bfloat162* in, const float* g, int N, float
 cudaError_t conv_wgrad_tc(const __nv_bfloat16* in, const float* g, int N, bool last, float* dw,
                           float* db, cudaStream_t st) {
   if (N % 16) return cudaErrorNotSupported;
-  static const cudaError_t attr = [] {
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_conv_wgrad_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(
-        k_conv_wgrad_tc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  }();
-  if (attr != cudaSuccess) return attr;
   const int nruns = N * N * ((N + RUN - 1) / RUN);
   const int cap = 2 * cg_sm_count();
   prof_mark(st, CG_ST_OTHER);

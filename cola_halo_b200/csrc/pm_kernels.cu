@@ -2058,17 +2058,17 @@ cudaError_t deposit_smem_attr() {
   else return set_smem((const void*)k_deposit_box<c.chunk, c.vmax>, sizeof(float) * c.vmax);
 }
 
+cudaError_t deposit_set_smem() {
+  cudaError_t e = deposit_smem_attr<0>();
+  if (e == cudaSuccess) e = deposit_smem_attr<1>();
+  if (e == cudaSuccess) e = deposit_smem_attr<2>();
+  if (e == cudaSuccess) e = deposit_smem_attr<3>();
+  if (e == cudaSuccess) e = deposit_smem_attr<4>();
+  return e;
+}
+
 // The CIC scatter into the mesh (which holds -1) with deposit variant v.
 void launch_deposit(PmPlan* p, const float* const x[3], long long n, int v, cudaStream_t st) {
-  static const cudaError_t attr = [] {
-    cudaError_t e = deposit_smem_attr<0>();
-    if (e == cudaSuccess) e = deposit_smem_attr<1>();
-    if (e == cudaSuccess) e = deposit_smem_attr<2>();
-    if (e == cudaSuccess) e = deposit_smem_attr<3>();
-    if (e == cudaSuccess) e = deposit_smem_attr<4>();
-    return e;
-  }();
-  (void)attr;
   switch (v) {
     case 1: deposit_variant<1>(p, x, n, st); break;
     case 2: deposit_variant<2>(p, x, n, st); break;
@@ -2261,6 +2261,7 @@ cudaError_t pm_plan_alloc(PmPlan* p, int N, int factor, float L) {
   CG_TRY(cudaMemset(p->dsum, 0, sizeof(double)));
   CG_TRY(cudaMemset(p->err, 0, sizeof(unsigned)));
   CG_TRY(set_all_smem(N));
+  CG_TRY(deposit_set_smem());
   CG_TRY(interp_prefer_l1());
   bool zexplicit = false;
   const int zmode = z_gather_mode(N, &zexplicit);

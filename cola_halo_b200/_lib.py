@@ -47,6 +47,7 @@ SIGNATURES = {
     "cg_sim_drift_coeffs": (i32, [P, f32, f32, f32]),
     "cg_sim_snapshot": (i32, [P, f64, f32, P]),
     "cg_sim_sync": (i32, [P]),
+    "cg_sim_post_error": (i32, [P, ctypes.c_uint]),
     "cg_sim_get_mesh": (i32, [P, i32, P]),
     "cg_sim_keep_density": (i32, [P, i32]),
     "cg_sim_power_spectrum": (i32, [P, i32, i32, P, P, P]),

@@ -315,7 +315,8 @@ static int check_err_word(cg_sim* s) {
   CG_CHECK(cudaStreamSynchronize(s->st), "sync");
   if (err & CG_ERR_TMA_WAIT) {
     cudaMemsetAsync(s->pm.err, 0, sizeof(unsigned), s->st);
-    return set_err(CG_ECUDA, "z transform: a TMA gather did not complete (error word 0x%x)", err);
+    return set_err(CG_ECUDA, "x or z transform: a TMA gather did not complete (error word 0x%x)",
+                   err);
   }
   if (err) {
     cudaMemsetAsync(s->pm.err, 0, sizeof(unsigned), s->st);
@@ -467,6 +468,17 @@ extern "C" int cg_sim_sync(cg_sim* s) {
   return check_err_word(s);
 }
 
+extern "C" int cg_sim_post_error(cg_sim* s, unsigned word) {
+  if (!s) return set_err(CG_EINVAL, "cg_sim_post_error: NULL");
+  unsigned err = 0;
+  CG_CHECK(cudaMemcpyAsync(&err, s->pm.err, sizeof(err), cudaMemcpyDeviceToHost, s->st), "read");
+  CG_CHECK(cudaStreamSynchronize(s->st), "sync");
+  err |= word;
+  CG_CHECK(cudaMemcpyAsync(s->pm.err, &err, sizeof(err), cudaMemcpyHostToDevice, s->st), "write");
+  CG_CHECK(cudaStreamSynchronize(s->st), "sync");
+  return CG_OK;
+}
+
 extern "C" int cg_sim_power_spectrum(cg_sim* s, int nbins, int flags, double* k, double* pk,
                                      double* nmodes) {
   if (!s || !k || !pk || nbins < 1 || nbins > s->pm.N)
@@ -477,12 +489,21 @@ extern "C" int cg_sim_power_spectrum(cg_sim* s, int nbins, int flags, double* k,
            "power spectrum");
   double* h = (double*)malloc(sizeof(double) * 3 * nbins);
   if (!h) return set_err(CG_ENOMEM, "host malloc");
+  unsigned err = 0;
   cudaError_t e = cudaMemcpyAsync(h, s->pm.pk_acc, sizeof(double) * 3 * nbins,
                                   cudaMemcpyDeviceToHost, s->st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&err, s->pm.err, sizeof(err), cudaMemcpyDeviceToHost, s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   if (e != cudaSuccess) {
     free(h);
     return cuda_err(e, "power spectrum readback");
+  }
+  // columns that the x pass's gather gave up on are not transformed (particles
+  // that the deposit left out are the next check's to report)
+  if (err & CG_ERR_TMA_WAIT) {
+    free(h);
+    return check_err_word(s);
   }
   const double N = s->pm.N, L = s->L;
   const double kf = 2.0 * M_PI / L;

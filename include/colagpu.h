@@ -133,13 +133,18 @@ int cg_sim_drift_coeffs(cg_sim* s, float dyyy, float da1, float da2);
 int cg_sim_snapshot(cg_sim* s, double aout, float omega_m, void* pmin_out);
 /* Wait for all queued work of the handle; reports device-side errors. */
 int cg_sim_sync(cg_sim* s);
+/* Set bits of the handle's device error word as a kernel does (1: a negative
+ * cell, 2: a position that is not finite, 4: a TMA gather that did not
+ * complete), to test how a program takes the errors; synchronous. */
+int cg_sim_post_error(cg_sim* s, unsigned word);
 /* Power spectrum of the particles' CIC density on the PM mesh (no
  * reference counterpart; the reference writes only a coarse density grid,
  * coarse_grid.c).  delta_k = r2c(delta)/ngrid^3, P = L^3 |delta_k|^2
  * averaged over shells: bin b has |n| in [b+1/2, b+3/2) in units of the
  * fundamental 2 pi/L.  Outputs nbins values each of mean k (h/Mpc), P(k)
  * ((Mpc/h)^3) and the number of modes.  nbins <= ngrid.  Overwrites the
- * density mesh; synchronous. */
+ * density mesh; synchronous.  CG_ECUDA when a transform's gather did not
+ * complete. */
 #define CG_PK_DECONVOLVE_CIC 1   /* divide by the CIC window squared */
 #define CG_PK_SUBTRACT_SHOT 2    /* subtract L^3 / np */
 int cg_sim_power_spectrum(cg_sim* s, int nbins, int flags, double* k, double* pk,

@@ -78,3 +78,26 @@ def test_pk_shells_of_all_meshes(gpu_lib, N, deconv):
         gain = po[ok] / flat[ok]
         assert np.all(np.abs(pk[ok] - po[ok]) <= 2e-5 * flat[ok].max() * gain)
     sim.close()
+
+
+def test_pk_reports_a_gather_that_gave_up(gpu_lib):
+    """The x pass in front of the shells may leave columns untransformed: the call
+    that used them fails, and the next one works.  Errors of the particles keep to
+    the calls that reported them before."""
+    from cola_halo_b200 import PARTICLE_DTYPE, Simulation
+    nc, L = 16, 100.0
+    p = np.zeros(nc ** 3, dtype=PARTICLE_DTYPE)
+    p["x"] = np.random.default_rng(1).uniform(0, L, (nc ** 3, 3))
+    sim = Simulation(nc, 2 * nc, L, OM)
+    sim.set_particles(p, 1.0, 1.0)
+    want = sim.power_spectrum()[1]
+    assert gpu_lib.cg_sim_post_error(sim.h, 4) == 0
+    with pytest.raises(RuntimeError, match="x or z transform"):
+        sim.power_spectrum()
+    assert gpu_lib.cg_sim_sync(sim.h) == 0
+    np.testing.assert_allclose(sim.power_spectrum()[1], want, rtol=1e-4)
+    assert gpu_lib.cg_sim_post_error(sim.h, 2) == 0
+    sim.power_spectrum()
+    assert gpu_lib.cg_sim_sync(sim.h) == -5
+    assert gpu_lib.cg_sim_sync(sim.h) == 0
+    sim.close()

@@ -78,6 +78,7 @@ SIGNATURES = {
     "cg_batch_get_snapshot": (i32, [P, i32, P]),
     "cg_batch_power_spectrum": (i32, [P, i32, P, P, P]),
     "cg_batch_num_nodes": (i32, [P, ctypes.POINTER(sz)]),
+    "cg_batch_post_error": (i32, [P, i32, ctypes.c_uint]),
     "cg_batch_last_ms": (i32, [P, fptr]),
     "cg_fof": (i32, [P, i64, f32, f32, i32, P, i64, ctypes.POINTER(i64)]),
     "cg_coarse_grid": (i32, [P, i64, i64, f32, i32, P, ctypes.POINTER(f64)]),

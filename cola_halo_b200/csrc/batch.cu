@@ -383,6 +383,15 @@ extern "C" int cg_batch_run(cg_batch* b) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->main);
   if (e == cudaSuccess) e = cudaEventElapsedTime(&b->last_ms, b->t0, b->t1);
   if (e != cudaSuccess) return fail(CG_ECUDA, "cg_batch_run: launch", e);
+  // gathers that gave up, whose columns no transform reached
+  for (auto& sb : b->streams) {
+    unsigned err = 0;
+    e = cudaMemcpy(&err, sb.plan.err, sizeof(err), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return fail(CG_ECUDA, "cg_batch_run: error word", e);
+    if (!(err & CG_ERR_TMA_WAIT)) continue;
+    cudaMemset(sb.plan.err, 0, sizeof(err));
+    return fail(CG_ECUDA, "cg_batch_run: x or z transform: a TMA gather did not complete");
+  }
   // density checks of every force evaluation (pm.c:548-553)
   for (auto& r : b->reals) {
     std::vector<double> d(r.nforce);
@@ -394,6 +403,17 @@ extern "C" int cg_batch_run(cg_batch* b) {
       if (fabs(v) > tol) return fail(CG_EDENSITY, "cg_batch_run: CIC density sum check failed");
   }
   return CG_OK;
+}
+
+extern "C" int cg_batch_post_error(cg_batch* b, int i, unsigned word) {
+  if (!b || i < 0 || i >= (int)b->reals.size())
+    return fail(CG_EINVAL, "cg_batch_post_error: bad arguments");
+  unsigned* const at = b->streams[b->reals[i].stream].plan.err;
+  unsigned err = 0;
+  cudaError_t e = cudaMemcpy(&err, at, sizeof(err), cudaMemcpyDeviceToHost);
+  err |= word;
+  if (e == cudaSuccess) e = cudaMemcpy(at, &err, sizeof(err), cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? CG_OK : fail(CG_ECUDA, "cg_batch_post_error", e);
 }
 
 extern "C" int cg_batch_get_snapshot(cg_batch* b, int i, void* pmin_out) {

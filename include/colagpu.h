@@ -249,8 +249,11 @@ int cg_batch_set_particles(cg_batch* b, int i, const void* particles, long long 
  * inside the graph (0: never).  Default: the cg_sim policy (every sixth
  * move from 2^23 particles).  Only before the first cg_batch_run. */
 int cg_batch_set_sort_interval(cg_batch* b, int every);
-/* Launch (recording first if needed) and wait; checks every density sum. */
+/* Launch (recording first if needed) and wait; checks every density sum and
+ * that every gather completed. */
 int cg_batch_run(cg_batch* b);
+/* cg_sim_post_error for the stream of realization i. */
+int cg_batch_post_error(cg_batch* b, int i, unsigned word);
 int cg_batch_get_snapshot(cg_batch* b, int i, void* pmin_out);
 int cg_batch_power_spectrum(cg_batch* b, int i, double* k, double* pk, double* nmodes);
 /* Number of nodes of the recorded graph (after the first run). */

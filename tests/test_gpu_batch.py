@@ -93,3 +93,21 @@ def test_batch_at_batched_workload_sizes(gpu_lib, bbks_table, sort_every):
         assert np.abs(p[upto] / ps[upto] - 1).max() < 1e-3
         sim.close()
     b.close()
+
+
+def test_batch_reports_a_gather_that_gave_up(gpu_lib, bbks_table):
+    """A graph whose transforms may have left columns untouched fails, whichever
+    stream they ran on, and the next launch works."""
+    from cola_halo_b200.batch import Batch
+    specs = [dict(nc=16, ngrid=48, boxsize=100.0, a_init=0.1, nsteps=2, aout=1.0)] * 2
+    b = Batch(specs, OM, nstreams=2)
+    for i in range(2):
+        b.set_particles(i, lattice_particles(16, 100.0, 7 + i, OM, 0.1, bbks_table))
+    b.run()
+    for i in range(2):
+        assert gpu_lib.cg_batch_post_error(b.h, i, 4) == 0
+        with pytest.raises(RuntimeError, match="x or z transform"):
+            b.run()
+        b.run()
+    assert gpu_lib.cg_batch_post_error(b.h, 2, 4) != 0
+    b.close()

@@ -785,7 +785,7 @@ extern "C" int cg_net_train_step(cg_net* h, cg_sim* coarse, cg_sim* fine, float 
   const float* fc[3] = {coarse->ps.f[0], coarse->ps.f[1], coarse->ps.f[2]};
   CG_CHECK(cnet_features(&h->n, coarse->pm.dens, true, st), "features");
   CG_CHECK(cnet_target(&h->n, x, coarse->ps.n, coarse->L, ff, fc, st), "target");
-  CG_CHECK(cnet_forward(&h->n, st, false, true), "forward");
+  CG_CHECK(cnet_forward(&h->n, st, false), "forward");
   CG_CHECK(cnet_loss_grad(&h->n, 1.0 / (double)coarse->ps.n, st), "loss");
   CG_CHECK(cnet_backward(&h->n, st, true), "backward");
   if (lr > 0) CG_CHECK(cnet_adam(&h->n, lr, st), "adam");
@@ -805,7 +805,7 @@ extern "C" int cg_net_forces(cg_net* h, cg_sim* coarse) {
   cudaStream_t st = coarse->st;   // stay on the realization's stream
   const float* x[3] = {coarse->ps.x[0], coarse->ps.x[1], coarse->ps.x[2]};
   CG_CHECK(cnet_features(&h->n, coarse->pm.dens, false, st), "features");
-  CG_CHECK(cnet_forward(&h->n, st, false), "forward");
+  CG_CHECK(cnet_forward(&h->n, st, false, false), "forward");
   CG_CHECK(cnet_apply(&h->n, x, coarse->ps.n, coarse->L, coarse->ps.f, st), "apply");
   return CG_OK;
 }

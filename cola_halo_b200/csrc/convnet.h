@@ -47,10 +47,11 @@ cudaError_t cnet_features(CNet* n, const float* delta, bool wide, cudaStream_t s
 bool cnet_narrow_input(const CNet* n);
 // full: also write the [v][16] output that the loss and the host API read
 // (the packed out4 is always written).  wide: the first layer from act[0], whose
-// sums run in the order of the other pipeline variants.  A training step takes it
-// (36 us more at 128^3): a few voxels decide its loss, where one bf16 rounding of a
-// hidden value shows at 1e-5, so that a step stays the same on every variant.
-cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true, bool wide = false);
+// sums run in one order on every pipeline variant.  A training step takes it (36 us
+// more at 128^3): a few voxels decide its loss, where one bf16 rounding of a
+// hidden value shows at 1e-5; and the host forward and backward, so that they
+// give what a training step computes.  A force reads the pairs (feat).
+cudaError_t cnet_forward(CNet* n, cudaStream_t st, bool full = true, bool wide = true);
 // loss and dL/dout (g0 and its bf16 copy gb) from out4 and the residual sums
 cudaError_t cnet_loss_grad(CNet* n, double inv_msum, cudaStream_t st);
 // gb_ready: gb holds g0 in bf16 already

@@ -211,10 +211,13 @@ int cg_net_set_tensor_cores(cg_net* h, int on);
 /* Pipeline of the tensor-core convolutions, for every net: -1 by mesh size
  * (the default), 0 two stages, 1 one stage, 2 the sweep that uses each
  * input row for the three output rows it touches.  All give bit-identical
- * outputs. */
+ * outputs (the first layer of cg_net_forces is the same on all of them). */
 int cg_net_set_conv_variant(int variant);
-/* Host-array forward / backward (checks): in2 [v][2] scaled features,
- * out3 [v][3] raw outputs, grad3 = dLoss/dout3, grads [num_params]. */
+/* Host-array forward / backward (checks), through the layers as
+ * cg_net_train_step runs them: in2 [v][2] scaled features, out3 [v][3] raw
+ * outputs, grad3 = dLoss/dout3, grads [num_params].  cg_net_forces reads the
+ * first layer's input as pairs on meshes that are multiples of 128: the same
+ * products, added in another order. */
 int cg_net_forward_host(cg_net* h, const float* in2, float* out3);
 int cg_net_backward_host(cg_net* h, const float* in2, const float* grad3, float* grads);
 /* Training step on two realizations holding the same particles; returns the

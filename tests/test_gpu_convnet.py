@@ -133,11 +133,11 @@ def test_training_on_pm_pairs_reduces_force_error(gpu_lib, bbks_table):
 
 
 def test_line_ring_conv_bit_identical(gpu_lib):
-    """At 128^3 the tensor-core convolutions reuse input lines along y (the
-    line ring); its MMAs and operands are those of the one-stage kernel,
-    so forward outputs are bit-identical.  The parameter gradients agree to
-    the rounding of the weight gradient's float atomics, whose order varies
-    from run to run."""
+    """The sweep (variant 2, the default) adds the products of an output in the
+    order of the kernels that take one tile at a time (two stages, one stage), in
+    all three layers as a training step runs them: forward outputs are
+    bit-identical.  The parameter gradients agree to the rounding of the weight
+    gradient's float atomics, whose order varies from run to run."""
     from cola_halo_b200.learned import ConvNet
     n = 128
     rng = np.random.default_rng(5)
@@ -146,14 +146,15 @@ def test_line_ring_conv_bit_identical(gpu_lib):
     net = ConvNet(n, seed=3)
     out, grads = [], []
     try:
-        for v in (1, 2):
+        for v in (1, 2, 0, -1):
             assert gpu_lib.cg_net_set_conv_variant(v) == 0
             out.append(net.forward_host(x))
             grads.append(net.backward_host(x, g))
     finally:
         gpu_lib.cg_net_set_conv_variant(-1)
-    np.testing.assert_array_equal(out[0], out[1])
-    np.testing.assert_allclose(grads[0], grads[1], rtol=1e-4, atol=1e-6 * np.abs(grads[0]).max())
+    for o, d in zip(out[1:], grads[1:]):
+        np.testing.assert_array_equal(out[0], o)
+        np.testing.assert_allclose(grads[0], d, rtol=1e-4, atol=1e-6 * np.abs(grads[0]).max())
     assert gpu_lib.cg_net_set_conv_variant(5) != 0
     net.close()
 
@@ -218,10 +219,10 @@ def test_conv_sweep_two_tiles_per_line(gpu_lib):
 
 
 @pytest.mark.parametrize("n,taps", [(128, (0, 13, 26)), (128, (2, 9, 20)), (256, (6, 17, 24))])
-def test_first_layer_from_packed_features(gpu_lib, n, taps):
-    """The first layer reads the two live input channels as pairs: weights that
-    pick one tap and channel each (tile and line ends, all three periodic faces)
-    give the shifted inputs back exactly, the other layers passing them on."""
+def test_first_layer_taps(gpu_lib, n, taps):
+    """Weights that pick one tap and channel each (tile and line ends, all three
+    periodic faces) give the shifted inputs back exactly, the other layers
+    passing them on."""
     net, p = _net(n)
     p = np.zeros_like(p)
     w = p.reshape(3, CR.LAYER)[:, :CR.WSZ].reshape(3, 27, 16, 16)
@@ -262,3 +263,95 @@ def test_weight_gradients_of_every_layer_exact(gpu_lib, n):
             want[t, :len(chans), :3] = a.reshape(-1, 2)[:, list(chans)].T.astype(np.float64) @ gm
         np.testing.assert_array_equal(got[layer][:CR.WSZ].reshape(27, 16, 16), want, str(layer))
         np.testing.assert_array_equal(got[layer][CR.WSZ:CR.WSZ + 3], gm.sum(axis=0))
+
+
+def _first_layer_only(net, w0, bias):
+    """Parameters with first-layer weights w0 [27][2][3] and biases, passed on to
+    the three outputs (hidden values are not negative)."""
+    p = np.zeros(net.nparams, dtype=np.float32).reshape(3, CR.LAYER)
+    w = p[:, :CR.WSZ].reshape(3, 27, 16, 16)
+    w[0, :, :2, :3] = w0
+    p[0, CR.WSZ: CR.WSZ + 3] = bias
+    for c in range(3):
+        w[1, 13, c, c] = w[2, 13, c, c] = 1.0
+    net.set_params(p.ravel())
+
+
+def test_host_forward_is_the_training_step_s(gpu_lib):
+    """The host forward adds the first layer's taps one after another on every
+    pipeline, as a training step does (the pairs that a force reads are added 8
+    taps at a time): 2^24, 1 and -2^24 on three taps in a row give 0."""
+    from cola_halo_b200.learned import ConvNet
+    n = 128
+    net = ConvNet(n, seed=1)
+    w0 = np.zeros((27, 2, 3), dtype=np.float32)
+    w0[[0, 1, 2], 0] = np.array([[2.0 ** 24], [1.0], [-2.0 ** 24]])
+    _first_layer_only(net, w0, 0.0)
+    x = np.ones((n, n, n, 2), dtype=np.float32)
+    try:
+        for v in (0, 1, 2, -1):
+            assert gpu_lib.cg_net_set_conv_variant(v) == 0
+            assert (net.forward_host(x) == 0).all(), v
+    finally:
+        gpu_lib.cg_net_set_conv_variant(-1)
+        net.close()
+
+
+@pytest.mark.parametrize("n", [128, 256])
+def test_force_first_layer_from_packed_features(gpu_lib, n):
+    """cg_net_forces reads its first layer's input as pairs on these meshes.
+    Particles on mesh points give a density of whole numbers, and the output of
+    their own cell: weights 0 and 1 on all taps of the density add up exactly
+    (below 256, so that bf16 holds the hidden value).  A tap of the potential is
+    one product, with which the CUDA-core layers, which read the 16-channel
+    layout, agree exactly.  The net's output is the difference of two float
+    forces: 2^-22 of the larger of them."""
+    from cola_halo_b200 import PARTICLE_DTYPE, Simulation
+    from cola_halo_b200.learned import ConvNet
+    rng = np.random.default_rng(n)
+    m = 20000
+    at = np.concatenate([rng.integers(0, n, (m - 512, 3)),
+                         rng.integers(0, 2, (512, 3)) * (n - 1)])       # and the corners
+    p = np.zeros(m, dtype=PARTICLE_DTYPE)
+    p["x"] = at
+    sim = Simulation(n // 2, n, float(n), 0.273)
+    sim.set_particles(p, 0.5, 0.5)
+    sim.forces()
+    plain = sim.get_forces().astype(np.float64)
+    net = ConvNet(n, seed=1)
+    net.set_scales(1.0, 1.0, 1.0)
+    count = np.zeros((n, n, n))
+    np.add.at(count, tuple(at.T), 8.0)           # (ngrid / nc)^3 a particle
+    pick = tuple(at.T)
+
+    def correction():
+        net.forces(sim)
+        return sim.get_forces().astype(np.float64) - plain
+
+    taps = rng.integers(0, 2, (27, 3)).astype(np.float32)
+    taps[[0, 13, 26]] = 1.0
+    taps *= (np.cumsum(taps, axis=0) <= 8)       # at most 8 taps an output
+    w0 = np.zeros((27, 2, 3), dtype=np.float32)
+    w0[:, 0] = taps
+    _first_layer_only(net, w0, taps.sum(axis=0))     # sum w (count - 1) + sum w
+    got = correction()
+    for c in range(3):
+        want = sum(np.roll(count, (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2))
+                   for t in range(27) if taps[t, c])[pick]
+        ok = want < 256
+        assert ok.mean() > 0.5
+        tol = 2.0 ** -22 * (np.abs(plain[:, c]) + want)
+        assert (np.abs(got[:, c] - want) <= tol)[ok].all(), c
+    for t0 in range(0, 27, 3):
+        w0 = np.zeros((27, 2, 3), dtype=np.float32)
+        for c in range(3):
+            w0[t0 + c, 1, c] = 1.0
+        _first_layer_only(net, w0, 0.0)
+        net.tensor_cores(True)
+        packed = correction()
+        net.tensor_cores(False)
+        wide = correction()
+        assert np.abs(packed).max() > 0
+        np.testing.assert_array_equal(packed, wide, str(t0))
+    net.close()
+    sim.close()

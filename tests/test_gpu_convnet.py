@@ -164,10 +164,14 @@ def test_tensor_core_weight_gradient(gpu_lib, n):
     """The tensor-core weight gradient of the last layer against float64, on
     meshes of one and of two z runs per line and with remainders of 16.  The
     first two layers are set to exact copies (powers of two of non-negative
-    bf16 inputs), so the last layer's input is known bit for bit.  Bound: the
-    float32 sums of a weight take at most 2 x 8 tensor-core steps per run, one
-    addition per run of a CTA and one atomic per CTA, each at most 2^-23 of
-    the sum of |terms|."""
+    bf16 inputs), so the last layer's input is known bit for bit.  A weight's
+    sums take at most 2 x 8 tensor-core steps in a run, one addition per run of a
+    CTA and one atomic per CTA; their errors, at most 2^-23 of a partial sum whose
+    terms have random signs, add up as the root of their number: 8 times that, of
+    the 2-norm of the terms, leaves the largest of the 1296 weights room and is 50
+    times less than g in single bf16 terms would be off.  A bias adds up to four
+    gradients of a run in float32, the rest in double, then nine warps and up to
+    592 CTAs in float32."""
     from cola_halo_b200.learned import ConvNet
     rng = np.random.default_rng(n)
     net = ConvNet(n, seed=1)
@@ -185,17 +189,18 @@ def test_tensor_core_weight_gradient(gpu_lib, n):
     act = np.concatenate([x.astype(np.float64) * 2.0 ** -k for k in range(8)], axis=-1)
     act, g64 = act.reshape(n, n, n, 16), g.astype(np.float64)
     runs = n * n * -(-n // 128)
-    steps = 16 * -(-runs // 148) + 592
+    ctas = 2 * 148
+    tol = 8 * np.sqrt(16 + -(-runs // ctas) + min(runs, ctas)) * 2.0 ** -23
     for t in range(27):
         a = np.roll(act, (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), axis=(0, 1, 2)).reshape(-1, 16)
         want = a.T @ g64.reshape(-1, 3)
-        size = a.T @ np.abs(g64.reshape(-1, 3))
+        size = np.sqrt((a * a).T @ (g64 * g64).reshape(-1, 3))
         d = got[: CR.WSZ].reshape(27, 16, 16)[t]
-        assert (np.abs(d[:, :3] - want) <= steps * 2.0 ** -23 * size).all(), t
+        assert (np.abs(d[:, :3] - want) <= tol * size).all(), t
         assert (d[:, 3:] == 0).all()
     db = got[CR.WSZ:]
     size = np.abs(g64).sum(axis=(0, 1, 2))
-    assert (np.abs(db[:3] - g64.sum(axis=(0, 1, 2))) <= 128 * steps * 2.0 ** -23 * size).all()
+    assert (np.abs(db[:3] - g64.sum(axis=(0, 1, 2))) <= (4 + 9 + 592) * 2.0 ** -24 * size).all()
     assert (db[3:] == 0).all()
 
 
@@ -355,3 +360,55 @@ def test_force_first_layer_from_packed_features(gpu_lib, n):
         np.testing.assert_array_equal(packed, wide, str(t0))
     net.close()
     sim.close()
+
+
+@pytest.mark.parametrize("n", [16, 48, 128, 144])
+@pytest.mark.parametrize("layer", [0, 1, 2])
+def test_weight_gradients_need_every_term(gpu_lib, n, layer):
+    """Weight gradients of one layer, exact, where its output gradient is a whole
+    number of 18 bits with the lowest set: rounded to one bf16 term, or two, it
+    is another number.  The last layer is given it; the layers below get it as the
+    sum of three of six bits in steps of 2^6 (the data gradients multiply bf16
+    numbers, which hold each), on all 16 channels.  Six voxels a call, at the ends of
+    lines, runs and products, and inputs of 1 and 2: every partial sum is a whole
+    number below 2^22."""
+    rng = np.random.default_rng(100 * n + layer)
+    net, p = _net(n)
+    p = np.zeros_like(p)
+    w = p.reshape(3, CR.LAYER)[:, :CR.WSZ].reshape(3, 27, 16, 16)
+    for c in range(16):
+        w[0, 13, c % 2, c] = 1.0
+    if layer == 0:
+        w[1, 13, :, :3] = 1.0                     # gradients of three channels, added up
+        for c in range(3):
+            w[2, 13, c, c] = 1.0
+    else:
+        w[1, 13] = np.eye(16)
+        w[2, 13, :, :3] = 1.0
+    net.set_params(p)
+    net.tensor_cores(True)
+    x = rng.integers(1, 3, (n, n, n, 2)).astype(np.float32)
+    step = np.array([4096, 64, 1])
+    for call in range(4):
+        g = np.zeros((n, n, n, 3), dtype=np.float32)
+        z = rng.permutation([0, n - 1, 15, n - 16, rng.integers(n), min(127, n - 2)])
+        at = np.stack([rng.permutation(n)[:6], rng.choice([0, 1, n - 1, n // 2], 6), z], axis=1)
+        parts = 2 * rng.integers(16, 32, (6, 3)) + 1          # odd, 33 .. 63
+        if layer == 2:
+            g[tuple(at.T)] = (2 * rng.integers(1 << 16, 1 << 17, (6, 3)) + 1) * rng.choice(
+                [-1, 1], (6, 3))
+        else:
+            g[tuple(at.T)] = parts * step
+        got = net.backward_host(x, g).reshape(3, CR.LAYER)[layer]
+        # the layer's output gradient: the given one, or its channels' sum on all 16
+        out = g if layer == 2 else np.repeat(g.sum(axis=-1, keepdims=True), 16, axis=-1)
+        nout = out.shape[-1]
+        chans = [c % 2 for c in range(2 if layer == 0 else 16)]
+        dw = got[:CR.WSZ].reshape(27, 16, 16)
+        for t in range(27):
+            src = (at + (t // 9 - 1, t // 3 % 3 - 1, t % 3 - 1)) % n
+            want = x[tuple(src.T)][:, chans].T.astype(np.float64) @ out[tuple(at.T)]
+            np.testing.assert_array_equal(dw[t, :len(chans), :nout], want, str((call, t)))
+        np.testing.assert_array_equal(got[CR.WSZ:CR.WSZ + nout],
+                                      out.reshape(-1, nout).sum(axis=0, dtype=np.float64))
+    net.close()

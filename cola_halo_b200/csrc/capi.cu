@@ -487,13 +487,12 @@ extern "C" int cg_sim_power_spectrum(cg_sim* s, int nbins, int flags, double* k,
   CG_CHECK(pm_power_spectrum(&s->pm, x, s->ps.n, nbins, flags & CG_PK_DECONVOLVE_CIC,
                              s->pm.pk_acc, s->st),
            "power spectrum");
-  double* h = (double*)malloc(sizeof(double) * 3 * nbins);
+  // the sums and, behind the last bin that there can be, the error word
+  const size_t words = 3 * (size_t)s->pm.N + 1;
+  double* h = (double*)malloc(sizeof(double) * words);
   if (!h) return set_err(CG_ENOMEM, "host malloc");
-  unsigned err = 0;
-  cudaError_t e = cudaMemcpyAsync(h, s->pm.pk_acc, sizeof(double) * 3 * nbins,
+  cudaError_t e = cudaMemcpyAsync(h, s->pm.pk_acc, sizeof(double) * words,
                                   cudaMemcpyDeviceToHost, s->st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&err, s->pm.err, sizeof(err), cudaMemcpyDeviceToHost, s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   if (e != cudaSuccess) {
     free(h);
@@ -501,6 +500,8 @@ extern "C" int cg_sim_power_spectrum(cg_sim* s, int nbins, int flags, double* k,
   }
   // columns that the x pass's gather gave up on are not transformed (particles
   // that the deposit left out are the next check's to report)
+  unsigned err = 0;
+  memcpy(&err, h + words - 1, sizeof(err));
   if (err & CG_ERR_TMA_WAIT) {
     free(h);
     return check_err_word(s);

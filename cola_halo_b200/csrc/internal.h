@@ -48,7 +48,7 @@ struct PmPlan {
   float2* twN;              // exp(-2 pi i k/N), k < N
   float2* twH;              // exp(-2 pi i k/(N/2)), k < N/2
   double* dsum;             // device: sum of the density mesh (check)
-  double* pk_acc;           // device: 3 N doubles of power-spectrum bin sums
+  double* pk_acc;           // device: 3 N doubles of power-spectrum bin sums, then err
   unsigned* err;            // device: error word
   size_t mesh_bytes;        // bytes of one real mesh
   size_t spec_bytes;        // bytes of one half spectrum

@@ -2248,8 +2248,8 @@ cudaError_t pm_plan_alloc(PmPlan* p, int N, int factor, float L) {
   CG_TRY(cudaMalloc(&p->twN, sizeof(float2) * lenN));
   CG_TRY(cudaMalloc(&p->twH, sizeof(float2) * lenH));
   CG_TRY(cudaMalloc(&p->dsum, sizeof(double)));
-  CG_TRY(cudaMalloc(&p->pk_acc, sizeof(double) * 3 * N));
-  CG_TRY(cudaMalloc(&p->err, sizeof(unsigned)));
+  CG_TRY(cudaMalloc(&p->pk_acc, sizeof(double) * (3 * N + 1)));
+  p->err = reinterpret_cast<unsigned*>(p->pk_acc + 3 * N);
   {
     float2* h = (float2*)malloc(sizeof(float2) * (lenN > lenH ? lenN : lenH));
     twiddle_table(h, N);
@@ -2414,7 +2414,6 @@ void pm_plan_free(PmPlan* p) {
   cudaFree(p->twH);
   cudaFree(p->dsum);
   cudaFree(p->pk_acc);
-  cudaFree(p->err);
   cudaFree(p->cb_cnt);
   cudaFree(p->cb_bsum);
   cudaFree(p->cb_rank);

@@ -250,11 +250,14 @@ __global__ void __launch_bounds__(THREADS, CPS)
 // row x' (the four lines y0-1 .. y0+2) adds to the outputs of rows x'-1, x'
 // and x'+1 at once: one MMA of M = 128 voxels, N = 48 columns (the three
 // rows' 16 output channels, with the weights of dx = +1, 0, -1) and K = 16
-// per output line, dy and dz.  The A operand (128 rows of 32 bytes from shared
-// memory) is what an MMA of N <= 64 waits for, so this does 9 reads of it per
-// output line where one tile at a time (N = 16) needs 27; and the lines come
-// from L2 twice per output line instead of three (k_conv_ring before this) or
-// nine times.
+// per output line, dy and dz.  So the A operand (128 rows of 32 bytes from
+// shared memory) is read 9 times per output line where one tile at a time
+// (N = 16) reads it 27 times, and the lines come from L2 twice per output line
+// instead of nine times.  128^3: 79-90 us a layer under ncu.  The operand reads
+// (32 clocks each) come to about 19 us of that and the layer's bytes to 20; the
+// rest is the chain of a row: wait for its copy, issue, commit, wait, drain,
+// zero, barrier, which four CTAs per SM overlap in part (tensor pipe active 20 %
+// of the time).
 //
 // The three accumulators of an output column y sit in tensor-memory slots o
 // mod 3 (o the output row counted from the run's start).  The rows x'-1, x',
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(THREADS, SWEEP_CPS)
   uint8_t* sB = sm + 2 * SROW_BYTES;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sB + 9 * SB_BYTES);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -636,13 +639,12 @@ cudaError_t launch_v(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, con
 // COLAGPU_CONV_VARIANT=0/1/2 selects one.
 int g_conv_variant = -1;      // conv_tc_set_variant
 
-int conv_variant(int N) {
+int conv_variant() {
   static const int forced = [] {
     const char* e = getenv("COLAGPU_CONV_VARIANT");
     return e ? atoi(e) : -1;
   }();
   const int v = forced >= 0 ? forced : g_conv_variant;
-  (void)N;
   return v == 0 || v == 1 ? v : 2;
 }
 
@@ -650,7 +652,7 @@ template <bool FLIP>
 cudaError_t launch(const __nv_bfloat16* in, int N, const __nv_bfloat16* w, const float* bias,
                    int act, const __nv_bfloat16* gate, float* of, __nv_bfloat16* ob, float4* o4, cudaStream_t st) {
   if (N < TILE_M || N % TILE_M) return cudaErrorNotSupported;
-  const int v = conv_variant(N);
+  const int v = conv_variant();
   if (v == 2) return launch_sweep<FLIP>(in, N, w, bias, act, gate, of, ob, o4, st);
   if (v == 1) return launch_v<FLIP, 1, 4>(in, N, w, bias, act, gate, of, ob, o4, st);
   return launch_v<FLIP, 2, 2>(in, N, w, bias, act, gate, of, ob, o4, st);

@@ -28,9 +28,9 @@
 // 256^3 particles, L = 600, ll = 0.2 spacings, a third of them in halos: the
 // link kernel takes 5.3 ms (12.4 with all 27 neighbour cells and a union-find
 // over the original indices; 8.8 with one candidate at a time), and the whole call
-// 10.2 ms (26.6).  The link kernel is bound by its chains of dependent L2 loads:
-// cell starts, candidates, parents; two thirds of it are the slots outside
-// clumps.
+// 9.5 to 10.7 ms (26.6), of which about 2 go to the allocation.  The link kernel
+// is bound by its chains of dependent loads: cell starts (134M of them, four
+// times L2), candidates, parents; two thirds of it are the slots outside clumps.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>

@@ -28,7 +28,7 @@ inline int grid_for(long long n) { return cg_grid(n, 16); }
 enum {
   CG_ERR_BAD_CELL = 1,      // a particle's y or z cell index was negative
   CG_ERR_NONFINITE = 2,     // a particle position was NaN or infinite
-  CG_ERR_TMA_WAIT = 4,      // a TMA gather of the z transform did not complete
+  CG_ERR_TMA_WAIT = 4,      // a TMA gather of the x or z transform did not complete
 };
 
 // Mesh transform plan: every buffer of one PM mesh size.

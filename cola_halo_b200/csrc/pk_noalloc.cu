@@ -65,7 +65,7 @@ unsigned long long current_context_id() {
   return id;
 }
 
-// Same binning as the PM power spectrum (pm_kernels.cu k_pk_bin), for the
+// Same binning as the PM power spectrum (pm_kernels.cu k_fy_pk), for the
 // half-spectrum layout spec[kx][ky][kz], kz = 0..N/2 fastest.
 __global__ void __launch_bounds__(T) k_pk_bin_xyz(const float2* __restrict__ spec, int N,
                                                   int nbins, int deconv,

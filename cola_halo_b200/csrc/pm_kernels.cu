@@ -54,7 +54,7 @@ bool x_maps_for(PmPlan* p, int tk);
 namespace {
 
 constexpr int T = CG_THREADS;
-constexpr size_t kL2Bytes = (size_t)126 << 20;
+constexpr size_t kL2Bytes = (size_t)126 << 20;   // B200's (the device reports 126.5 MiB)
 constexpr int TY = 16;   // z-lines per CTA in FZ / ZI
 constexpr int BY = 8;    // y-lines per CTA in FY
 
@@ -495,9 +495,13 @@ __host__ __device__ constexpr GreenCfg green_cfg(int N, int v) {
 // nor __restrict__ there.
 template <bool RESET> using DensPtr = typename std::conditional<RESET, float*, const float*>::type;
 
-// Threads of the z r2c by mesh size: those whose radix-16 stages (TY N / 32
-// butterflies a CTA) fill them in whole rounds.  us with 256 threads and with these: 512:
-// 275, 261; 384: 134, 119; 128: 10.4, 8.7.
+// Threads of the z r2c by mesh size, by timing: us with 128 and with 256
+// threads, alone: 16: 4.1, 3.9; 32: 4.2, 4.1; 48: 4.3, 4.1; 64: 5.1, 4.3; 96: 6.3,
+// 6.2; 128: 8.3, 10.3; 144: 12.1, 14.0; 192: 20.8, 20.6; 256: 40.9, 41.1; 384: 120,
+// 135; 512: 263, 276; 768: 1273, 935; 1024: 3070, 2342.  (A CTA's TY N / 32
+// radix-16 butterflies leave half of 256 threads without one at 128 and in the second
+// round at 144 and 384; from 768 up a thread of 128 would hold several at a
+// time.)
 __host__ __device__ constexpr int fz_threads(int N) {
   return N == 128 || N == 144 || (N >= 256 && N <= 512) ? 128 : 256;
 }

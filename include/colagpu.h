@@ -396,8 +396,10 @@ int cg_set_force_interp(int mode);
  *   (caller)             buffer forces back to their owners, added to theirs.
  * cg_sim_state_ptrs gives the device arrays of positions and forces (three
  * each); cg_sim_spectrum_ptr the half spectrum (0) or the force spectra
- * (1..3), laid out [kz][kx][ky].  cola_halo_b200/slab.py drives them over
- * torch.distributed. */
+ * (1..3), laid out [kz][kx][ky].  Pointer 0 holds the density's spectrum from
+ * cg_sim_slab_density to cg_sim_slab_kspace; every other call that makes a
+ * force or a P(k) uses it as scratch.  cola_halo_b200/slab.py drives them
+ * over torch.distributed. */
 int cg_sim_state_ptrs(cg_sim* s, float** x, float** f);
 int cg_sim_spectrum_ptr(cg_sim* s, int which, void** ptr);
 int cg_sim_slab_density(cg_sim* s, int x0, int nx, const float* bx, long long nb,

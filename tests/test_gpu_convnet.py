@@ -366,8 +366,8 @@ def test_force_first_layer_from_packed_features(gpu_lib, n):
 @pytest.mark.parametrize("layer", [0, 1, 2])
 def test_weight_gradients_need_every_term(gpu_lib, n, layer):
     """Weight gradients of one layer, exact, where its output gradient is a whole
-    number of 18 bits with the lowest set: rounded to one bf16 term, or two, it
-    is another number.  The last layer is given it; the layers below get it as the
+    number of 18 bits with the lowest set: rounded to one bf16 term it is another
+    number, and every other one to two.  The last layer is given it; the layers below get it as the
     sum of three of six bits in steps of 2^6 (the data gradients multiply bf16
     numbers, which hold each), on all 16 channels.  Six voxels a call, at the ends of
     lines, runs and products, and inputs of 1 and 2: every partial sum is a whole

@@ -383,15 +383,20 @@ extern "C" int cg_batch_run(cg_batch* b) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->main);
   if (e == cudaSuccess) e = cudaEventElapsedTime(&b->last_ms, b->t0, b->t1);
   if (e != cudaSuccess) return fail(CG_ECUDA, "cg_batch_run: launch", e);
-  // gathers that gave up, whose columns no transform reached
+  // gathers that gave up, whose columns no transform reached; every stream's
+  // word is cleared, so that the next launch answers for itself
+  bool gave_up = false;
   for (auto& sb : b->streams) {
     unsigned err = 0;
     e = cudaMemcpy(&err, sb.plan.err, sizeof(err), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && (err & CG_ERR_TMA_WAIT)) {
+      gave_up = true;
+      e = cudaMemset(sb.plan.err, 0, sizeof(err));
+    }
     if (e != cudaSuccess) return fail(CG_ECUDA, "cg_batch_run: error word", e);
-    if (!(err & CG_ERR_TMA_WAIT)) continue;
-    cudaMemset(sb.plan.err, 0, sizeof(err));
-    return fail(CG_ECUDA, "cg_batch_run: x or z transform: a TMA gather did not complete");
   }
+  if (gave_up)
+    return fail(CG_ECUDA, "cg_batch_run: x or z transform: a TMA gather did not complete");
   // density checks of every force evaluation (pm.c:548-553)
   for (auto& r : b->reals) {
     std::vector<double> d(r.nforce);

@@ -109,5 +109,10 @@ def test_batch_reports_a_gather_that_gave_up(gpu_lib, bbks_table):
         with pytest.raises(RuntimeError, match="x or z transform"):
             b.run()
         b.run()
+    for i in range(2):
+        assert gpu_lib.cg_batch_post_error(b.h, i, 4) == 0
+    with pytest.raises(RuntimeError, match="x or z transform"):
+        b.run()
+    b.run()
     assert gpu_lib.cg_batch_post_error(b.h, 2, 4) != 0
     b.close()
